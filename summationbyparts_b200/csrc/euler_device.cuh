@@ -24,17 +24,15 @@ struct BlockDev {
     int nx, ny, npad;
     int op_xi, op_eta;
     int instance;
-    int simd_f64;  // columns j < simd_f64 use fused column sums (f64x8 lanes)
-    int simd_f32;  // same for f32x16 lanes
     int bc_kind[4];
     int bc_nb[4];
     int bc_aux[4];   // BC_INTERPOLATE: interpolation operator; BC_MULTIGRID: first segment in the table
     int bc_aux2[4];  // BC_MULTIGRID: number of segments
     int64_t q_off, m_off, x_off;
     int64_t e_off;  // slot of this block's first edge point in the edge-k buffer (see edge_index)
-    int64_t r_off;  // compensated f32: this block's free-stream dissipation plane (see InstanceDev)
+    int64_t r_off;  // this block's free-stream dissipation plane (compensated f32, see InstanceDev),
+                    // or its 1 / J plane (f64)
     double idx_xi, idx_eta;  // 1/(1/(n-1)) per direction, f64
-    float idx_xi_f, idx_eta_f;
     double hi_xi, hi_eta;  // SAT penalty (n-1)/H_0 (euler/src/lib.rs:1033-1037)
 };
 

@@ -94,18 +94,21 @@ SBP_COEF_ALL_DISS(UPWIND9H2, UPWIND9H2)
 #undef SBP_COEF_ALL_DISS
 
 
-// The interior diagonals (v) and start-closure blocks (st, M x N by rows) in f32 as
-// compile-time constants (the same literals as the constant tables): the micro-tile kernel takes
-// its stencil coefficients from here, so each tap's coefficient is an immediate and the zero tap
-// of a central difference is skipped.
-template <int OP, int KIND>
+// The interior diagonals (v) and start-closure blocks (st, M x N by rows) as compile-time constants
+// (the same literals as the constant tables): the stage kernels take their stencil coefficients
+// from here, so each tap's coefficient is an immediate and the zero tap of a central difference is
+// skipped.
+template <int OP, int KIND, class T>
 struct CDiag;
-#define SBP_CD(OP, TAG, KINDV, KINDN)                                              \
-    template <>                                                                     \
-    struct CDiag<OP, KINDV> {                                                       \
-        static constexpr float v[] = {SBPC_##TAG##_##KINDN##_DIAG(SBPC_LIT_F32)};   \
-        static constexpr float st[] = {SBPC_##TAG##_##KINDN##_START(SBPC_LIT_F32)}; \
+#define SBP_CD1(OP, TAG, KINDV, KINDN, T, LIT)                         \
+    template <>                                                        \
+    struct CDiag<OP, KINDV, T> {                                       \
+        static constexpr T v[] = {SBPC_##TAG##_##KINDN##_DIAG(LIT)};   \
+        static constexpr T st[] = {SBPC_##TAG##_##KINDN##_START(LIT)}; \
     };
+#define SBP_CD(OP, TAG, KINDV, KINDN)                 \
+    SBP_CD1(OP, TAG, KINDV, KINDN, double, SBPC_LIT_F64) \
+    SBP_CD1(OP, TAG, KINDV, KINDN, float, SBPC_LIT_F32)
 SBP_CD(UPWIND4, UPWIND4, DIFF, DIFF)
 SBP_CD(UPWIND4H2, UPWIND4H2, DIFF, DIFF)
 SBP_CD(UPWIND9, UPWIND9, DIFF, DIFF)
@@ -117,6 +120,7 @@ SBP_CD(UPWIND4H2, UPWIND4H2, DISS, DISS)
 SBP_CD(UPWIND9, UPWIND9, DISS, DISS)
 SBP_CD(UPWIND9H2, UPWIND9H2, DISS, DISS)
 #undef SBP_CD
+#undef SBP_CD1
 
 template <int OP, int KIND, class T>
 __device__ __forceinline__ T coef_end(int i, int k) {
@@ -246,35 +250,6 @@ __device__ __forceinline__ T sum_unfused0(int i, int n, P&& p) {
         const int b = i - H;
 #pragma unroll
         for (int d = 0; d < D; ++d) f = f + C::diag(d) * p(b + d);
-    }
-    return f;
-}
-
-// Closure rows only (i < M or i >= n - M), as rolled loops with runtime-indexed coefficients:
-// the same sums in the same order as the unrolled forms above, in a fraction of the code.
-// FUSED selects the fma chain from zero, otherwise t = c0*p0; t = t + ck*pk (ZERO_START = false)
-// or f = 0 + ck*pk (ZERO_START = true).
-template <int OP, int KIND, class T, int MODE, class P>
-__device__ __noinline__ T closure_sum(int i, int n, P p) {
-    constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N;
-    using C = Coef<OP, KIND, T>;
-    const bool start = i < M;
-    const int r = start ? i : i - (n - M);
-    const int b = start ? 0 : n - N;
-    auto coef = [&](int k) { return start ? C::start(r * N + k) : coef_end<OP, KIND, T>(r, k); };
-    if (MODE == 0) {  // row order, unfused
-        T t = coef(0) * p(b);
-#pragma unroll 1
-        for (int k = 1; k < N; ++k) t = t + coef(k) * p(b + k);
-        return t;
-    }
-    T f = T(0);
-    if (MODE == 1) {  // fused column lanes
-#pragma unroll 1
-        for (int k = 0; k < N; ++k) f = fma_rn(p(b + k), coef(k), f);
-    } else {  // unfused column remainder
-#pragma unroll 1
-        for (int k = 0; k < N; ++k) f = f + coef(k) * p(b + k);
     }
     return f;
 }

@@ -1,4 +1,4 @@
-// Instantiations of the fused stage kernel for the SBP4/SBP8 operator pairs and of the edge (SAT) kernel, f64 state (reference arithmetic, built with -fmad=false).
+// Instantiations of the fused stage kernel for the SBP4/SBP8 operator pairs and of the edge (SAT) kernel, f64 state (built with -fmad=false).
 #include "stage_dispatch.h"
 #include "stage_kernel.cuh"
 

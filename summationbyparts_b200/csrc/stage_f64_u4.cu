@@ -1,4 +1,4 @@
-// Instantiations of the fused stage kernel: Upwind4/Upwind4h2 operator pairs, f64 state (reference arithmetic, built with -fmad=false).
+// Instantiations of the fused stage kernel: Upwind4/Upwind4h2 operator pairs, f64 state (built with -fmad=false).
 #include "stage_dispatch.h"
 #include "stage_kernel.cuh"
 

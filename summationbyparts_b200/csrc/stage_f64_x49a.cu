@@ -1,5 +1,5 @@
 // Instantiations of the fused stage kernel for operator pairs of two families: Upwind4-family xi operator with an Upwind9-family eta operator;
-// f64 state (reference arithmetic, built with -fmad=false).  The reference composes any (eta, xi)
+// f64 state (built with -fmad=false).  The reference composes any (eta, xi)
 // pair of its six operators (sbp/src/operators.rs:115-150, multigrid/src/parsing.rs:153-164); the
 // upwind form needs an upwind operator in both directions, every other pair runs RHS_trad.
 #include "stage_dispatch.h"

@@ -19,17 +19,30 @@
 // runs one thread per edge point.
 //
 // Work decomposition.  A persistent grid of 256-thread CTAs walks a list of (block, y0, x0)
-// output tiles of TY rows x 32 columns.  Lane = column, warp w owns rows w*R .. w*R+R-1
-// (R = TY/8).  Phase 1 evaluates the pointwise quantities once per point of the
-// cross-shaped region the stencils read -- Ehat and alpha_u q on the tile rows widened by the
-// xi halo, Fhat and alpha_v q on the tile columns widened by the eta halo (boundary closures
-// widen it to the M x N block) -- into shared memory.  Phase 2 applies the 8 xi and 8 eta
-// stencils from shared memory: the eta sums of a thread's R rows share one register window
-// (R + D - 1 loads for R outputs); interior rows and columns take branch-free paths and only
-// the warps on a block edge run the closure code.
+// output tiles of TY rows x 32 columns.  One direction at a time: the fluxes of the tile rows
+// widened by the xi halo (Ehat and alpha_u q, 4 components each) go to a shared flux buffer and
+// every thread forms the xi sums of its micro-tile in registers; the fluxes of the tile columns
+// widened by the eta halo (Fhat, alpha_v q) then replace them in the same buffer for the eta sums.
+// Holding one direction's fluxes instead of both leaves room for the tile's raw state and metric
+// rows, which arrive by asynchronous copies: the next tile's copies start as soon as the eta fluxes
+// are formed and run under the eta sums, the update and the other resident CTA's work.
+//   What bounds it.  With direct loads and both directions' fluxes in shared memory (the form
+// before this one, one output of four components per thread) a tile waited on global loads for
+// most of its time: dropping every stencil sum made an Upwind9 f64 launch only 16% shorter.  Now the
+// shared-memory pipe (about 11 wavefronts per point, 53% busy) and issue (42%) lead; FP64 is at 25%
+// and HBM at 24%.
+//   Micro-tiles.  64 threads per component, each MR rows x MC columns of it (2 x 4 on 16-row tiles):
+// a xi window of MC + 2 H values serves MC outputs and an eta window of MR + 2 H rows serves MR, in
+// 16-byte loads, instead of D loads per output.  The sums then pass through shared memory once, so
+// the update pass reads and writes global memory with consecutive threads on consecutive columns.
+//   Measured (f64, the 256 first instances of the seed-1 ensemble, one stage 1 launch): Upwind9
+// (3.74 M points) 537 -> 315 us, Upwind4 (3.06 M points) 372 -> 204 us.  One bulk copy per row and
+// plane instead of the per-lane copies: 490 us (188 small copies per tile hold up their issuing warp).
 //
-// Precision: T = double reproduces the reference's f64 arithmetic operation by operation
-// (compile with -fmad=false).  T = float with COMP = true runs fluxes, dissipation and
+// Precision: T = double is the f64 form: the reference's terms and stencil sums, with the taps of
+// an output in the reference's order as fma chains, one reciprocal of rho per point and a product
+// with 1 / J in place of its divisions (compile with -fmad=false, so that every tile shape rounds
+// the same way).  T = float with COMP = true runs fluxes, dissipation and
 // stencils in f32 and keeps the RK4 state as a (hi, lo) f32 pair; the step's increment
 // sum_j (b_j dt) k_j is accumulated in f32 and added to the pair once per step with TwoSum;
 // the f32 metrics hold 1 / J (rounded from f64), so the flux divergence is scaled by a product.
@@ -46,7 +59,6 @@
 namespace sbp {
 
 constexpr int kStageThreads = 256;
-constexpr int kStageWarps = kStageThreads / 32;
 constexpr int kTileX = 32;
 
 template <class T>
@@ -70,10 +82,10 @@ struct StageArgs {
     const EvalDev* eval;     // expression programs of SBP_BC_EVAL sides
     double* evz;             // SBP_BC_EVAL data of the launch's edge points (eval_kernel), 4 per point
     const T* met;            // metric planes in T
+    const T* jinv;           // f64: 1 / J planes (BlockDev::r_off)
     const double* met64;     // metric planes in f64 (SAT terms)
     const float* rinf;       // compensated f32, upwind: free-stream dissipation planes (BlockDev::r_off)
     const double* xy;        // coordinates
-    const T* coef;           // operator tables, see coef_base
     double gamma;
     unsigned* status;
 };
@@ -81,13 +93,6 @@ struct StageArgs {
 // Stage index of the k-only mode: the launch computes k = RHS(u_in) (SATs included) into u_out
 // and updates nothing else; explicit tableaus other than RK4 combine the k on the host side.
 constexpr int kStageK = 4;
-
-// Device coefficient table (one per precision): for operator o and kind k the rows
-// [start block M rows][end block M rows][interior diagonal], each row padded to kCoefRow
-// elements (16-byte aligned rows), at coef_base(o, k).
-constexpr int kCoefRow = 16;
-constexpr int kCoefStride = (2 * 8 + 1) * kCoefRow;
-__host__ __device__ constexpr int coef_base(int op, int kind) { return (2 * op + kind) * kCoefStride; }
 
 // Tiles along a line of n outputs (tile_starts in system.cu) start at multiples of T, except that
 // the last tile starts at e = n - M rounded down to even whenever a multiple of T would fall in
@@ -104,28 +109,6 @@ constexpr int region_extent(int T, int H, int M, int N) {
 // Output rows and columns of a tile: the tile list holds (block, y0, x0, th << 16 | tw).
 __device__ __forceinline__ int tile_rows(const int4& td) { return td.w >> 16; }
 __device__ __forceinline__ int tile_cols(const int4& td) { return td.w & 0xffff; }
-
-// Shared-memory geometry of one tile: xi arrays are TY rows x XP columns, eta arrays HYP rows
-// x 32 columns.
-template <int OPX, int OPY, int TY>
-struct StageGeom {
-    static constexpr int XP = region_extent(kTileX, OpShape<OPX>::H, OpShape<OPX>::M, OpShape<OPX>::N);
-    static constexpr int HYP = region_extent(TY, OpShape<OPY>::H, OpShape<OPY>::M, OpShape<OPY>::N);
-    static constexpr int XA = TY * XP;       // elements of one xi array
-    static constexpr int YA = HYP * kTileX;  // elements of one eta array
-};
-
-// Phase-2 operands staged in shared memory by cp.async while phase 1 runs (compensated-f32
-// kernel): slot 0 plane 0 of the f32 metrics (1 / J), then up to three state arrays x 4
-// components (see stage_operands).
-constexpr int kStageSlots = 13;
-__host__ __device__ constexpr int staged_elems(bool comp, int TY) { return comp ? kStageSlots * TY * kTileX : 0; }
-
-template <int OPX, int OPY, int TY, class T>
-constexpr size_t stage_smem(bool upw, bool comp) {
-    using G = StageGeom<OPX, OPY, TY>;
-    return sizeof(T) * ((size_t)(4 * G::XA + 4 * G::YA) * (upw ? 2 : 1) + staged_elems(comp, TY));
-}
 
 // Characteristic SAT of one edge point (euler/src/lib.rs:1150-1252), f64, written row by row
 // so no 4x4 matrix is ever live.  Same operations in the same order as the reference.
@@ -241,76 +224,31 @@ __device__ __forceinline__ void sat_point_fast(double gamma, const double y[4], 
     k[3] += ht * (phi2 * igm1 * l0 + rho * w * l1 + (phi2_c2 + c * theta) * a2 + (phi2_c2 - c * theta) * a3);
 }
 
-// Pointwise quantities of one point (fluxes, euler/src/lib.rs:680-735; upwind_dissipation
-// 619-674) from its state qv and metrics m = (dxi/dx, dxi/dy, deta/dx, deta/dy), each times
-// detJ.  Writes the xi-direction values (Ehat, alpha_u q) and/or eta-direction values (Fhat,
-// alpha_v q) into shared memory at the given slots.
-template <class T, bool UPW, bool EXACT>
-__device__ __forceinline__ void pointwise(const T qv[4], const T m[4], T gamma, T* sxi, int xa, T* seta, int ya,
-                                          bool want_xi, bool want_eta, unsigned& bad) {
-    const T rho = qv[0], rhou = qv[1], rhov = qv[2], e = qv[3];
-    T E[4], F[4];
-    T p_, u = T(0), v = T(0), c = T(0);
-    if constexpr (EXACT) {
-        // the reference's operations, each division rounded on its own
-        p_ = pressure<T>(gamma, rho, rhou, rhov, e);
-        E[1] = rhou * rhou / rho + p_;
-        E[2] = rhou * rhov / rho;
-        E[3] = rhou * (e + p_) / rho;
-        F[2] = rhov * rhov / rho + p_;
-        F[3] = rhov * (e + p_) / rho;
-        if constexpr (UPW) {
-            u = rhou / rho;
-            v = rhov / rho;
-            c = sqrt(gamma * p_ / rho);
-        }
-    } else {
-        // f32 bulk: one reciprocal of rho shared by every quotient
-        const T ri = T(1) / rho;
-        u = rhou * ri;
-        v = rhov * ri;
-        p_ = (gamma - T(1)) * (e - T(0.5) * (rhou * u + rhov * v));
-        E[1] = rhou * u + p_;
-        E[2] = rhou * v;
-        E[3] = u * (e + p_);
-        F[2] = rhov * v + p_;
-        F[3] = v * (e + p_);
-        if constexpr (UPW) c = sqrt(gamma * p_ * ri);
-    }
-    E[0] = rhou;
-    F[0] = rhov;
-    F[1] = E[2];
+// Pointwise quantities of one point of the f64 form in one direction (fluxes,
+// euler/src/lib.rs:680-735; upwind_dissipation 619-674) from its state qv and the direction's metrics
+// jx, jy (each times detJ): the flux Ehat or Fhat and alpha q into shared memory at dst.  The
+// reference divides nine times and takes three roots per point; here one reciprocal of rho serves
+// every quotient, and c |J grad| is one root, sqrt(c^2 |J grad|^2): an f64 division or root is
+// about twenty instructions, and the region of a tile holds almost two points per output.
+template <bool UPW>
+__device__ __forceinline__ void pointwise(const double qv[4], double jx, double jy, double gamma, double* dst,
+                                          int stride, unsigned& bad) {
+    const double rho = qv[0], rhou = qv[1], rhov = qv[2], e = qv[3];
+    const double ri = 1.0 / rho;
+    const double u = rhou * ri, v = rhov * ri;
+    const double p = (gamma - 1.0) * fma_rn(-0.5, fma_rn(rhou, u, rhov * v), e);
+    const double h = e + p;
+    const double E[4] = {rhou, fma_rn(rhou, u, p), rhou * v, u * h};
+    const double F[4] = {rhov, E[2], fma_rn(rhov, v, p), v * h};
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) dst[cc * stride] = fma_rn(jx, E[cc], jy * F[cc]);
     if constexpr (UPW) {
-        if (!(rho > T(0))) bad |= STATUS_RHO;
-        if (!(p_ > T(0))) bad |= STATUS_P;
-    }
-    if (want_xi) {
-        const T jxx = m[0], jxy = m[1];
+        if (!(rho > 0.0)) bad |= STATUS_RHO;
+        if (!(p > 0.0)) bad |= STATUS_P;
+        const double a = fabs(fma_rn(jx, u, jy * v)) + sqrt(gamma * p * ri * fma_rn(jx, jx, jy * jy));
+        double* d = dst + 4 * stride;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) sxi[cc * xa] = jxx * E[cc] + jxy * F[cc];
-        if constexpr (UPW) {
-            const T uhat = jxx * u + jxy * v;
-            const T au = fabs(uhat) + c * sqrt(jxx * jxx + jxy * jxy);
-            T* d = sxi + 4 * xa;
-            d[0] = au * rho;
-            d[xa] = au * rhou;
-            d[2 * xa] = au * rhov;
-            d[3 * xa] = au * e;
-        }
-    }
-    if (want_eta) {
-        const T jyx = m[2], jyy = m[3];
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) seta[cc * ya] = jyx * E[cc] + jyy * F[cc];
-        if constexpr (UPW) {
-            const T vhat = jyx * u + jyy * v;
-            const T av = fabs(vhat) + c * sqrt(jyx * jyx + jyy * jyy);
-            T* d = seta + 4 * ya;
-            d[0] = av * rho;
-            d[ya] = av * rhou;
-            d[2 * ya] = av * rhov;
-            d[3 * ya] = av * e;
-        }
+        for (int cc = 0; cc < 4; ++cc) d[cc * stride] = a * qv[cc];
     }
 }
 
@@ -387,191 +325,28 @@ __device__ __forceinline__ void pointwise_dev(const float d[4], const float m[4]
     if (want_eta) store(m[2], m[3], seta, ya);
 }
 
-// Eta sums of R consecutive rows r0.. of one column from a shared column (stride 32), into
-// out[R], scaled by idx.  `interior` (warp-uniform): every row in [M, ny-M).  EXACT selects the
-// reference's lane split (fma chain for fused columns, unfused sum otherwise); without it the
-// sum is a plain fma chain.  Warps holding closure rows run one N-tap loop per row with the
-// row's coefficients from the table (interior rows predicate off the padding).
-template <int OP, int KIND, class T, int R, bool EXACT>
-__device__ __forceinline__ void eta_rows(const T* __restrict__ col, int ly0, int r0, int nrows, int ny, bool interior,
-                                         bool fused, T idx, const T* __restrict__ ctab, T out[R]) {
-    constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N, D = OpShape<OP>::D, H = OpShape<OP>::H;
-    using C = Coef<OP, KIND, T>;
-    if (interior) {
-        T w[R + D - 1];
-#pragma unroll
-        for (int j = 0; j < R + D - 1; ++j) w[j] = col[(r0 - H + j - ly0) * kTileX];
-#pragma unroll
-        for (int u = 0; u < R; ++u) {
-            T f = T(0);
-            if (!EXACT || fused) {
-#pragma unroll
-                for (int d = 0; d < D; ++d) f = fma_rn(w[u + d], C::diag(d), f);
-            } else {
-#pragma unroll
-                for (int d = 0; d < D; ++d) f = f + C::diag(d) * w[u + d];
-            }
-            out[u] = f * idx;
-        }
-        return;
-    }
-    const T* tab = ctab + coef_base(OP, KIND);
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-        T f = T(0);
-        if (u < nrows) {
-            const int r = r0 + u;
-            const T* crow;
-            int base, ntaps;
-            if (r < M) {
-                crow = tab + r * kCoefRow;
-                base = 0;
-                ntaps = N;
-            } else if (r >= ny - M) {
-                crow = tab + (M + r - (ny - M)) * kCoefRow;
-                base = ny - N;
-                ntaps = N;
-            } else {
-                crow = tab + 2 * M * kCoefRow;
-                base = r - H;
-                ntaps = D;
-            }
-            const T* w = col + (base - ly0) * kTileX;
-            if (!EXACT || fused) {
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                    if (k < ntaps) f = fma_rn(w[k * kTileX], __ldg(crow + k), f);
-            } else {
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                    if (k < ntaps) f = f + __ldg(crow + k) * w[k * kTileX];
-            }
-        }
-        out[u] = f * idx;
-    }
-}
-
-// Xi sums of one kind for the thread's rows: out[c][u] for component c and row ty0 + u of the
-// tile, from the shared xi arrays `sb` (4 component arrays of XA elements, rows of XP, element 0
-// = column lx0).  EXACT: the reference's unfused row order; otherwise an fma chain.  In a tile
-// holding closure columns (`closure_tile`, tile-uniform) every lane loads its own coefficient
-// row once (16-byte vector loads) and runs the same N-tap loop for all 4R sums, so the warp
-// does not diverge; interior lanes predicate off the padding taps.
-template <int OP, int KIND, class T, int R, bool EXACT, int XA, int XP>
-__device__ __forceinline__ void xi_rows(const T* __restrict__ sb, int ty0, int nrows, int lx0, int col, int nx, T idx,
-                                        bool closure_tile, const T* __restrict__ ctab, T out[4][R]) {
-    constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N, D = OpShape<OP>::D, H = OpShape<OP>::H;
-    using C = Coef<OP, KIND, T>;
-    if (!closure_tile) {
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-            for (int u = 0; u < R; ++u) {
-                T t = T(0);
-                if (u < nrows) {
-                    const T* w = sb + cc * XA + (ty0 + u) * XP + (col - H - lx0);
-                    if constexpr (EXACT) {
-                        t = diag_unfused<OP, KIND, T>([&](int d) { return w[d]; });
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < D; ++d) t = fma_rn(w[d], C::diag(d), t);
-                    }
-                }
-                out[cc][u] = t * idx;
-            }
-        return;
-    }
-    const T* crow;
-    int base, ntaps;
-    {
-        const T* tab = ctab + coef_base(OP, KIND);
-        if (col < M) {
-            crow = tab + col * kCoefRow;
-            base = 0;
-            ntaps = N;
-        } else if (col >= nx - M) {
-            crow = tab + (M + col - (nx - M)) * kCoefRow;
-            base = nx - N;
-            ntaps = N;
-        } else {
-            crow = tab + 2 * M * kCoefRow;
-            base = col - H;
-            ntaps = D;
-        }
-    }
-    constexpr int V = 16 / sizeof(T), NV = (N + V - 1) / V;
-    T cf[NV * V];
-    using VT = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) *reinterpret_cast<VT*>(cf + v * V) = __ldg(reinterpret_cast<const VT*>(crow) + v);
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-        for (int u = 0; u < R; ++u) {
-            T t = T(0);
-            if (u < nrows) {
-                const T* w = sb + cc * XA + (ty0 + u) * XP + (base - lx0);
-                t = cf[0] * w[0];
-#pragma unroll
-                for (int k = 1; k < N; ++k)
-                    if (k < ntaps) {
-                        if constexpr (EXACT) t = t + cf[k] * w[k];
-                        else t = fma_rn(cf[k], w[k], t);
-                    }
-            }
-            out[cc][u] = t * idx;
-        }
-}
-
-// Asynchronous global -> shared copy of one element (cp.async, sm_80+), and the wait for all
-// of this thread's copies.
-template <class T>
-__device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem));
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// The state arrays this stage's RK update reads (compensated form), in slot order:
-// stage 0: u_in (= prev_hi); stages 1, 2: delta (acc_hi), prev_hi; stage 3: delta, prev_hi, prev_lo.
-template <class T>
-__device__ __forceinline__ int stage_operands(const StageArgs<T>& A, const T* src[3]) {
-    if (A.stage == 0) {
-        src[0] = A.u_in;
-        return 1;
-    }
-    src[0] = A.acc_hi;
-    src[1] = A.prev_hi;
-    src[2] = A.prev_lo;
-    return A.stage < 3 ? 2 : 3;
-}
-
-// Compensated RK update of one component at element e with its operands taken from the
-// staging slots (sop(a) = operand array a of this component at this point); same arithmetic
-// as rk_update.  cb, ca: this stage's B and A tableau entries times dt, already in f32.
-// The step's increment delta = sum_j (b_j dt) k_j is accumulated in f32 (acc_hi) and added to
-// the (hi, lo) state once, in stage 3, with TwoSum.
-template <class T, class SOP>
-__device__ __forceinline__ void rk_update_staged(const StageArgs<T>& A, int64_t e, float cb, float ca, T kc, SOP sop) {
+// This stage's RK4 update of one component at element e (see the header comment) with its operands
+// in registers: o0, o1, o2 as loaded by the update pass of stage_kernel; cb, ca this stage's B and A
+// tableau entries times dt (ca unused in stage 3).  The compensated form accumulates the step's
+// increment delta = sum_j (b_j dt) k_j in f32 (acc_hi) and adds it to the (hi, lo) state once, in
+// stage 3, with TwoSum.
+template <class T, bool COMP>
+__device__ __forceinline__ void rk_update_ops(const StageArgs<T>& A, int64_t e, T cb, T ca, T k, T o0, T o1, T o2) {
     if (A.stage == kStageK) {
-        A.u_out[e] = kc;
-        return;
-    }
-    const float kf = float(kc);
-    if (A.stage == 0) {
-        A.u_out[e] = T(float(sop(0)) + ca * kf);
-        A.acc_hi[e] = T(cb * kf);
+        A.u_out[e] = k;
+    } else if (A.stage == 0) {
+        A.u_out[e] = fma_rn(ca, k, o0);
+        A.acc_hi[e] = COMP ? cb * k : fma_rn(cb, k, o0);
     } else if (A.stage < 3) {
-        A.u_out[e] = T(float(sop(1)) + ca * kf);
-        A.acc_hi[e] = T(float(sop(0)) + cb * kf);
+        A.u_out[e] = fma_rn(ca, k, o1);
+        A.acc_hi[e] = fma_rn(cb, k, o0);
+    } else if constexpr (COMP) {
+        float hi = o1, lo = o2;
+        comp_add(hi, lo, fma_rn(cb, k, o0));
+        A.new_hi[e] = hi;
+        A.new_lo[e] = lo;
     } else {
-        const float d = float(sop(0)) + cb * kf;
-        float hi = float(sop(1));
-        float lo = float(sop(2));
-        comp_add(hi, lo, d);
-        A.new_hi[e] = T(hi);
-        A.new_lo[e] = T(lo);
+        A.new_hi[e] = fma_rn(cb, k, o0);
     }
 }
 
@@ -749,25 +524,293 @@ __device__ __forceinline__ void sat_edge(const StageArgs<T>& A, const InstanceDe
     }
 }
 
+// ---- geometry of one tile ------------------------------------------------------------------
+// Tiles are TY rows x tile_tx(TY) columns; 256 threads, 64 per component.  A thread's micro-tile
+// is tile_mr(TY) rows x tile_mc(TY) columns, so 8 x 8 threads cover a tile of one component.
+__host__ __device__ constexpr int tile_tx(int ty) { return ty == 8 ? 16 : kTileX; }
+__host__ __device__ constexpr int tile_mr(int ty) { return ty / 8; }
+__host__ __device__ constexpr int tile_mc(int ty) { return tile_tx(ty) / 8; }
+
+// Local column of column x is x - x0 + xi_lead: room for the H halo columns, and for the N - M
+// columns before the last M that an end-closure block reads; even, so that a column's parity and
+// the alignment of its pair do not depend on the tile.  Rows have the same without the evenness.
+__host__ __device__ constexpr int lead_of(int H, int M, int N) { return H > N - M ? H : N - M; }
+__host__ __device__ constexpr int xi_lead(int H, int M, int N) { return (lead_of(H, M, N) + 1) & ~1; }
+// 16-byte (f64) pairs of adjacent columns that one thread's xi window spans.
+__host__ __device__ constexpr int xi_window(int ty, int H, int M, int N) {
+    return (((xi_lead(H, M, N) - H) & 1) + tile_mc(ty) + 2 * H + 1) / 2;
+}
+// Column pairs of one xi row: every region column, and every thread's window.
+__host__ __device__ constexpr int xi_pairs(int ty, int H, int M, int N) {
+    const int L = xi_lead(H, M, N), a = L + (tile_tx(ty) + H > N ? tile_tx(ty) + H : N);
+    const int b = tile_tx(ty) - tile_mc(ty) + 2 * ((L - H) / 2) + 2 * xi_window(ty, H, M, N);
+    return ((a > b ? a : b) + 1) / 2;
+}
+// Pair p of a row is at slot (p & 1) * S + (p >> 1): the 8 threads of one micro-row read pairs
+// of one parity, 8 consecutive 16-byte slots.  S = 4 (mod 8) puts 16 consecutive columns stored
+// by phase 1 on 16 different 8-byte banks; an odd number of slots per row spreads the rows that
+// the closure pass reads down a column.
+__host__ __device__ constexpr int xi_split(int ty, int H, int M, int N) {
+    return (xi_pairs(ty, H, M, N) + 1) / 2 <= 4 ? 4 : 12;
+}
+__host__ __device__ constexpr int xi_pitch(int ty, int H, int M, int N) {
+    return 2 * ((xi_split(ty, H, M, N) + xi_pairs(ty, H, M, N) / 2) | 1);
+}
+__host__ __device__ constexpr int eta_rows(int ty, int H, int M, int N) {
+    return lead_of(H, M, N) + (ty + H > N ? ty + H : N);
+}
+// Raw rows of a tile's region (state and xi metrics) and of its columns (eta metrics), widened to
+// 16-byte boundaries; `al` elements are 16 bytes.
+__host__ __device__ constexpr int raw_pitch(int w, int al) { return (w + 2 * (al - 1)) / al * al; }
+__host__ __device__ constexpr int xi_region(int ty, int H, int M, int N) {
+    return region_extent(tile_tx(ty), H, M, N);
+}
+__host__ __device__ constexpr int flux_elems(int ty, int hx, int mx, int nx, int hy, int my, int ny) {
+    const int a = ty * xi_pitch(ty, hx, mx, nx), b = eta_rows(ty, hy, my, ny) * tile_tx(ty);
+    return a > b ? a : b;
+}
+// Shared memory of a tile in bytes (elements of `ts` bytes): the raw rows and the fluxes of one
+// direction.
+__host__ __device__ constexpr int tile_smem(int ty, bool upw, int ts, int hx, int mx, int nx, int hy, int my, int ny) {
+    const int al = 16 / ts, rp = raw_pitch(xi_region(ty, hx, mx, nx), al), ep = raw_pitch(tile_tx(ty), al);
+    const int rh = eta_rows(ty, hy, my, ny);
+    return ts * (4 * rh * rp + 2 * ty * rp + 2 * rh * ep + (upw ? 8 : 4) * flux_elems(ty, hx, mx, nx, hy, my, ny));
+}
+
+template <int OPX, int OPY, int TY, class T>
+struct TileGeom {
+    using X = OpShape<OPX>;
+    using Y = OpShape<OPY>;
+    static constexpr int TX = tile_tx(TY), MR = tile_mr(TY), MC = tile_mc(TY);
+    static constexpr int XL = xi_lead(X::H, X::M, X::N), YL = lead_of(Y::H, Y::M, Y::N);
+    static constexpr int NP = xi_window(TY, X::H, X::M, X::N);
+    static constexpr int XS = xi_split(TY, X::H, X::M, X::N), XP = xi_pitch(TY, X::H, X::M, X::N);
+    static constexpr int XA = TY * XP;                                    // elements of one xi array
+    static constexpr int YA = eta_rows(TY, Y::H, Y::M, Y::N) * TX;        // elements of one eta array
+    static constexpr int RH = eta_rows(TY, Y::H, Y::M, Y::N);
+    static constexpr int RP = raw_pitch(xi_region(TY, X::H, X::M, X::N), 16 / (int)sizeof(T));
+    static constexpr int EP = raw_pitch(TX, 16 / (int)sizeof(T));
+    static constexpr int FL = flux_elems(TY, X::H, X::M, X::N, Y::H, Y::M, Y::N);
+    static_assert(xi_pairs(TY, X::H, X::M, X::N) <= 24, "xi rows fit the split");
+    // element of local column c in a xi row
+    __device__ __forceinline__ static int xpos(int c) { return (((c >> 1) & 1) * XS + (c >> 2)) * 2 + (c & 1); }
+    // Element of tile column c in an eta row.  Micro-tiles of 4 columns: the even column pairs
+    // first, then the odd ones with their halves of 4 pairs exchanged, so both the 16-byte loads of
+    // phase 2 (8 threads, one parity) and the 8-byte stores of 16 consecutive columns use every
+    // bank once.  Micro-tiles of 2 columns: in order.
+    __device__ __forceinline__ static int epos(int c) {
+        if constexpr (MC == 2) return c;
+        const int p = c >> 1;
+        return (((p & 1) * (TX / 4)) + ((p >> 1) ^ ((p & 1) * 4))) * 2 + (c & 1);
+    }
+};
+
+template <class T>
+struct PairOf;
+template <>
+struct PairOf<double> {
+    using type = double2;
+};
+template <>
+struct PairOf<float> {
+    using type = float2;
+};
+
+// acc += sign * (taps I .. D - 1 of one interior stencil), w[d] the input of tap d; coefficients
+// are compile-time constants and zero taps cost nothing.
+template <int OP, int KIND, int SIGN, int I, class T>
+__device__ __forceinline__ void add_taps(const T* w, T& acc) {
+    if constexpr (I < OpShape<OP>::D) {
+        constexpr T c = CDiag<OP, KIND, T>::v[I];
+        if constexpr (c != T(0)) acc = fma_rn(T(SIGN) * c, w[I], acc);
+        add_taps<OP, KIND, SIGN, I + 1>(w, acc);
+    }
+}
+
+// Xi sums of a micro-tile: acc[u][j] += sign * stencil at (row u, column j); row 0's array row at
+// `row`, the first pair of the thread's window at slot `s0` of parity PAR0.
+template <int OP, int KIND, int SIGN, class G, class T>
+__device__ __forceinline__ void xi_sums(const T* __restrict__ row, int gx, T acc[G::MR][G::MC]) {
+    using V = typename PairOf<T>::type;
+    constexpr int OFF = G::XL - OpShape<OP>::H;  // local column of the first tap of tile column 0
+#pragma unroll
+    for (int u = 0; u < G::MR; ++u) {
+        T w[2 * G::NP];
+#pragma unroll
+        for (int q = 0; q < G::NP; ++q) {
+            // pair p = gx MC / 2 + OFF / 2 + q
+            int slot;
+            if constexpr (G::MC == 4) {
+                constexpr int o = OFF / 2;
+                slot = ((o + q) & 1) * G::XS + gx + ((o + q) >> 1);
+            } else {
+                const int p = gx + OFF / 2 + q;
+                slot = (p & 1) * G::XS + (p >> 1);
+            }
+            const V v = reinterpret_cast<const V*>(row + u * G::XP)[slot];
+            w[2 * q] = v.x;
+            w[2 * q + 1] = v.y;
+        }
+#pragma unroll
+        for (int j = 0; j < G::MC; ++j) add_taps<OP, KIND, SIGN, 0>(w + (OFF & 1) + j, acc[u][j]);
+    }
+}
+
+// Row R of the eta window applied to the MR outputs of each column, then the rows after it.
+template <int OP, int KIND, int SIGN, class G, int R, int U, class T>
+__device__ __forceinline__ void eta_row_taps(const T v[G::MC], T acc[G::MR][G::MC]) {
+    if constexpr (U < G::MR) {
+        constexpr int d = R - U;
+        if constexpr (d >= 0 && d < OpShape<OP>::D) {
+            constexpr T c = CDiag<OP, KIND, T>::v[d];
+            if constexpr (c != T(0)) {
+#pragma unroll
+                for (int j = 0; j < G::MC; ++j) acc[U][j] = fma_rn(T(SIGN) * c, v[j], acc[U][j]);
+            }
+        }
+        eta_row_taps<OP, KIND, SIGN, G, R, U + 1>(v, acc);
+    }
+}
+template <int OP, int KIND, int SIGN, class G, int R, class T>
+__device__ __forceinline__ void eta_sums(const T* __restrict__ col, int gx, T acc[G::MR][G::MC]) {
+    using V = typename PairOf<T>::type;
+    if constexpr (R < G::MR + OpShape<OP>::D - 1) {
+        T v[G::MC];
+        const V* p = reinterpret_cast<const V*>(col + R * G::TX);
+        const V a = p[gx];
+        v[0] = a.x;
+        v[1] = a.y;
+        if constexpr (G::MC == 4) {
+            const V b = p[G::TX / 4 + (gx ^ 4)];
+            v[2] = b.x;
+            v[3] = b.y;
+        }
+        eta_row_taps<OP, KIND, SIGN, G, R, 0>(v, acc);
+        eta_sums<OP, KIND, SIGN, G, R + 1>(col, gx, acc);
+    }
+}
+
+// Closure-block coefficient (row I, input K) of one end of a line: the start block, or the end
+// block (row I applies -/+ st[(M - 1 - I) N + (N - 1 - K)], DIFF negated).
+template <int OP, int KIND, bool RIGHT, int I, int K, class T>
+struct ClosureCoef {
+    static constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N;
+    static constexpr T value = RIGHT ? (KIND == DIFF ? T(-1) : T(1)) * CDiag<OP, KIND, T>::st[(M - 1 - I) * N + (N - 1 - K)]
+                                     : CDiag<OP, KIND, T>::st[I * N + K];
+};
+// Row I of the closure block: the sum over the N inputs v, first product then an fma chain.
+template <int OP, int KIND, bool RIGHT, int I, int K = 1, class T>
+__device__ __forceinline__ T closure_sum(const T* v, T t) {
+    if constexpr (K == 1) t = v[0] * ClosureCoef<OP, KIND, RIGHT, I, 0, T>::value;
+    if constexpr (K < OpShape<OP>::N) {
+        constexpr T c = ClosureCoef<OP, KIND, RIGHT, I, K, T>::value;
+        return closure_sum<OP, KIND, RIGHT, I, K + 1>(v, fma_rn(v[K], c, t));
+    } else {
+        return t;
+    }
+}
+// st(i, diss - diff) for closure rows i = I .. I + CNT - 1.
+template <int OP, bool UPW, bool RIGHT, int I, int CNT, class T, class ST>
+__device__ __forceinline__ void closure_out(const T* ve, const T* va, const ST& st) {
+    if constexpr (CNT > 0) {
+        T d = T(0);
+        if constexpr (UPW) d = closure_sum<OP, DISS, RIGHT, I>(va, T(0));
+        st(I, d - closure_sum<OP, DIFF, RIGHT, I>(ve, T(0)));
+        closure_out<OP, UPW, RIGHT, I + 1, CNT - 1>(ve, va, st);
+    }
+}
+
+// Closure outputs part * CNT .. of one line (diss - diff) into o[CNT], for the warp-uniform run-time
+// `part` of PARTS: ld(kind, k) is input k of the closure block.
+template <int OP, bool UPW, bool RIGHT, int PARTS, int P, class T, class LD>
+__device__ __forceinline__ void closure_part(int part, const LD& ld, T* o) {
+    constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N, CNT = M >= PARTS ? M / PARTS : 1;
+    if constexpr (P * CNT < M && P < PARTS) {
+        if (part == P) {
+            T ve[N], va[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                ve[k] = ld(DIFF, k);
+                va[k] = UPW ? ld(DISS, k) : T(0);
+            }
+            closure_out<OP, UPW, RIGHT, P * CNT, CNT>(ve, va, [&](int i, T v) { o[i - P * CNT] = v; });
+        } else {
+            closure_part<OP, UPW, RIGHT, PARTS, P + 1>(part, ld, o);
+        }
+    }
+}
+
+// 16-byte asynchronous global -> shared copy (cp.async), and the wait for all of this thread's.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <int OPX, int OPY, class T, bool UPW, bool COMP, int TY>
-__global__ void __launch_bounds__(kStageThreads, 2) stage_kernel(const StageArgs<T> A) {
-    using G = StageGeom<OPX, OPY, TY>;
-    constexpr int R = TY / kStageWarps;
-    constexpr int XA = G::XA, YA = G::YA, XP = G::XP;
-    constexpr int P1B = sizeof(T) == 4 ? 4 : 2;  // phase-1 points per thread and batch
+__global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 : 2) stage_kernel(const StageArgs<T> A) {
+    using G = TileGeom<OPX, OPY, TY, T>;
+    using V = typename PairOf<T>::type;
+    constexpr int TX = G::TX, MR = G::MR, MC = G::MC, XA = G::XA, YA = G::YA, RP = G::RP, EP = G::EP, RH = G::RH;
+    constexpr int HY = OpShape<OPY>::H, MX = OpShape<OPX>::M, MY = OpShape<OPY>::M;
+    constexpr int AL = 16 / sizeof(T);  // elements of a 16-byte copy unit
+    // update pass: points and components per thread
+    constexpr int PTS = TY * TX, PPT = PTS >= kStageThreads ? PTS / kStageThreads : 1;
+    constexpr int CPT = PTS >= kStageThreads ? 4 : 4 * PTS / kStageThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* sE = reinterpret_cast<T*>(smem_raw);       // [UPW ? 8 : 4][TY][XP]: Ehat (0..3), alpha_u q (4..7)
-    T* sF = sE + (UPW ? 8 : 4) * XA;              // [UPW ? 8 : 4][HYP][32]: Fhat (0..3), alpha_v q (4..7)
-    T* sR = sF + (UPW ? 8 : 4) * YA;              // [13][TY][32]: staged phase-2 operands (COMP)
+    T* rq = reinterpret_cast<T*>(smem_raw);  // [4][RH][RP]: raw state of the tile's region
+    T* rx = rq + 4 * RH * RP;                // [2][TY][RP]: raw xi metrics of the tile rows
+    T* re = rx + 2 * TY * RP;                // [2][RH][EP]: raw eta metrics of the tile columns
+    T* fl = re + 2 * RH * EP;                // fluxes of one direction: [UPW ? 8 : 4] xi or eta arrays
     const T gamma = T(A.gamma);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tid = threadIdx.x;
+    const int comp = tid >> 6, gx = tid & 7, gy = (tid >> 3) & 7;  // stencil phases
     unsigned bad = 0;
+
+    // Starts the asynchronous copies of one tile's raw rows: every row of the region's state planes,
+    // the xi metrics of the tile rows and the eta metrics of the tile columns, a warp per row, in
+    // 16-byte pieces widened to 16-byte boundaries (a plane's padding holds the overhang).
+    auto fetch = [&](const int4 td) {
+        const BlockDev& B = A.blocks[td.x];
+        const int nx = B.nx, np = B.npad, y0 = td.y, x0 = td.z;
+        const int th = tile_rows(td), tw = tile_cols(td);
+        int lx0, lx1, ly0, ly1;
+        region_of<OPX>(x0, x0 + tw, nx, lx0, lx1);
+        region_of<OPY>(y0, y0 + th, B.ny, ly0, ly1);
+        const T* q = A.u_in + B.q_off;
+        const T* mt = A.met + B.m_off;
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int r = warp; r < ly1 - ly0; r += kStageThreads / 32) {
+            const int off = (ly0 + r) * nx;
+            {
+                const int e = ((off + lx0) & ~(AL - 1)) + lane * AL;
+                if (e < off + lx1) {
+#pragma unroll
+                    for (int pl = 0; pl < 4; ++pl) cp_async16(rq + (pl * RH + r) * RP + lane * AL, q + pl * np + e);
+                    const int tr = ly0 + r - y0;
+                    if (tr >= 0 && tr < th) {
+#pragma unroll
+                        for (int pl = 0; pl < 2; ++pl)
+                            cp_async16(rx + (pl * TY + tr) * RP + lane * AL, mt + (1 + pl) * np + e);
+                    }
+                }
+            }
+            const int e = ((off + x0) & ~(AL - 1)) + lane * AL;
+            if (e < off + x0 + tw) {
+#pragma unroll
+                for (int pl = 0; pl < 2; ++pl) cp_async16(re + (pl * RH + r) * EP + lane * AL, mt + (3 + pl) * np + e);
+            }
+        }
+    };
+    static_assert(RP <= 32 * AL && EP <= 32 * AL, "one 16-byte piece per lane");
+
+    if (blockIdx.x < A.ntiles) fetch(A.tiles[blockIdx.x]);
 
     for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
         const int4 td = A.tiles[t];
         const BlockDev& B = A.blocks[td.x];
         const int nx = B.nx, ny = B.ny;
-        const int64_t np = B.npad;
+        const int np = B.npad;  // in-block offsets fit 32 bits (checked when the system is built)
         const int y0 = td.y, x0 = td.z;
         const int th = tile_rows(td), tw = tile_cols(td);
         const int y1 = y0 + th, x1 = x0 + tw;
@@ -775,165 +818,220 @@ __global__ void __launch_bounds__(kStageThreads, 2) stage_kernel(const StageArgs
         region_of<OPX>(x0, x1, nx, lx0, lx1);
         region_of<OPY>(y0, y1, ny, ly0, ly1);
         // Everything later phases need from the block and instance descriptors is read here,
-        // once: the global stores of phase 2 would otherwise force the compiler to reload it.
-        const int64_t qoff = B.q_off, eoff = B.e_off;
-        const T* q = A.u_in + qoff;
-        const T* mt = A.met + B.m_off;
+        // once: the global stores of the update would otherwise force the compiler to reload it.
+        const int64_t qoff = B.q_off, eoff = B.e_off, roff = B.r_off;
         const InstanceDev& I = A.inst[B.instance];
-        const double cb = A.stage < 4 ? I.cb[A.stage] : 0.0;
-        const double ca = A.stage < 3 ? I.ca[A.stage] : 0.0;
-
-        // ---------------- phase 1: pointwise quantities ----------------
-        // Stage this thread's phase-2 operands (1 / J, RK state) into shared memory; the copies
-        // run while phase 1 computes.
-        if constexpr (COMP) {
-            const int pr0 = y0 + warp * R, prn = min(R, y1 - pr0);
-            if (lane < tw) {
-                const T* src[3];
-                const int nsrc = stage_operands<T>(A, src);
-#pragma unroll
-                for (int u = 0; u < R; ++u)
-                    if (u < prn) {
-                        const int ty = pr0 - y0 + u;
-                        const int pt = (pr0 + u) * nx + x0 + lane;
-                        T* slot = sR + ty * kTileX + lane;
-                        cp_async_elem(slot, mt + pt);
-                        for (int a = 0; a < nsrc; ++a)
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc)
-                                cp_async_elem(slot + (1 + 4 * a + cc) * TY * kTileX, src[a] + qoff + cc * np + pt);
-                    }
-            }
+        const T cb = T(A.stage < 4 ? I.cb[A.stage] : 0.0);
+        const T ca = T(A.stage < 3 ? I.ca[A.stage] : 0.0);
+        // the f64 sums still lack the spacing factors (the f32 metrics carry them)
+        const T fx = COMP ? T(1) : T(B.idx_xi), fy = COMP ? T(1) : T(B.idx_eta);
+        // The tile list gives every closure column of a block row to its first or its last tile
+        // and no tile both (tile_starts), and likewise for rows.
+        const bool left_cl = x0 < MX, right_cl = x1 > nx - MX;
+        const bool top_cl = y0 < MY, bot_cl = y1 > ny - MY;
+        if ((left_cl && right_cl) || (top_cl && bot_cl)) {  // a tile list not made by tile_starts
+            if (tid == 0) atomicOr(A.status, STATUS_BAD_LAUNCH);
+            return;
         }
-
-        // One index space over all threads: eta-region points (rows ly0..ly1, 32 slots per row,
-        // slots >= tw idle) followed by the xi-halo points (tile rows x hw columns, packed).
-        // A thread takes points p = tid, tid + 256, ... in batches of P1B: all loads of a batch
-        // are issued before any of its points is evaluated, so a thread waits for memory once
-        // per batch rather than once per point.
-        const int eh = ly1 - ly0;
-        const int hl = x0 - lx0, hw = hl + (lx1 - x1);
-        const int n_eta = eh * kTileX, n_all = n_eta + th * hw;
-        const unsigned hw_inv = hw ? (65536u + hw - 1) / hw : 0u;  // exact floor(h / hw) for h < 1024
-        for (int pb = threadIdx.x; pb < n_all; pb += P1B * kStageThreads) {
-            int pt[P1B], oxi[P1B], oeta[P1B];  // point, xi slot (-1: none), eta slot (-1: none)
-            T qv[P1B][4], m[P1B][4];
-#pragma unroll
-            for (int b = 0; b < P1B; ++b) {
-                const int p = pb + b * kStageThreads;
-                pt[b] = -1;
-                oxi[b] = -1;
-                oeta[b] = -1;
-                if (p < n_eta) {
-                    const int row = ly0 + (p >> 5), tx = p & 31;
-                    if (tx < tw) {
-                        const int col = x0 + tx;
-                        pt[b] = row * nx + col;
-                        oeta[b] = (row - ly0) * kTileX + tx;
-                        if (row >= y0 && row < y1) oxi[b] = (row - y0) * XP + (col - lx0);
-                    }
-                } else if (p < n_all) {
-                    const int h = p - n_eta;
-                    const int ty = (int)(((unsigned)h * hw_inv) >> 16);
-                    const int hc = h - ty * hw;
-                    const int col = hc < hl ? lx0 + hc : x1 + (hc - hl);
-                    pt[b] = (y0 + ty) * nx + col;
-                    oxi[b] = ty * XP + (col - lx0);
-                }
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    qv[b][cc] = T(1);
-                    m[b][cc] = T(0);
-                }
-                if (pt[b] >= 0) {
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) qv[b][cc] = __ldg(q + cc * np + pt[b]);
-                    if (oxi[b] >= 0) {
-                        m[b][0] = __ldg(mt + np + pt[b]);
-                        m[b][1] = __ldg(mt + 2 * np + pt[b]);
-                    }
-                    if (oeta[b] >= 0) {
-                        m[b][2] = __ldg(mt + 3 * np + pt[b]);
-                        m[b][3] = __ldg(mt + 4 * np + pt[b]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < P1B; ++b)
-                if (pt[b] >= 0) {
-                    if constexpr (COMP)
-                        pointwise_dev<UPW>(qv[b], m[b], gamma, I.ref, sE + (oxi[b] >= 0 ? oxi[b] : 0), XA,
-                                           sF + (oeta[b] >= 0 ? oeta[b] : 0), YA, oxi[b] >= 0, oeta[b] >= 0, bad);
-                    else
-                        pointwise<T, UPW, true>(qv[b], m[b], gamma, sE + (oxi[b] >= 0 ? oxi[b] : 0), XA,
-                                                sF + (oeta[b] >= 0 ? oeta[b] : 0), YA, oxi[b] >= 0, oeta[b] >= 0,
-                                                bad);
-                }
-        }
-        if constexpr (COMP) cp_async_wait_all();
+        const bool xi_pre = left_cl || right_cl, eta_pre = top_cl || bot_cl;
+        cp_async_wait_all();
         __syncthreads();
 
-        // ---------------- phase 2: stencils and stage update ----------------
-        // Interior points finish component by component (k_c, then the RK update of c); points
-        // on a block edge store k_c for the edge kernel.
-        const int r0 = y0 + warp * R;  // first global row of this thread
-        const int nrows = min(R, y1 - r0);
-        if (lane < tw && nrows > 0) {
-            const int col = x0 + lane;
-            // the compensated form's f32 metrics carry the spacing factors already
-            const T idxx = COMP ? T(1) : (sizeof(T) == 8 ? T(B.idx_xi) : T(B.idx_xi_f));
-            const T idxy = COMP ? T(1) : (sizeof(T) == 8 ? T(B.idx_eta) : T(B.idx_eta_f));
-            const bool fused = col < (sizeof(T) == 8 ? B.simd_f64 : B.simd_f32);
-            const bool eta_interior = r0 >= OpShape<OPY>::M && r0 + R <= ny - OpShape<OPY>::M;
-            const bool edge_col = col == 0 || col == nx - 1;
-            const bool xi_closure = x0 < OpShape<OPX>::M || x1 > nx - OpShape<OPX>::M;
-            const float cbf = float(cb), caf = float(ca);
-            // metrics plane 0: J in f64 (the reference divides by it), 1 / J in the f32 metrics
-            T jac[R];
-#pragma unroll
-            for (int u = 0; u < R; ++u) {
-                if constexpr (COMP) jac[u] = u < nrows ? sR[(r0 - y0 + u) * kTileX + lane] : T(1);
-                else jac[u] = u < nrows ? __ldg(mt + (r0 + u) * nx + col) : T(1);
+        // ---------------- xi fluxes of the tile rows, widened by the xi halo ----------------
+        {
+            const int cw = lx1 - lx0;
+            const unsigned inv = (65536u + cw - 1) / cw;  // exact floor(p / cw) for p * cw < 65536
+            for (int p = tid; p < th * cw; p += kStageThreads) {
+                const int r = (int)(((unsigned)p * inv) >> 16), c = p - r * cw;
+                const int a = (((y0 + r) * nx + lx0) & (AL - 1)) + c;
+                const T* s = rq + (y0 - ly0 + r) * RP + a;
+                const T* m = rx + r * RP + a;
+                const T qv[4] = {s[0], s[RH * RP], s[2 * RH * RP], s[3 * RH * RP]};
+                T* o = fl + r * G::XP + G::xpos(lx0 + c - x0 + G::XL);
+                if constexpr (COMP) {
+                    const T mm[4] = {m[0], m[TY * RP], T(0), T(0)};
+                    pointwise_dev<UPW>(qv, mm, gamma, I.ref, o, XA, o, XA, true, false, bad);
+                } else {
+                    pointwise<UPW>(qv, m[0], m[TY * RP], gamma, o, XA, bad);
+                }
             }
-            T ex[4][R], dx[4][R];
-            xi_rows<OPX, DIFF, T, R, !COMP, XA, XP>(sE, r0 - y0, nrows, lx0, col, nx, idxx, xi_closure, A.coef, ex);
-            if constexpr (UPW)
-                xi_rows<OPX, DISS, T, R, !COMP, XA, XP>(sE + 4 * XA, r0 - y0, nrows, lx0, col, nx, idxx, xi_closure,
-                                                        A.coef, dx);
+        }
+        __syncthreads();
+
+        // the next tile, its block descriptor brought near for fetch
+        const int tn = t + (int)gridDim.x;
+        int4 ntd = make_int4(0, 0, 0, 0);
+        if (tn < A.ntiles) {
+            ntd = A.tiles[tn];
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.blocks + ntd.x));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(A.blocks + ntd.x) + 128));
+        }
+        // ---------------- xi sums ----------------
+        // Thread (comp, gy, gx): component comp at rows y0 + gy MR .., columns x0 + gx MC ...  In a
+        // tile with closure columns every thread runs the interior path, and the closure outputs
+        // (diss - diff, all threads, compile-time coefficients) then replace its result through the
+        // flux buffer.
+        T ax[MR][MC], ay[MR][MC];
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                T dF[R];
-                eta_rows<OPY, DIFF, T, R, !COMP>(sF + cc * YA + lane, ly0, r0, nrows, ny, eta_interior, fused, idxy,
-                                                 A.coef, dF);
-                T ay[R];
-                if constexpr (UPW)
-                    eta_rows<OPY, DISS, T, R, !COMP>(sF + (4 + cc) * YA + lane, ly0, r0, nrows, ny, eta_interior,
-                                                     fused, idxy, A.coef, ay);
+        for (int u = 0; u < MR; ++u)
 #pragma unroll
-                for (int u = 0; u < R; ++u) {
-                    if (u < nrows) {
-                        const int row = r0 + u;
-                        T kc;
-                        if constexpr (UPW) kc = -ex[cc][u] - dF[u] + dx[cc][u] + ay[u];
-                        else kc = -ex[cc][u] - dF[u];
-                        if constexpr (COMP) kc = kc * jac[u];
-                        else kc = kc / jac[u];
-                        if constexpr (COMP && UPW)
-                            kc = kc + I.ref.q[cc] * __ldg(A.rinf + B.r_off + (int64_t)row * nx + col);
-                        if (edge_col || row == 0 || row == ny - 1)
-                            A.kedge[4 * (eoff + edge_index(row, col, nx, ny)) + cc] = kc;
-                        else if constexpr (COMP)
-                            rk_update_staged<T>(A, qoff + cc * np + row * nx + col, cbf, caf, kc, [&](int a) {
-                                return sR[((1 + 4 * a + cc) * TY + row - y0) * kTileX + lane];
-                            });
-                        else
-                            rk_update<T, COMP>(A, qoff + cc * np + row * nx + col, q[cc * np + row * nx + col], kc,
-                                               cb, ca);
+            for (int j = 0; j < MC; ++j) ax[u][j] = ay[u][j] = T(0);
+        const int r0 = gy * MR, c0 = gx * MC;
+        const bool active = c0 < tw && r0 < th;
+        if (active) {
+            const T* xr = fl + comp * XA + r0 * G::XP;
+            xi_sums<OPX, DIFF, -1, G>(xr, gx, ax);
+            if constexpr (UPW) xi_sums<OPX, DISS, 1, G>(xr + 4 * XA, gx, ax);
+        }
+        if (xi_pre) {
+            constexpr int PARTS = kStageThreads / (4 * TY), CNT = MX >= PARTS ? MX / PARTS : 1;
+            const int r = tid % TY, cc = (tid / TY) & 3, part = tid / (4 * TY);
+            T o[CNT];
+            const bool own = r < th && part * CNT < MX;
+            if (own) {
+                const int lc = (right_cl ? nx - OpShape<OPX>::N : 0) - x0 + G::XL;
+                const T* e = fl + cc * XA + r * G::XP;
+                auto ld = [&](int kind, int k) { return e[(kind == DISS ? 4 * XA : 0) + G::xpos(lc + k)]; };
+                if (right_cl) closure_part<OPX, UPW, true, PARTS, 0>(part, ld, o);
+                else closure_part<OPX, UPW, false, PARTS, 0>(part, ld, o);
+            }
+            __syncthreads();
+            if (own) {
+#pragma unroll
+                for (int i = 0; i < CNT; ++i) fl[(cc * MX + part * CNT + i) * TY + r] = o[i];
+            }
+            __syncthreads();
+            if (active) {
+#pragma unroll
+                for (int j = 0; j < MC; ++j) {
+                    const int ci = x0 + c0 + j - (left_cl ? 0 : nx - MX);
+                    if (ci >= 0 && ci < MX) {
+#pragma unroll
+                        for (int u = 0; u < MR; ++u) ax[u][j] = fl[(comp * MX + ci) * TY + r0 + u];
                     }
                 }
             }
         }
-        // Every thread is done with this tile's shared arrays before the next tile's phase 1.
+        __syncthreads();
+
+        // ---------------- eta fluxes of the tile columns, widened by the eta halo ----------------
+        for (int p = tid; p < (ly1 - ly0) * TX; p += kStageThreads) {
+            const int r = p / TX, c = p % TX;
+            if (c < tw) {
+                const int off = (ly0 + r) * nx;
+                const T* s = rq + r * RP + ((off + lx0) & (AL - 1)) + (x0 - lx0) + c;
+                const T* m = re + r * EP + ((off + x0) & (AL - 1)) + c;
+                const T qv[4] = {s[0], s[RH * RP], s[2 * RH * RP], s[3 * RH * RP]};
+                T* o = fl + (ly0 + r - y0 + G::YL) * TX + G::epos(c);
+                if constexpr (COMP) {
+                    const T mm[4] = {T(0), T(0), m[0], m[RH * EP]};
+                    pointwise_dev<UPW>(qv, mm, gamma, I.ref, o, YA, o, YA, false, true, bad);
+                } else {
+                    pointwise<UPW>(qv, m[0], m[RH * EP], gamma, o, YA, bad);
+                }
+            }
+        }
+        __syncthreads();
+        // the raw rows are no longer needed: the next tile's copies run from here on
+        if (tn < A.ntiles) fetch(ntd);
+
+        // Operands of the update pass for this thread's points (coalesced: consecutive threads take
+        // consecutive columns), loaded before the eta sums so that their latency is hidden:
+        // 1 / J, the free-stream plane, and up to three state arrays.
+        constexpr int NOP = COMP ? 3 : 2;
+        T jinv[PPT], rv[PPT], op[NOP][PPT][CPT];
+        int pe[PPT];  // element of the point in a plane (-1: not in the tile)
+        const int uc = PTS >= kStageThreads ? 0 : (tid / PTS) * CPT;  // first component
+        const T* src[3] = {A.stage == 0 ? A.u_in + qoff : A.acc_hi + qoff, A.prev_hi + qoff, A.prev_lo + qoff};
+        const int nsrc = A.stage == kStageK ? 0 : (A.stage == 0 ? 1 : (A.stage < 3 ? 2 : (COMP ? 3 : 1)));
+        const T* ji = COMP ? A.met + B.m_off : A.jinv + roff;
+        // ---------------- eta sums ----------------
+        if (active) {
+            const T* ec = fl + comp * YA + (r0 + G::YL - HY) * TX;
+            eta_sums<OPY, DIFF, -1, G, 0>(ec, gx, ay);
+            if constexpr (UPW) eta_sums<OPY, DISS, 1, G, 0>(ec + 4 * YA, gx, ay);
+        }
+        if (eta_pre) {
+            constexpr int PARTS = kStageThreads / (4 * TX), CNT = MY >= PARTS ? MY / PARTS : 1;
+            const int col = tid % TX, cc = (tid / TX) & 3, part = tid / (4 * TX);
+            T o[CNT];
+            const bool own = col < tw && part * CNT < MY;
+            if (own) {
+                const int lr = (bot_cl ? ny - OpShape<OPY>::N : 0) - y0 + G::YL;
+                const T* f = fl + cc * YA + lr * TX + G::epos(col);
+                auto ld = [&](int kind, int k) { return f[(kind == DISS ? 4 * YA : 0) + k * TX]; };
+                if (bot_cl) closure_part<OPY, UPW, true, PARTS, 0>(part, ld, o);
+                else closure_part<OPY, UPW, false, PARTS, 0>(part, ld, o);
+            }
+            __syncthreads();
+            if (own) {
+#pragma unroll
+                for (int i = 0; i < CNT; ++i) fl[(cc * MY + part * CNT + i) * TX + col] = o[i];
+            }
+            __syncthreads();
+            if (active) {
+#pragma unroll
+                for (int u = 0; u < MR; ++u) {
+                    const int ri = y0 + r0 + u - (top_cl ? 0 : ny - MY);
+                    if (ri >= 0 && ri < MY) {
+#pragma unroll
+                        for (int j = 0; j < MC; ++j) ay[u][j] = fl[(comp * MY + ri) * TX + c0 + j];
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // the sums through shared memory to the update pass
+        if (active) {
+#pragma unroll
+            for (int u = 0; u < MR; ++u) {
+                T s[MC];
+#pragma unroll
+                for (int j = 0; j < MC; ++j)
+                    s[j] = COMP ? ax[u][j] + ay[u][j] : fma_rn(ax[u][j], fx, ay[u][j] * fy);
+                V* o = reinterpret_cast<V*>(fl + comp * PTS + (r0 + u) * TX);
+                o[gx] = {s[0], s[1]};
+                if constexpr (MC == 4) o[TX / 4 + (gx ^ 4)] = {s[2], s[3]};
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            const int p = tid % (PTS < kStageThreads ? PTS : kStageThreads) + i * kStageThreads;
+            const int ur = p / TX, ux = p % TX;
+            pe[i] = ur < th && ux < tw ? (y0 + ur) * nx + x0 + ux : -1;
+            jinv[i] = T(1);
+            rv[i] = T(0);
+            if (pe[i] >= 0) {
+                jinv[i] = __ldg(ji + pe[i]);
+                if constexpr (COMP && UPW) rv[i] = __ldg(A.rinf + roff + pe[i]);
+#pragma unroll
+                for (int a = 0; a < NOP; ++a)
+#pragma unroll
+                    for (int cc = 0; cc < CPT; ++cc)
+                        op[a][i][cc] = a < nsrc ? src[a][(uc + cc) * np + pe[i]] : T(0);
+            }
+        }
+        __syncthreads();
+
+        // ---------------- update pass ----------------
+        // Interior points finish; points on a block edge store k for the edge kernel.
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            if (pe[i] < 0) continue;
+            const int p = tid % (PTS < kStageThreads ? PTS : kStageThreads) + i * kStageThreads;
+            const int ur = p / TX, ux = p % TX;
+            const int row = y0 + ur, col = x0 + ux;
+            const bool edge = row == 0 || row == ny - 1 || col == 0 || col == nx - 1;
+#pragma unroll
+            for (int cc = 0; cc < CPT; ++cc) {
+                T k = fl[(uc + cc) * PTS + ur * TX + G::epos(ux)] * jinv[i];
+                if constexpr (COMP && UPW) k = fma_rn(I.ref.q[uc + cc], rv[i], k);
+                const int64_t e = qoff + (uc + cc) * np + pe[i];
+                if (edge) A.kedge[4 * (eoff + edge_index(row, col, nx, ny)) + uc + cc] = k;
+                else rk_update_ops<T, COMP>(A, e, cb, ca, k, op[0][i][cc], op[1][i][cc], COMP ? op[NOP - 1][i][cc] : T(0));
+            }
+        }
+        // Every thread is done with the flux buffer before the next tile's fluxes.
         __syncthreads();
     }
     if (bad) atomicOr(A.status, bad);

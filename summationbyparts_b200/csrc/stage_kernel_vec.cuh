@@ -64,11 +64,11 @@ struct PairTaps {
         if constexpr (I <= D) {
             const float2 v = ld(I);
             if constexpr (I < D) {
-                constexpr float c = CDiag<OP, KIND>::v[I];
+                constexpr float c = CDiag<OP, KIND, float>::v[I];
                 if constexpr (c != 0.0f) a0 = ffma2(v, c, a0);
             }
             if constexpr (I >= 1) {
-                constexpr float c = CDiag<OP, KIND>::v[I - 1];
+                constexpr float c = CDiag<OP, KIND, float>::v[I - 1];
                 if constexpr (c != 0.0f) a1 = ffma2(v, c, a1);
             }
             PairTaps<OP, KIND, I + 1, D>::run(ld, a0, a1);
@@ -114,38 +114,6 @@ constexpr size_t vec_stage_smem(bool upw) {
                             closure_eta_elems(OpShape<OPY>::M));
 }
 
-// Closure-block coefficient (row I, input K) of one end of a line: the start block, or the end
-// block (row I applies -/+ st[(M - 1 - I) N + (N - 1 - K)], DIFF negated).
-template <int OP, int KIND, bool RIGHT, int I, int K>
-struct ClosureCoef {
-    static constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N;
-    static constexpr float value = RIGHT ? (KIND == DIFF ? -1.0f : 1.0f) * CDiag<OP, KIND>::st[(M - 1 - I) * N + (N - 1 - K)]
-                                         : CDiag<OP, KIND>::st[I * N + K];
-};
-// Rows I.. of the closure block: the sum over the N inputs v, first product then an fma chain
-// (the table path's order).
-template <int OP, int KIND, bool RIGHT, int I, int K = 1>
-__device__ __forceinline__ float closure_sum(const float* v, float t) {
-    if constexpr (K == 1) t = v[0] * ClosureCoef<OP, KIND, RIGHT, I, 0>::value;
-    if constexpr (K < OpShape<OP>::N) {
-        constexpr float c = ClosureCoef<OP, KIND, RIGHT, I, K>::value;
-        return closure_sum<OP, KIND, RIGHT, I, K + 1>(v, __fmaf_rn(v[K], c, t));
-    } else {
-        return t;
-    }
-}
-
-// Writes closure columns I .. I + CNT - 1 of closure_xi.
-template <int OP, bool UPW, bool RIGHT, int I, int CNT, int PITCH = kClosurePitch>
-__device__ __forceinline__ void closure_out(const float* ve, const float* va, float* cb) {
-    if constexpr (CNT > 0) {
-        float d = 0.0f;
-        if constexpr (UPW) d = closure_sum<OP, DISS, RIGHT, I>(va, 0.0f);
-        cb[I * PITCH] = d - closure_sum<OP, DIFF, RIGHT, I>(ve, 0.0f);
-        closure_out<OP, UPW, RIGHT, I + 1, CNT - 1, PITCH>(ve, va, cb);
-    }
-}
-
 // The xi term diss_xi(alpha_u q) - diff_xi(Ehat) of closure columns I0 .. I0 + CNT - 1 at one end
 // of a line, for one component and tile row: e / a are the transposed Ehat / alpha_u q arrays at
 // the row, `lc` the local column of the block's first input (the inputs carry the spacing
@@ -162,7 +130,7 @@ __device__ __forceinline__ void closure_xi(const float* __restrict__ e, const fl
         ve[k] = e[o];
         va[k] = UPW ? a[o] : 0.0f;
     }
-    closure_out<OP, UPW, RIGHT, I0, CNT>(ve, va, cb);
+    closure_out<OP, UPW, RIGHT, I0, CNT>(ve, va, [&](int i, float t) { cb[i * kClosurePitch] = t; });
 }
 
 // The eta term diss_eta(alpha_v q) - diff_eta(Fhat) of closure rows I0 .. I0 + CNT - 1 at one
@@ -179,7 +147,7 @@ __device__ __forceinline__ void closure_eta(const float* __restrict__ f, const f
         ve[k] = f[(lr + k) * kTileX];
         va[k] = UPW ? a[(lr + k) * kTileX] : 0.0f;
     }
-    closure_out<OP, UPW, BOTTOM, I0, CNT, kTileX>(ve, va, cb);
+    closure_out<OP, UPW, BOTTOM, I0, CNT>(ve, va, [&](int i, float t) { cb[i * kTileX] = t; });
 }
 
 // The two values of a thread's row u at columns c0, c0 + 1 from `p` (the element of (r0, c0)).

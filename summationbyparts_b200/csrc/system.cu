@@ -28,7 +28,6 @@
 
 namespace sbp {
 const double* op_h_weights(int op);
-void fill_coef_table(int prec, void* out, int stride, int row);
 
 const void* stage_kernel_ptr(int prec, int opx, int opy, bool upw, int ty, int sc) {
     using F = const void* (*)(int, int, bool, int, int);
@@ -66,7 +65,7 @@ constexpr int64_t kMaxBlockPoints = (int64_t)1 << 28;
 // The compensated-f32 kernel of 32-row tiles is the 2 x 2 micro-tile kernel (stage_kernel_vec).
 bool vec_kernel(int prec, int ty) { return prec == 1 && ty == kVecRows; }
 
-// Shared memory of one stage-kernel CTA (mirrors StageGeom in stage_kernel.cuh and VecGeom in
+// Shared memory of one stage-kernel CTA (tile_smem in stage_kernel.cuh, VecGeom in
 // stage_kernel_vec.cuh).
 size_t stage_smem_host(int prec, int opx, int opy, bool upw, int ty) {
     OpInfo ox, oy;
@@ -79,11 +78,7 @@ size_t stage_smem_host(int prec, int opx, int opy, bool upw, int ty) {
                ((size_t)(4 * 2 * ((xc + 1) / 2) * kVecPitch + 4 * hyp * kTileX) * (upw ? 2 : 1) + closure_xi_elems(ox.M) +
                 closure_eta_elems(oy.M));
     }
-    const int xp = region_extent(kTileX, (ox.D - 1) / 2, ox.M, ox.N);
-    const int hyp = region_extent(ty, (oy.D - 1) / 2, oy.M, oy.N);
-    const size_t elems =
-        (size_t)(4 * ty * xp + 4 * hyp * kTileX) * (upw ? 2 : 1) + staged_elems(prec == 1, ty);
-    return elems * (prec == 0 ? sizeof(double) : sizeof(float));
+    return (size_t)tile_smem(ty, upw, prec == 0 ? 8 : 4, (ox.D - 1) / 2, ox.M, ox.N, (oy.D - 1) / 2, oy.M, oy.N);
 }
 
 struct Group {
@@ -149,6 +144,7 @@ struct sbp_system {
     void *prev_hi = nullptr, *prev_lo = nullptr, *acc_hi = nullptr, *acc_lo = nullptr, *uA = nullptr, *uB = nullptr;
     double* met64 = nullptr;
     float* met32 = nullptr;
+    double* jinv64 = nullptr;  // f64: 1 / J planes (BlockDev::r_off)
     float* rinf = nullptr;  // compensated f32: free-stream dissipation planes (BlockDev::r_off)
     double* xy = nullptr;
     double* hw = nullptr;
@@ -162,7 +158,6 @@ struct sbp_system {
     unsigned* status = nullptr;
     double* d_sums = nullptr;
     unsigned long long* d_speeds = nullptr;
-    void* d_coef = nullptr;  // stage-kernel coefficient table in the state precision
     void* kedge = nullptr;   // k of block-edge points between the stage and the edge kernel
     double* egeo = nullptr;   // compensated f32: edge geometry (kEdgeGeo per point, edge_geo_kernel)
     int64_t nedge = 0;
@@ -234,7 +229,7 @@ void destroy_all(sbp_system* s) {
     void* ptrs[] = {s->d_blocks, s->d_inst, s->d_active, s->prev_hi, s->prev_lo, s->acc_hi, s->acc_lo,
                     s->uA,       s->uB,     s->met64,    s->met32,   s->xy,      s->hw,      s->d_hoff,
                     s->d_poff4,  s->d_poff8, s->d_zero,  s->staging, s->status,  s->d_sums,  s->d_speeds,
-                    s->d_coef,   s->kedge,  s->d_mg,     s->kbuf,    s->d_eval,  s->rinf,    s->egeo};
+                    s->jinv64,   s->kedge,  s->d_mg,     s->kbuf,    s->d_eval,  s->rinf,    s->egeo};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (auto st : s->side) cudaStreamDestroy(st);
@@ -344,10 +339,10 @@ StageArgs<T> stage_args(sbp_system* s, int stage, const Group& g) {
     a.new_hi = prev;
     a.new_lo = static_cast<T*>(s->prev_lo);
     a.met = s->prec == 0 ? reinterpret_cast<const T*>(s->met64) : reinterpret_cast<const T*>(s->met32);
+    a.jinv = s->prec == 0 ? reinterpret_cast<const T*>(s->jinv64) : nullptr;
     a.met64 = s->met64;
     a.rinf = s->rinf;
     a.xy = s->xy;
-    a.coef = static_cast<const T*>(s->d_coef);
     a.kedge = static_cast<T*>(s->kedge);
     a.egeo = s->egeo;
     a.mg = s->d_mg;
@@ -980,8 +975,6 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
         B.op_xi = D.op_xi;
         B.op_eta = D.op_eta;
         B.instance = D.instance;
-        B.simd_f64 = (int)(8 * (D.nx / 8));
-        B.simd_f32 = (int)(16 * (D.nx / 16));
         for (int d = 0; d < 4; ++d) {
             B.bc_kind[d] = D.bc_kind[d];
             if (D.bc_kind[d] == SBP_BC_EVAL) s->has_eval = true;
@@ -1006,8 +999,6 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
         s->nx2 += 2 * (int64_t)B.npad;
         B.idx_xi = inv_spacing<double>(ox.h2, D.nx);
         B.idx_eta = inv_spacing<double>(oy.h2, D.ny);
-        B.idx_xi_f = inv_spacing<float>(ox.h2, D.nx);
-        B.idx_eta_f = inv_spacing<float>(oy.h2, D.ny);
         // SAT_north/.. penalties: (n-1)/H_0, or (n-2)/H_0 for h2 (euler/src/lib.rs:1033-1037, 1093-1097)
         B.hi_eta = (oy.h2 ? double(D.ny - 2) : double(D.ny - 1)) / op_h_weights(D.op_eta)[0];
         B.hi_xi = (ox.h2 ? double(D.nx - 2) : double(D.nx - 1)) / op_h_weights(D.op_xi)[0];
@@ -1041,6 +1032,8 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
         e = e ?: alloc(&s->prev_lo, s->nq * ts);
         e = e ?: alloc((void**)&s->met32, s->nm * sizeof(float));
         e = e ?: alloc((void**)&s->rinf, (s->nq / 4) * sizeof(float));
+    } else {
+        e = e ?: alloc((void**)&s->jinv64, (s->nq / 4) * sizeof(double));
     }
     e = e ?: alloc((void**)&s->met64, s->nm * sizeof(double));
     e = e ?: alloc((void**)&s->xy, s->nx2 * sizeof(double));
@@ -1055,7 +1048,6 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
     // per-block norms, then kNormParts partial sums per block (error_terms / diff_terms)
     e = e ?: alloc((void**)&s->d_sums, (size_t)nblocks * (1 + kNormParts) * sizeof(double));
     e = e ?: alloc((void**)&s->d_speeds, 2 * nblocks * sizeof(unsigned long long));
-    e = e ?: alloc(&s->d_coef, 12 * kCoefStride * ts);
     e = e ?: alloc(&s->kedge, 4 * s->nedge * ts);
     if (s->prec == 1) {
         e = e ?: alloc((void**)&s->egeo, kEdgeGeo * s->nedge * sizeof(double));
@@ -1077,9 +1069,6 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
     e = e ?: cudaMemcpyAsync(s->d_hoff, s->hoff.data(), nblocks * sizeof(int64_t), cudaMemcpyHostToDevice, st);
     if (!mg_host.empty())
         e = e ?: cudaMemcpyAsync(s->d_mg, mg_host.data(), mg_host.size() * sizeof(int4), cudaMemcpyHostToDevice, st);
-    std::vector<double> coef_host(12 * kCoefStride);  // large enough for either precision
-    fill_coef_table(s->prec, coef_host.data(), kCoefStride, kCoefRow);
-    e = e ?: cudaMemcpyAsync(s->d_coef, coef_host.data(), 12 * kCoefStride * ts, cudaMemcpyHostToDevice, st);
     {
         std::vector<int64_t> p8(nblocks);
         for (int b = 0; b < nblocks; ++b) p8[b] = 2 * s->dense_off[b];
@@ -1134,6 +1123,8 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
         e = narrow_f32(s->met64, s->met32, s->nm, st);
         e = e ?: jacobian_inverse_f32(s->d_blocks, nblocks, s->met64, s->met32, s->max_points, st);
     }
+    if (e == cudaSuccess && s->jinv64)
+        e = jacobian_inverse_f64(s->d_blocks, nblocks, s->met64, s->jinv64, s->max_points, st);
     if (e != cudaSuccess) return fail(cuda_status(e, "metrics"));
     if (s->rinf) {
         // the state starts at zero: in the compensated form a deviation of -qref

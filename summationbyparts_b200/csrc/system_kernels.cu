@@ -295,6 +295,15 @@ cudaError_t narrow_f32(const double* in, float* out, int64_t n, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// 1 / J planes of the f64 stage kernel: it scales the flux divergence by a product.
+__global__ void jacobian_inverse_f64_kernel(const BlockDev* __restrict__ blocks, const double* __restrict__ met64,
+                                            double* __restrict__ jinv) {
+    const BlockDev& B = blocks[blockIdx.y];
+    const int64_t n = (int64_t)B.nx * B.ny;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        jinv[B.r_off + i] = 1.0 / met64[B.m_off + i];
+}
+
 // The single-precision metrics of the compensated stage kernels: plane 0 holds 1 / J (rounded
 // once from the f64 quotient), so the flux divergence is scaled by a product; planes 1-2 (J dxi/dx,
 // J dxi/dy) are multiplied by the block's xi spacing factor idx_xi and planes 3-4 by idx_eta (in
@@ -320,6 +329,12 @@ __global__ void jacobian_inverse_kernel(const BlockDev* __restrict__ blocks, con
 cudaError_t jacobian_inverse_f32(const BlockDev* blocks, int nblocks, const double* met64, float* met32,
                                  int64_t max_points, cudaStream_t st) {
     jacobian_inverse_kernel<<<per_block_grid(nblocks, max_points), kT, 0, st>>>(blocks, met64, met32);
+    return cudaGetLastError();
+}
+
+cudaError_t jacobian_inverse_f64(const BlockDev* blocks, int nblocks, const double* met64, double* jinv,
+                                 int64_t max_points, cudaStream_t st) {
+    jacobian_inverse_f64_kernel<<<per_block_grid(nblocks, max_points), kT, 0, st>>>(blocks, met64, jinv);
     return cudaGetLastError();
 }
 

@@ -20,6 +20,10 @@ cudaError_t narrow_f32(const double* in, float* out, int64_t n, cudaStream_t st)
 cudaError_t jacobian_inverse_f32(const BlockDev* blocks, int nblocks, const double* met64, float* met32,
                                  int64_t max_points, cudaStream_t st);
 
+// 1 / J of every block (plane 0 of its metrics) into the block's plane at r_off.
+cudaError_t jacobian_inverse_f64(const BlockDev* blocks, int nblocks, const double* met64, double* jinv,
+                                 int64_t max_points, cudaStream_t st);
+
 // Vortex initial data for every block whose instance is selected (instance < 0: all).
 // f64 state: q_hi only.  f32 state: (hi, lo) split of the f64 value.
 cudaError_t vortex_init(const BlockDev* blocks, const InstanceDev* inst, int nblocks, int instance, double gamma,
