@@ -26,7 +26,8 @@ constexpr int kDzP[kLayers] = {32, 32, 32, 32, 16};    // stored channels of eac
 
 // Elementwise kernels around the network ----------------------------------------------------
 
-// a0[n][p][c] = (state[n][c][p] - mean[c]) * inv[c] for c < 4, 0 for the 12 padding channels.
+// Chunk 0 of the network input: channels c < 4 = (state[n][c][p] - mean[c]) * inv[c], zeros above; chunk
+// 1 (padding) stays zero from the network's creation.
 template <class T>
 __global__ void pack_input_kernel(const T* __restrict__ st, int64_t img_stride, int n, float4 mean, float4 inv,
                                   __nv_bfloat16* __restrict__ a0) {
@@ -36,19 +37,12 @@ __global__ void pack_input_kernel(const T* __restrict__ st, int64_t img_stride, 
     const T* s = st + img * img_stride + p;
     const float v0 = (float(s[0]) - mean.x) * inv.x, v1 = (float(s[kPix]) - mean.y) * inv.y;
     const float v2 = (float(s[2 * kPix]) - mean.z) * inv.z, v3 = (float(s[3 * kPix]) - mean.w) * inv.w;
-    uint4 lo, hi = make_uint4(0u, 0u, 0u, 0u);
-    lo.x = pack_bf16(v0, v1);
-    lo.y = pack_bf16(v2, v3);
-    lo.z = 0u;
-    lo.w = 0u;
-    uint4* d = reinterpret_cast<uint4*>(a0 + i * 16);
-    d[0] = lo;
-    d[1] = hi;
+    reinterpret_cast<uint4*>(a0)[img * 2 * kPix + p] = make_uint4(pack_bf16(v0, v1), pack_bf16(v2, v3), 0u, 0u);
 }
 
 // Loss and output gradient: t = (fine_r - coarse) / out_scale per channel, the squared error
-// summed per CTA into part (CTA order), dy = 2 (y - t) / count into dz4 (16 channels, zeros
-// above 4).
+// summed per CTA into part (CTA order), dy = 2 (y - t) / count into chunk 0 of dz4 (chunk 1 stays
+// zero).
 template <class T>
 __global__ void loss_kernel(const float* __restrict__ y, const T* __restrict__ coarse, int64_t img_stride,
                             const double* __restrict__ fine_r, int n, float4 oscale, float inv_count,
@@ -69,14 +63,7 @@ __global__ void loss_kernel(const float* __restrict__ y, const T* __restrict__ c
             se += d * d;
             g[k] = 2.0f * d * inv_count;
         }
-        uint4 lo, hi = make_uint4(0u, 0u, 0u, 0u);
-        lo.x = pack_bf16(g[0], g[1]);
-        lo.y = pack_bf16(g[2], g[3]);
-        lo.z = 0u;
-        lo.w = 0u;
-        uint4* d = reinterpret_cast<uint4*>(dz4 + i * 16);
-        d[0] = lo;
-        d[1] = hi;
+        reinterpret_cast<uint4*>(dz4)[img * 2 * kPix + p] = make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), 0u, 0u);
     }
     red[threadIdx.x] = se;
     __syncthreads();
@@ -87,58 +74,48 @@ __global__ void loss_kernel(const float* __restrict__ y, const T* __restrict__ c
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// corrected[n][c][p] = coarse[n][c][p] + y[n][p][c] * out_scale[c]  (f64 output planes)
-template <class T>
-__global__ void apply_kernel(const float* __restrict__ y, const T* __restrict__ coarse, int64_t img_stride, int n,
-                             float4 oscale, double* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)n * kPix) return;
-    const int64_t img = i / kPix, p = i % kPix;
-    const T* c = coarse + img * img_stride + p;
-    double* o = out + img * 4 * kPix + p;
-    const float sc[4] = {oscale.x, oscale.y, oscale.z, oscale.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o[k * kPix] = double(c[k * kPix]) + double(y[i * 8 + k]) * double(sc[k]);
+// One layer's parameters: offset and size of its weights [cout][9][cin] (its cout biases follow), and the
+// bf16 weights of its convolution and of its gradient convolution (null for the first layer) in
+// conv_weight_index order.
+struct LayerParams {
+    int off, nw, cout, cin, dzp;  // dzp: stored channels of the layer's output gradient
+    __nv_bfloat16 *wb, *wt;
+};
+struct NetParams {
+    LayerParams l[5];
+};
+
+__device__ __forceinline__ void store_bf16_weight(const LayerParams& L, int e, float v) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    const int co = e / (9 * L.cin), tap = (e / L.cin) % 9, ci = e % L.cin;
+    L.wb[conv_weight_index(co, tap, ci, L.cin, L.cout < 16 ? 16 : L.cout)] = h;
+    if (L.wt) L.wt[conv_weight_index(ci, 8 - tap, co, L.dzp, L.cin)] = h;
 }
 
-// Adam (Kingma & Ba) on one layer's weights (nw elements, [cout][9][cin]) and biases (nb), with
-// the bias corrections c1 = 1 / (1 - beta1^t), c2 = 1 / (1 - beta2^t) from the host.  Writes the
-// bf16 weights and, when wt is given, the bf16 weights of the gradient convolution:
-// wt[ci][8 - tap][co] (dz channels dzp) = w[co][tap][ci].
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, int nw, int nb, float lr, float b1, float b2, float c1, float c2,
-                            float eps, int cout, int cin, int dzp, __nv_bfloat16* __restrict__ wb,
-                            __nv_bfloat16* __restrict__ wt) {
+// Adam (Kingma & Ba) on every layer (blockIdx.y), with the bias corrections c1 = 1 / (1 - beta1^t),
+// c2 = 1 / (1 - beta2^t) from the host; rewrites the bf16 weights.
+__global__ void adam_kernel(const NetParams N, float* __restrict__ P, const float* __restrict__ G,
+                            float* __restrict__ Mo, float* __restrict__ Ve, float lr, float b1, float b2, float c1,
+                            float c2, float eps) {
+    const LayerParams& L = N.l[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nw + nb) return;
-    const float ge = g[e];
-    const float me = b1 * m[e] + (1.0f - b1) * ge;
-    const float ve = b2 * v[e] + (1.0f - b2) * ge * ge;
-    m[e] = me;
-    v[e] = ve;
-    const float pe = p[e] - lr * (me * c1) / (sqrtf(ve * c2) + eps);
-    p[e] = pe;
-    if (e < nw) {
-        const __nv_bfloat16 h = __float2bfloat16_rn(pe);
-        wb[e] = h;
-        if (wt) {
-            const int co = e / (9 * cin), tap = (e / cin) % 9, ci = e % cin;
-            wt[((int64_t)ci * 9 + (8 - tap)) * dzp + co] = h;
-        }
-    }
+    if (e >= L.nw + L.cout) return;
+    const int i = L.off + e;
+    const float ge = G[i];
+    const float me = b1 * Mo[i] + (1.0f - b1) * ge;
+    const float ve = b2 * Ve[i] + (1.0f - b2) * ge * ge;
+    Mo[i] = me;
+    Ve[i] = ve;
+    const float pe = P[i] - lr * (me * c1) / (sqrtf(ve * c2) + eps);
+    P[i] = pe;
+    if (e < L.nw) store_bf16_weight(L, e, pe);
 }
 
 // bf16 copies of the parameters (after set_params)
-__global__ void weights_bf16_kernel(const float* __restrict__ p, int nw, int cout, int cin, int dzp,
-                                    __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wt) {
+__global__ void weights_bf16_kernel(const NetParams N, const float* __restrict__ P) {
+    const LayerParams& L = N.l[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nw) return;
-    const __nv_bfloat16 h = __float2bfloat16_rn(p[e]);
-    wb[e] = h;
-    if (wt) {
-        const int co = e / (9 * cin), tap = (e / cin) % 9, ci = e % cin;
-        wt[((int64_t)ci * 9 + (8 - tap)) * dzp + co] = h;
-    }
+    if (e < L.nw) store_bf16_weight(L, e, P[L.off + e]);
 }
 
 // Tensor-product restriction: out[n][c][i][j] = sum_a sum_b wy[i][a] wx[j][b] f[n][c][iy[i]+a][ix[j]+b]
@@ -231,8 +208,7 @@ struct sbp_cnn {
 namespace {
 
 template <int CIN, int COUT, int EPI>
-cudaError_t conv(const sbp_cnn* c, int n, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias,
-                 const float* zprev, float* zout, __nv_bfloat16* yout) {
+cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     constexpr int bytes = ConvTcLayout<CIN, COUT>::BYTES;
     static bool configured = false;  // per instantiation; the attribute is per function
     if (!configured) {
@@ -241,10 +217,19 @@ cudaError_t conv(const sbp_cnn* c, int n, const __nv_bfloat16* x, const __nv_bfl
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    conv3x3_tc_kernel<CIN, COUT, EPI><<<n * (kImg / kBand), kConvThreads, bytes, c->st()>>>(x, w, bias, zprev, zout,
-                                                                                            yout, c->status);
+    a.status = c->status;
+    conv3x3_tc_kernel<CIN, COUT, EPI><<<n * (kImg / kBand), kConvThreads, bytes, c->st()>>>(a);
     return cudaGetLastError();
 }
+
+NetParams net_params(const sbp_cnn* c) {
+    NetParams N;
+    for (int l = 0; l < kLayers; ++l)
+        N.l[l] = LayerParams{(int)c->w_off[l], (int)c->nw[l], kCoutP[l], kCinP[l], kDzP[l], c->Wb[l],
+                             l > 0 ? c->Wt[l] : nullptr};
+    return N;
+}
+constexpr int kMaxLayerParams = 32 * 9 * 32 + 32;
 
 // The device status word after the stream has drained: a tensor-core wait that gave up.
 sbp_status device_status(sbp_cnn* c) {
@@ -284,7 +269,10 @@ sbp_status check_batch(const sbp_cnn* c, int n) {
     return SBP_OK;
 }
 
-sbp_status forward(sbp_cnn* c, int n, const void* state, int dtype, int64_t img_stride) {
+// The network on n states.  keep_z: the pre-activations are written for a backward pass; out: the
+// output layer also writes the corrected states there.
+sbp_status forward(sbp_cnn* c, int n, const void* state, int dtype, int64_t img_stride, bool keep_z,
+                   double* out = nullptr) {
     const int64_t total = (int64_t)n * kPix;
     const int blocks = (int)((total + 255) / 256);
     if (dtype == SBP_F64)
@@ -294,13 +282,37 @@ sbp_status forward(sbp_cnn* c, int n, const void* state, int dtype, int64_t img_
         pack_input_kernel<float><<<blocks, 256, 0, c->st()>>>(static_cast<const float*>(state), img_stride, n,
                                                               c->in_mean, c->in_inv, c->a[0]);
     SBP_TRY_CUDA(cudaGetLastError());
-    const float* P = c->P;
-    SBP_TRY_CUDA((conv<16, 32, EPI_GELU>(c, n, c->a[0], c->Wb[0], P + c->b_off[0], nullptr, c->z[0], c->a[1])));
-    for (int l = 1; l < 4; ++l)
-        SBP_TRY_CUDA(
-            (conv<32, 32, EPI_GELU>(c, n, c->a[l], c->Wb[l], P + c->b_off[l], nullptr, c->z[l], c->a[l + 1])));
-    SBP_TRY_CUDA((conv<32, 8, EPI_LINEAR>(c, n, c->a[4], c->Wb[4], P + c->b_off[4], nullptr, c->y, nullptr)));
+    for (int l = 0; l < kLayers; ++l) {
+        ConvArgs a{};
+        a.x = c->a[l];
+        a.w = c->Wb[l];
+        a.bias = c->P + c->b_off[l];
+        if (l < kLayers - 1) {
+            a.zout = keep_z ? c->z[l] : nullptr;
+            a.yout = c->a[l + 1];
+            SBP_TRY_CUDA((l == 0 ? conv<16, 32, EPI_GELU>(c, n, a) : conv<32, 32, EPI_GELU>(c, n, a)));
+        } else {
+            a.zout = c->y;
+            a.coarse = state;
+            a.coarse_f64 = dtype == SBP_F64;
+            a.img_stride = img_stride;
+            a.oscale = c->out_scale;
+            a.out = out;
+            SBP_TRY_CUDA((out ? conv<32, 8, EPI_APPLY>(c, n, a) : conv<32, 8, EPI_LINEAR>(c, n, a)));
+        }
+    }
     return SBP_OK;
+}
+
+// Gradient of layer l's input through its transposed convolution: dz[l - 1] from dz[l].
+template <int DZ>
+cudaError_t conv_input_gradient(const sbp_cnn* c, int n, int l) {
+    ConvArgs a{};
+    a.x = c->dz[l];
+    a.w = c->Wt[l];
+    a.zprev = c->z[l - 1];
+    a.yout = c->dz[l - 1];
+    return conv<DZ, 32, EPI_DGELU>(c, n, a);
 }
 
 // Loss and gradients of all parameters into G; the loss (mean squared error of the normalised
@@ -318,10 +330,10 @@ sbp_status backward(sbp_cnn* c, int n, const void* coarse, int dtype, int64_t im
                                                         n, c->out_scale, inv_count, c->dz[4], c->part_loss);
     SBP_TRY_CUDA(cudaGetLastError());
     SBP_TRY_CUDA((wgrad<32, 16, 8>(c, n, 4, c->a[4], c->dz[4])));
-    SBP_TRY_CUDA((conv<16, 32, EPI_DGELU>(c, n, c->dz[4], c->Wt[4], nullptr, c->z[3], nullptr, c->dz[3])));
+    SBP_TRY_CUDA(conv_input_gradient<16>(c, n, 4));
     for (int l = 3; l >= 1; --l) {
         SBP_TRY_CUDA((wgrad<32, 32, 32>(c, n, l, c->a[l], c->dz[l])));
-        SBP_TRY_CUDA((conv<32, 32, EPI_DGELU>(c, n, c->dz[l], c->Wt[l], nullptr, c->z[l - 1], nullptr, c->dz[l - 1])));
+        SBP_TRY_CUDA(conv_input_gradient<32>(c, n, l));
     }
     SBP_TRY_CUDA((wgrad<16, 32, 32>(c, n, 0, c->a[0], c->dz[0])));
     if (loss) {
@@ -336,12 +348,8 @@ sbp_status backward(sbp_cnn* c, int n, const void* coarse, int dtype, int64_t im
 }
 
 sbp_status refresh_bf16(sbp_cnn* c) {
-    for (int l = 0; l < kLayers; ++l) {
-        const int nw = (int)c->nw[l];
-        weights_bf16_kernel<<<(nw + 255) / 256, 256, 0, c->st()>>>(c->P + c->w_off[l], nw, kCoutP[l], kCinP[l],
-                                                                  kDzP[l], c->Wb[l], l > 0 ? c->Wt[l] : nullptr);
-        SBP_TRY_CUDA(cudaGetLastError());
-    }
+    weights_bf16_kernel<<<dim3((kMaxLayerParams + 255) / 256, kLayers), 256, 0, c->st()>>>(net_params(c), c->P);
+    SBP_TRY_CUDA(cudaGetLastError());
     return SBP_OK;
 }
 
@@ -389,7 +397,7 @@ sbp_status sbp_cnn_create(int device, int max_batch, unsigned long long seed, sb
     e = e ?: alloc((void**)&c->Mo, c->nparams * 4);
     e = e ?: alloc((void**)&c->Ve, c->nparams * 4);
     for (int l = 0; l < kLayers; ++l) {
-        e = e ?: alloc((void**)&c->Wb[l], c->nw[l] * 2);
+        e = e ?: alloc((void**)&c->Wb[l], (int64_t)(kCoutP[l] < 16 ? 16 : kCoutP[l]) * 9 * kCinP[l] * 2);
         if (l > 0) e = e ?: alloc((void**)&c->Wt[l], (int64_t)kCinP[l] * 9 * kDzP[l] * 2);
         e = e ?: alloc((void**)&c->a[l], B * kPix * kCinP[l] * 2);
         e = e ?: alloc((void**)&c->dz[l], B * kPix * kDzP[l] * 2);
@@ -490,7 +498,7 @@ sbp_status sbp_cnn_forward(sbp_cnn* c, int n, const void* d_coarse, int dtype, i
     SBP_TRY(check_batch(c, n));
     if (!d_coarse || (dtype != SBP_F64 && dtype != SBP_F32) || img_stride < 4 * kPix) return SBP_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
-    return forward(c, n, d_coarse, dtype, img_stride);
+    return forward(c, n, d_coarse, dtype, img_stride, true);
 }
 
 sbp_status sbp_cnn_output(sbp_cnn* c, int n, float* d_y) {
@@ -508,7 +516,7 @@ sbp_status sbp_cnn_gradients(sbp_cnn* c, int n, const void* d_coarse, int dtype,
     if (!d_coarse || !d_fine_r || (dtype != SBP_F64 && dtype != SBP_F32) || img_stride < 4 * kPix)
         return SBP_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
-    SBP_TRY(forward(c, n, d_coarse, dtype, img_stride));
+    SBP_TRY(forward(c, n, d_coarse, dtype, img_stride, true));
     SBP_TRY(backward(c, n, d_coarse, dtype, img_stride, d_fine_r, loss));
     if (host_grads) {
         SBP_TRY_CUDA(cudaMemcpyAsync(host_grads, c->G, c->nparams * 4, cudaMemcpyDeviceToHost, c->st()));
@@ -526,32 +534,19 @@ sbp_status sbp_cnn_train_step(sbp_cnn* c, int n, const void* d_coarse, int dtype
     c->adam_t += 1;
     const float c1 = float(1.0 / (1.0 - std::pow(double(b1), c->adam_t)));
     const float c2 = float(1.0 / (1.0 - std::pow(double(b2), c->adam_t)));
-    for (int l = 0; l < kLayers; ++l) {
-        const int nw = (int)c->nw[l], nb = kCoutP[l];
-        // weights and biases of a layer are adjacent in P / G / Mo / Ve
-        adam_kernel<<<(nw + nb + 255) / 256, 256, 0, c->st()>>>(c->P + c->w_off[l], c->G + c->w_off[l],
-                                                                c->Mo + c->w_off[l], c->Ve + c->w_off[l], nw, nb, lr,
-                                                                b1, b2, c1, c2, eps, kCoutP[l], kCinP[l], kDzP[l],
-                                                                c->Wb[l], l > 0 ? c->Wt[l] : nullptr);
-        SBP_TRY_CUDA(cudaGetLastError());
-    }
+    adam_kernel<<<dim3((kMaxLayerParams + 255) / 256, kLayers), 256, 0, c->st()>>>(net_params(c), c->P, c->G, c->Mo, c->Ve,
+                                                                                  lr, b1, b2, c1, c2, eps);
+    SBP_TRY_CUDA(cudaGetLastError());
     return SBP_OK;
 }
 
 sbp_status sbp_cnn_apply(sbp_cnn* c, int n, const void* d_coarse, int dtype, int64_t img_stride, double* d_out) {
     clear_error();
-    SBP_TRY(sbp_cnn_forward(c, n, d_coarse, dtype, img_stride));
-    if (!d_out) return SBP_ERR_INVALID_ARGUMENT;
-    const int64_t total = (int64_t)n * kPix;
-    const int blocks = (int)((total + 255) / 256);
-    if (dtype == SBP_F64)
-        apply_kernel<double><<<blocks, 256, 0, c->st()>>>(c->y, static_cast<const double*>(d_coarse), img_stride, n,
-                                                          c->out_scale, d_out);
-    else
-        apply_kernel<float><<<blocks, 256, 0, c->st()>>>(c->y, static_cast<const float*>(d_coarse), img_stride, n,
-                                                         c->out_scale, d_out);
-    SBP_TRY_CUDA(cudaGetLastError());
-    return SBP_OK;
+    SBP_TRY(check_batch(c, n));
+    if (!d_coarse || (dtype != SBP_F64 && dtype != SBP_F32) || img_stride < 4 * kPix || !d_out)
+        return SBP_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(c->device);
+    return forward(c, n, d_coarse, dtype, img_stride, false, d_out);
 }
 
 sbp_status sbp_cnn_synchronize(sbp_cnn* c) {

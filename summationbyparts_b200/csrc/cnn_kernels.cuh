@@ -1,8 +1,16 @@
 // Kernels of the learned correction network: a 5-layer 3x3 convolutional network on the 64 x 64
 // coarse grid (4 -> 32 -> 32 -> 32 -> 32 -> 4 channels, GELU between layers).  Activations are
-// BF16 in NHWC layout (channels innermost), accumulation is FP32 on the tcgen05 tensor cores
-// with TMEM accumulators (convolutions forward and backward-data, and the weight gradients);
-// pre-activations, outputs, gradients and parameters are FP32.
+// BF16, accumulation is FP32 on the tcgen05 tensor cores with TMEM accumulators (convolutions
+// forward and backward-data, and the weight gradients); pre-activations, outputs, gradients and
+// parameters are FP32.
+//
+// Layout.  Activations and output gradients are chunk-major, [image][channel / 8][pixel][channel % 8]:
+// the 16 bytes of 8 channels of consecutive pixels are contiguous.  In shared memory that is the
+// tensor core's no-swizzle layout for both kinds of product -- rows of 16 bytes, 8 consecutive rows
+// a core matrix: K-major with pixels as M (convolutions) and MN-major with pixels as K (weight
+// gradients) -- and a tap's shift by whole pixels is an offset of the operand's start address, so no
+// operand is rearranged by a thread.  A warp's epilogue stores are 512 contiguous bytes.
+// Pre-activations are [image][channel / 4][pixel][channel % 4] for the same reason.
 //
 // Channel counts are padded to what one MMA step consumes: the 4-channel input is stored with
 // 16 channels (zeros above 4), the 4-channel output with 8, and the gradient of the output with
@@ -12,17 +20,19 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "bulk_copy.cuh"
+
 namespace sbp {
 namespace cnn {
 
 constexpr int kImg = 64;           // image side: the coarse grid
 constexpr int kPix = kImg * kImg;  // pixels per image
-constexpr int kBand = 4;           // image rows per CTA of the convolution kernel (256 pixels)
-constexpr int kConvThreads = 256;  // 8 warps: one pixel of the band per thread
+constexpr int kBand = 8;           // image rows per CTA of the convolution kernel
+constexpr int kConvThreads = 256;  // 8 warps: two accumulator tiles of 128 positions at a time
 constexpr int kWgradThreads = 128; // 4 warps: one accumulator row of a 128-row tile per thread
 constexpr int kWgradRows = 4;      // image rows per CTA in the weight-gradient kernel
 
-enum Epilogue { EPI_GELU = 0, EPI_LINEAR = 1, EPI_DGELU = 2 };
+enum Epilogue { EPI_GELU = 0, EPI_LINEAR = 1, EPI_DGELU = 2, EPI_APPLY = 3 };
 
 // erf(z) by the rational approximation of Abramowitz and Stegun, Handbook of Mathematical
 // Functions, formula 7.1.26: erf(z) = 1 - t (a1 + t (a2 + t (a3 + t (a4 + t a5)))) exp(-z^2),
@@ -59,21 +69,23 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Shared-memory matrix descriptor of a K-major bf16 operand in the canonical layout without
-// swizzling: core matrices of 8 rows x 16 bytes (128 contiguous bytes, row after row), adjacent
-// core matrices `lbo` bytes apart along K and `sbo` bytes apart along M (or N).  Fields: start
-// address / 16 (bits 0-13), lbo / 16 (16-29), sbo / 16 (32-45), descriptor version 1 (46-47),
-// base offset 0, layout type 0 = no swizzle (61-63).
+// Shared-memory matrix descriptor of a bf16 operand in the canonical layout without swizzling: core
+// matrices of 8 rows x 16 bytes (128 contiguous bytes, row after row).  K-major: a row holds 8 values
+// along K, core matrices are `lbo` bytes apart along K and `sbo` bytes apart along M (or N).
+// MN-major: a row holds 8 values along M (or N), core matrices are `lbo` bytes apart along K and
+// `sbo` bytes apart along M (or N).  Fields: start address / 16 (bits 0-13), lbo / 16 (16-29),
+// sbo / 16 (32-45), descriptor version 1 (46-47), base offset 0, layout type 0 = no swizzle (61-63).
 __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
 }
 
-// Instruction descriptor of tcgen05.mma kind::f16 with bf16 A and B (both K-major) and an f32
-// accumulator, M x N: D format (bits 4-5) = f32, A and B formats (7-9, 10-12) = bf16, N / 8
-// (17-22), M / 16 (24-28).
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor of tcgen05.mma kind::f16 with bf16 A and B and an f32 accumulator, M x N:
+// D format (bits 4-5) = f32, A and B formats (7-9, 10-12) = bf16, A and B MN-major (15, 16; both or
+// neither here), N / 8 (17-22), M / 16 (24-28).
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N, bool mn_major) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? 3u << 15 : 0u) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
 }
 
 // D (tmem) = A * B (+ D when accumulate != 0), issued by one thread.
@@ -89,20 +101,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
 __device__ __forceinline__ void umma_commit(uint64_t* mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
                  : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\nselp.b32 %0, 1, 0, q;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(mbar)), "r"(parity)
-        : "memory");
-    return done != 0;
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -137,155 +135,199 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 16-byte asynchronous global -> shared copy; src_bytes = 0 fills the destination with zeros.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
-                 : "memory");
-}
-
 // Bit of the network's device status word set when a convolution gave up waiting for its
 // tensor-core work (the wait is bounded, so a fault cannot hang the stream).
 constexpr unsigned kStatusMmaTimeout = 1u;
 constexpr int kMmaWaitLimit = 1 << 22;  // mbarrier polls before giving up
 
-// Shared-memory layout of the tcgen05 convolution (dynamic, 1024-byte aligned base).
+// Shared-memory layout of the tcgen05 convolution (dynamic).  A band of kBand rows with one halo row
+// on each side is one sequence of positions per channel chunk: each image row is preceded by a zero
+// position, which pads it on the left and the row before it on the right, so pixel (r, c) of the
+// band is position 1 + (r + 1) kPitch + c and the operand of tap (dy, dx) is the output's sequence
+// shifted by dy kPitch + dx.  Output position f = r kPitch + c; c = 64 is computed and dropped.
 template <int CIN, int COUT>
 struct ConvTcLayout {
-    static constexpr int NP = COUT < 16 ? 16 : COUT;        // N of the MMA (multiple of 16 for M = 128)
-    static constexpr int HR = kBand + 2;                    // halo rows
-    static constexpr int TILES = kBand * kImg / 128;        // M = 128 accumulator tiles (2)
-    static constexpr int TMEM_COLS = TILES * NP <= 32 ? 32 : 64;
-    static constexpr int PIX = HR * kImg;                   // pixels of one shifted copy
-    static constexpr int CH = CIN / 8;                      // 16-byte channel chunks per pixel
-    static constexpr int SBO = CH * 128;                    // bytes between 8-row groups
-    static constexpr int A_BYTES = PIX * CIN * 2;           // one shifted copy
-    static constexpr int B_TAP = NP * CIN * 2;              // weights of one tap
-    static constexpr int B_OFF = 3 * A_BYTES;
-    static constexpr int BAR_OFF = B_OFF + 9 * B_TAP;
-    static constexpr int BYTES = BAR_OFF + 16;
+    static constexpr int NP = COUT < 16 ? 16 : COUT;         // N of the MMA (multiple of 16 for M = 128)
+    static constexpr int HR = kBand + 2;                     // halo rows
+    static constexpr int PITCH = kImg + 1;
+    static constexpr int TILES = (kBand * PITCH + 127) / 128;  // M = 128 accumulator tiles (5)
+    static constexpr int TMEM_COLS = TILES * NP <= 128 ? 128 : 256;
+    static constexpr int POS = TILES * 128 + 2 * PITCH + 2;  // positions the operands can reach
+    static constexpr int CH = CIN / 8;                       // 16-byte channel chunks per pixel
+    static constexpr int PLANE = POS * 16;                   // bytes of one chunk's positions
+    static constexpr int B_TAP = NP * CIN * 2;               // weights of one tap: [chunk][NP][8]
+    static constexpr int B_OFF = CH * PLANE;
+    static constexpr int BAR_OFF = B_OFF + 9 * B_TAP;        // mbarriers: operands, one per tile
+    static constexpr int BYTES = BAR_OFF + 8 * (TILES + 1) + 8;
+    static_assert(PLANE % 16 == 0 && BAR_OFF % 8 == 0 && HR * PITCH + 1 <= POS, "layout");
 };
-// Byte offset of (row, 16-byte chunk kc) in a canonical no-swizzle K-major operand.
-template <int CH>
-__device__ __forceinline__ int canon_off(int row, int kc) {
-    return ((row >> 3) * CH + kc) * 128 + (row & 7) * 16;
+
+// Weights of a convolution as one contiguous block in the order of shared memory:
+// [tap][input chunk][NP outputs][8 input channels].
+__host__ __device__ constexpr int conv_weight_index(int n, int tap, int k, int cin, int np) {
+    return ((tap * (cin / 8) + k / 8) * np + n) * 8 + k % 8;
 }
+
+struct ConvArgs {
+    const __nv_bfloat16* x;    // input activations (or output gradients)
+    const __nv_bfloat16* w;    // weights, conv_weight_index order
+    const float* bias;         // forward
+    const float* zprev;        // EPI_DGELU: pre-activations of the layer below
+    float* zout;               // EPI_GELU: pre-activations (null: not kept); EPI_LINEAR, EPI_APPLY: y
+    __nv_bfloat16* yout;       // EPI_GELU, EPI_DGELU
+    const void* coarse;        // EPI_APPLY: states to correct (f64 or f32) and the corrected states
+    int coarse_f64;
+    int64_t img_stride;
+    float4 oscale;
+    double* out;
+    unsigned* status;
+};
 
 // 3x3 convolution with zero padding as an implicit GEMM on the tcgen05 tensor cores:
 // out[p][n] = sum over taps t and input channels k of x[p + off(t)][k] * w[n][t][k],
-// off(t) = (t / 3 - 1, t % 3 - 1).  One CTA of 256 threads computes kBand = 4 image rows
-// (two M = 128 pixel tiles, each 2 image rows) for all output channels (N = COUT, at least 16),
-// so the weights are staged once per 256 pixels: the input halo goes to
-// shared memory as three copies shifted by 0, 1 and 2 columns, each in the canonical K-major
-// layout, so the A operand of tap (dy, dx) is copy dx started dy image rows down -- an aligned
-// descriptor offset, no per-tap copy (tile h starts 2 h image rows further); the weights of the
-// 9 taps follow in the same layout.  One thread issues the 2 x 9 x CIN / 16 MMAs (K = 16 each)
-// into two TMEM accumulators of 128 lanes x N f32 columns and commits them to an mbarrier; after
-// the (bounded) wait warp w reads lanes 32 (w % 4) .. of tile w / 4 -- one pixel per thread, all
-// channels -- and runs the epilogue:
-//   EPI_GELU   z = acc + bias -> zout (f32), gelu(z) -> yout (bf16)   (hidden layers)
-//   EPI_LINEAR acc + bias -> zout (f32)                                (output layer)
+// off(t) = (t / 3 - 1, t % 3 - 1).  One CTA of 256 threads computes kBand = 8 image rows for all
+// output channels (N = COUT, at least 16): bulk copies bring the band's rows (1 KB per row and
+// chunk) and the layer's weights (one block) into shared memory, one thread issues the 9 x CIN / 16
+// MMAs (K = 16 each) of each of the 5 accumulator tiles and commits every tile to its own mbarrier,
+// and warp w reads lanes 32 (w % 4) .. of tiles w / 4, w / 4 + 2, ... -- one position per thread, all
+// channels -- while the later tiles are still being multiplied:
+//   EPI_GELU   z = acc + bias -> zout (f32, if kept), gelu(z) -> yout (bf16)   (hidden layers)
+//   EPI_LINEAR acc + bias -> zout (f32, [pixel][8])                            (output layer)
+//   EPI_APPLY  as EPI_LINEAR, and coarse + y * out_scale -> out (f64 planes)
 //   EPI_DGELU  acc * gelu'(zprev) -> yout (bf16)                       (gradient of a hidden layer)
+// Bound by memory (32 -> 32 layer, 64 images: 67 MB with pre-activations, 34 MB without).
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                  const __nv_bfloat16* __restrict__ w,
-                                                                  const float* __restrict__ bias,
-                                                                  const float* __restrict__ zprev,
-                                                                  float* __restrict__ zout,
-                                                                  __nv_bfloat16* __restrict__ yout,
-                                                                  unsigned* __restrict__ status) {
+__global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs A) {
     using L = ConvTcLayout<CIN, COUT>;
     static_assert(CIN % 16 == 0 && COUT % 8 == 0 && L::NP <= 32, "channel padding");
-    extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::BAR_OFF + 8);
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + L::TILES + 1);
     const int img = blockIdx.x / (kImg / kBand);
     const int r0 = (blockIdx.x % (kImg / kBand)) * kBand;
     const int tid = threadIdx.x, warp = tid >> 5;
 
     if (warp == 0) {
-        // TILES accumulators of 128 lanes x NP f32 columns (32 columns is the allocation minimum)
+        // TILES accumulators of 128 lanes x NP f32 columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(L::TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        mbar_init(mbar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid == 32)
+        for (int b = 0; b <= L::TILES; ++b) bulk_mbar_init(bar + b, 1);
+    // the zero positions between the rows, and the halo rows outside the image
+    for (int i = tid; i < (L::HR + 1) * L::CH; i += kConvThreads)
+        *reinterpret_cast<uint4*>(smem + (i % L::CH) * L::PLANE + (i / L::CH) * L::PITCH * 16) = make_uint4(0, 0, 0, 0);
+    const int hlo = r0 == 0 ? 1 : 0, hhi = r0 + kBand == kImg ? L::HR - 1 : L::HR;  // halo rows in the image
+    for (int i = tid; i < kImg * L::CH; i += kConvThreads) {
+        uint4* row = reinterpret_cast<uint4*>(smem + (i % L::CH) * L::PLANE) + 1 + i / L::CH;
+        if (hlo == 1) row[0] = make_uint4(0, 0, 0, 0);
+        if (hhi == L::HR - 1) row[(L::HR - 1) * L::PITCH] = make_uint4(0, 0, 0, 0);
     }
-    // Operands by asynchronous 16-byte copies straight into the canonical layout, all of a
-    // thread's copies in flight at once.  Weights: B[n][k] of tap t = w[n][t][k], rows n >= COUT
-    // zero-filled.
-    for (int i = tid; i < L::NP * 9 * L::CH; i += kConvThreads) {
-        const int kc = i % L::CH, t = (i / L::CH) % 9, n = i / (L::CH * 9);
-        const bool in = n < COUT;
-        cp_async16(smem + L::B_OFF + t * L::B_TAP + canon_off<L::CH>(n, kc),
-                   w + ((int64_t)(in ? n : 0) * 9 + t) * CIN + kc * 8, in ? 16u : 0u);
-    }
-    // input halo: rows r0 - 1 .. r0 + kBand, columns -1 .. 64 (zero outside the image), into the
-    // copies shifted by dx: copy dx, pixel (hr, c) = halo (hr, c + dx), i.e. image column c + dx - 1
-    for (int i = tid; i < 3 * L::HR * kImg * L::CH; i += kConvThreads) {
-        const int kc = i % L::CH, c = (i / L::CH) % kImg, hr = (i / (L::CH * kImg)) % L::HR;
-        const int dx = i / (L::CH * kImg * L::HR);
-        const int gr = r0 + hr - 1, gc = c + dx - 1;
-        const bool in = gr >= 0 && gr < kImg && gc >= 0 && gc < kImg;
-        const int64_t pix = in ? (int64_t)(img * kImg + gr) * kImg + gc : 0;
-        cp_async16(smem + dx * L::A_BYTES + canon_off<L::CH>(hr * kImg + c, kc), x + pix * CIN + kc * 8,
-                   in ? 16u : 0u);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    // the operands written through the generic proxy become visible to the tensor core's proxy
+    // the zeros written through the generic proxy become visible to the tensor core's proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    if (warp == 1) {
+        const int lane = tid & 31;
+        if (lane == 0) {
+            bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * kImg * 16 + 9 * L::B_TAP));
+            bulk_g2s(smem + L::B_OFF, A.w, 9 * L::B_TAP, bar);
+        }
+        __syncwarp();
+        for (int i = lane; i < (hhi - hlo) * L::CH; i += 32) {
+            const int kc = i % L::CH, hr = hlo + i / L::CH;
+            bulk_g2s(smem + kc * L::PLANE + (1 + hr * L::PITCH) * 16,
+                     A.x + (((int64_t)img * L::CH + kc) * kPix + (r0 + hr - 1) * kImg) * 8, kImg * 16, bar);
+        }
+    }
     if (tid == 0) {
-        constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP);
-        const uint32_t base = smem_u32(smem);
-        uint32_t acc = 0;
+        if (bulk_wait(bar, 0, kMmaWaitLimit)) {
+            constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP, false);
+            const uint32_t base = smem_u32(smem);
 #pragma unroll 1
-        for (int t = 0; t < 9; ++t) {
-            const int dy = t / 3, dx = t % 3;
+            for (int h = 0; h < L::TILES; ++h) {
+#pragma unroll 1
+                for (int t = 0; t < 9; ++t) {
+                    const uint32_t a = base + (h * 128 + (t / 3) * L::PITCH + t % 3) * 16;
+                    const uint32_t b = base + L::B_OFF + t * L::B_TAP;
 #pragma unroll
-            for (int j = 0; j < CIN / 16; ++j) {
-                const uint32_t b = base + L::B_OFF + t * L::B_TAP + 2 * j * 128;
-#pragma unroll
-                for (int h = 0; h < L::TILES; ++h) {
-                    const uint32_t a = base + dx * L::A_BYTES + (2 * h + dy) * (kImg / 8) * L::SBO + 2 * j * 128;
-                    umma_bf16(tmem + h * L::NP, umma_desc(a, 128, L::SBO), umma_desc(b, 128, L::SBO), idesc, acc);
+                    for (int j = 0; j < CIN / 16; ++j)
+                        umma_bf16(tmem + h * L::NP, umma_desc(a + 2 * j * L::PLANE, L::PLANE, 128),
+                                  umma_desc(b + 2 * j * L::NP * 16, L::NP * 16, 128), idesc, t > 0 || j > 0);
                 }
-                acc = 1;
+                umma_commit(bar + 1 + h);
             }
         }
-        umma_commit(mbar);
     }
-    bool done = false;
-    for (int it = 0; it < kMmaWaitLimit && !done; ++it) done = mbar_try_wait(mbar, 0);
-    tc_fence_after();
-    if (done) {
-        // thread tid holds row tid % 128 of accumulator tid / 128: pixel (r0 + tid / 64, tid % 64)
-        const int64_t p = (int64_t)(img * kImg + r0 + tid / kImg) * kImg + tid % kImg;
-        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (tid / 128) * L::NP;
+    __syncwarp();
+#pragma unroll 1
+    for (int h = warp >> 2; h < L::TILES; h += 2) {
+        const bool done = bulk_wait(bar + 1 + h, 0, kMmaWaitLimit);
+        tc_fence_after();
+        if (!done) {
+            if ((tid & 31) == 0) atomicOr(A.status, kStatusMmaTimeout);
+            break;
+        }
         float v[32];
+        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + h * L::NP;
         if constexpr (L::NP == 32) tmem_ld32(taddr, v);
         else tmem_ld16(taddr, v);
-#pragma unroll
-        for (int co = 0; co < COUT; co += 2) {
-            const float v0 = v[co], v1 = v[co + 1];
+        const int f = h * 128 + (tid & 127);  // this thread's position
+        const int r = f / L::PITCH, c = f % L::PITCH;
+        if (c < kImg && r < kBand) {
+            const int pix = (r0 + r) * kImg + c;
             if constexpr (EPI == EPI_GELU) {
-                const float z0 = v0 + bias[co], z1 = v1 + bias[co + 1];
-                *reinterpret_cast<float2*>(zout + p * COUT + co) = make_float2(z0, z1);
-                *reinterpret_cast<unsigned*>(yout + p * COUT + co) = pack_bf16(gelu(z0), gelu(z1));
-            } else if constexpr (EPI == EPI_LINEAR) {
-                *reinterpret_cast<float2*>(zout + p * COUT + co) = make_float2(v0 + bias[co], v1 + bias[co + 1]);
+                float4* z = A.zout ? reinterpret_cast<float4*>(A.zout) + (int64_t)img * (COUT / 4) * kPix + pix : nullptr;
+                uint4* y = reinterpret_cast<uint4*>(A.yout) + (int64_t)img * (COUT / 8) * kPix + pix;
+#pragma unroll
+                for (int q = 0; q < COUT / 8; ++q) {
+                    float zz[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) zz[i] = v[8 * q + i] + __ldg(A.bias + 8 * q + i);
+                    if (z) {
+                        z[(2 * q) * kPix] = make_float4(zz[0], zz[1], zz[2], zz[3]);
+                        z[(2 * q + 1) * kPix] = make_float4(zz[4], zz[5], zz[6], zz[7]);
+                    }
+                    y[q * kPix] = make_uint4(pack_bf16(gelu(zz[0]), gelu(zz[1])), pack_bf16(gelu(zz[2]), gelu(zz[3])),
+                                             pack_bf16(gelu(zz[4]), gelu(zz[5])), pack_bf16(gelu(zz[6]), gelu(zz[7])));
+                }
+            } else if constexpr (EPI == EPI_LINEAR || EPI == EPI_APPLY) {
+                static_assert(EPI == EPI_GELU || EPI == EPI_DGELU || COUT == 8, "output layer");
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] += __ldg(A.bias + i);
+                float4* y = reinterpret_cast<float4*>(A.zout) + ((int64_t)img * kPix + pix) * 2;
+                y[0] = make_float4(v[0], v[1], v[2], v[3]);
+                y[1] = make_float4(v[4], v[5], v[6], v[7]);
+                if constexpr (EPI == EPI_APPLY) {
+                    const float sc[4] = {A.oscale.x, A.oscale.y, A.oscale.z, A.oscale.w};
+                    double* o = A.out + (int64_t)img * 4 * kPix + pix;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int64_t at = img * A.img_stride + k * kPix + pix;
+                        const double cv = A.coarse_f64 ? static_cast<const double*>(A.coarse)[at]
+                                                       : double(static_cast<const float*>(A.coarse)[at]);
+                        o[k * kPix] = cv + double(v[k]) * double(sc[k]);
+                    }
+                }
             } else {
-                const float2 zp = *reinterpret_cast<const float2*>(zprev + p * COUT + co);
-                *reinterpret_cast<unsigned*>(yout + p * COUT + co) = pack_bf16(v0 * gelu_grad(zp.x), v1 * gelu_grad(zp.y));
+                const float4* zp = reinterpret_cast<const float4*>(A.zprev) + (int64_t)img * (COUT / 4) * kPix + pix;
+                uint4* y = reinterpret_cast<uint4*>(A.yout) + (int64_t)img * (COUT / 8) * kPix + pix;
+#pragma unroll
+                for (int q = 0; q < COUT / 8; ++q) {
+                    const float4 z0 = __ldg(zp + (2 * q) * kPix), z1 = __ldg(zp + (2 * q + 1) * kPix);
+                    const float* g = v + 8 * q;
+                    y[q * kPix] =
+                        make_uint4(pack_bf16(g[0] * gelu_grad(z0.x), g[1] * gelu_grad(z0.y)),
+                                   pack_bf16(g[2] * gelu_grad(z0.z), g[3] * gelu_grad(z0.w)),
+                                   pack_bf16(g[4] * gelu_grad(z1.x), g[5] * gelu_grad(z1.y)),
+                                   pack_bf16(g[6] * gelu_grad(z1.z), g[7] * gelu_grad(z1.w)));
+                }
             }
         }
-    } else if ((tid & 31) == 0) {
-        atomicOr(status, kStatusMmaTimeout);
     }
     tc_fence_before();
     __syncthreads();
@@ -295,64 +337,34 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __nv_bfl
     }
 }
 
-// Word k (0..3, a compile-time constant after unrolling) of a 16-byte vector, selected without
-// taking the vector's address (which would move it to local memory).
-__device__ __forceinline__ unsigned word_of(const uint4& u, int k) {
-    return k == 0 ? u.x : (k == 1 ? u.y : (k == 2 ? u.z : u.w));
-}
-
-// 8 x 8 transpose of bf16: in[j] holds 8 channels of pixel j, out[i] 8 pixels of channel i.
-__device__ __forceinline__ void transpose8x8_bf16(const uint4 in[8], uint4 out[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const unsigned sel = (i & 1) ? 0x7632u : 0x5410u;  // high or low halves of word i / 2
-        unsigned w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = __byte_perm(word_of(in[2 * q], i >> 1), word_of(in[2 * q + 1], i >> 1), sel);
-        out[i] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
-
-// Shared-memory layout of the tcgen05 weight-gradient kernel: the canonical A and B operands of
-// one image row, then the CTA's raw input rows (x with one halo row on each side, dz) as copied
-// from global memory.  Raw rows hold pixels channel-innermost with 16 bytes of padding after every
-// 8 pixels, so 8 threads reading the same channel chunk of 8 consecutive pixel groups hit 8
-// different 16-byte bank groups.
+// Shared-memory layout of the tcgen05 weight-gradient kernel.  A: planes of 16-byte pixel rows, one
+// per group of 8 accumulator rows: plane dx CIN / 8 + kc holds chunk kc of the band's x rows shifted
+// so that position (hr, c) is pixel (hr, c + dx - 1), then one plane of ones (channel 0), whose
+// accumulator row is the bias gradient.  An MMA takes 16 planes; those after the ones plane belong to
+// rows that are dropped, and may be any memory: they overlap B.
 template <int CIN, int M>
 struct WgradTcLayout {
-    static constexpr int ROWS = 9 * CIN + 1;                // (tap, input channel) rows + the ones row
-    static constexpr int TILES = (ROWS + 127) / 128;        // M = 128 tiles
-    static constexpr int AROWS = TILES * 128;
-    static constexpr int P = kImg;                          // pixels per chunk (one image row)
-    static constexpr int SBO = (P / 8) * 128;               // bytes between 8-row groups
-    static constexpr int A_BYTES = AROWS * P * 2;
-    static constexpr int B_OFF = A_BYTES;
-    static constexpr int XROW = P * CIN * 2 + (P / 8) * 16;  // bytes of one raw x row
-    static constexpr int ZROW = P * M * 2 + (P / 8) * 16;    // bytes of one raw dz row
-    static constexpr int XR_OFF = B_OFF + M * P * 2;
-    static constexpr int ZR_OFF = XR_OFF + (kWgradRows + 2) * XROW;
-    static constexpr int BAR_OFF = ZR_OFF + kWgradRows * ZROW;
-    static constexpr int BYTES = BAR_OFF + 16;
-    static constexpr int TMEM_COLS = TILES * M <= 32 ? 32 : (TILES * M <= 64 ? 64 : 128);
+    static constexpr int CH = CIN / 8;
+    static constexpr int HR = kWgradRows + 2;                // x rows with the halo
+    static constexpr int PLANE = HR * kImg * 16;
+    static constexpr int ONES = 3 * CH;                      // the ones plane
+    static constexpr int B_OFF = (ONES + 1) * PLANE;         // dz: [chunk][kWgradRows * 64][8]
+    static constexpr int BPLANE = kWgradRows * kImg * 16;
+    static constexpr int END = B_OFF + (M / 8) * BPLANE;
+    static constexpr int BAR_OFF = END > 16 * PLANE ? END : 16 * PLANE;
+    static constexpr int BYTES = BAR_OFF + 24;
+    static constexpr int TMEM_COLS = 3 * M <= 64 ? 64 : 128;
 };
-
-// Byte offset of pixel c, channel chunk kc of a raw row (C channels per pixel).
-template <int C>
-__device__ __forceinline__ int raw_off(int c, int kc) {
-    return c * C * 2 + (c >> 3) * 16 + kc * 16;
-}
 
 // Weight and bias gradients of one layer on the tcgen05 tensor cores, as partial sums per CTA
 // (kWgradRows image rows each) that wgrad_reduce_kernel adds up in a fixed order:
 // dw[m][t][k] = sum over pixels p of dz[p][m] * x[p + off(t)][k], db[m] = sum over p of dz[p][m].
-// The GEMM D[(t, k)][m] = sum over p of A[(t, k)][p] * B[m][p] has the 9 CIN (tap, channel) pairs
-// as its rows (M, in tiles of 128), the dz channels as N and the pixels as K.  The CTA's raw rows
-// of x (with the halo rows, zero outside the image) and dz arrive first, by 16-byte asynchronous
-// copies all in flight at once.  Per image row (64 pixels) the threads then write A and B in the
-// canonical K-major layout -- each 8 x 8 core matrix the register transpose of 8 pixels' 16-byte
-// channel vectors read from the raw rows -- and one thread issues TILES x 4 MMAs (K = 16)
-// accumulating in TMEM across the CTA's rows.  Row 9 CIN of A is all ones, so D's row 9 CIN is
-// the bias gradient; the remaining padding rows are zero.
+// For each row offset dy the GEMM D[(dx, k)][m] = sum over p of A[(dx, k)][p] * B[m][p] has the
+// 3 CIN (column offset, channel) pairs as its rows (M = 128 with the ones row and dropped rows), the
+// dz channels as N and the pixels as K; both operands are MN-major, as the chunk-major rows lie in
+// memory, so the bulk copies put them in place and one thread issues all 3 x kWgradRows x 4 MMAs
+// (K = 16) into three accumulators.  A row offset is a start offset of A; the column offsets are
+// three copies of the rows (an MMA's row groups lie one stride apart).
 // M = channels of dz as stored (16 or 32), MSTORE = rows of the layer's weight tensor (<= M).
 template <int CIN, int M, int MSTORE>
 __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bfloat16* __restrict__ x,
@@ -361,138 +373,102 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
                                                                 float* __restrict__ part_b,
                                                                 unsigned* __restrict__ status) {
     using L = WgradTcLayout<CIN, M>;
-    static_assert(CIN % 16 == 0 && M % 16 == 0 && MSTORE <= M && L::TILES * M <= 128, "channel padding");
-    constexpr int XCH = CIN / 8, ZCH = M / 8;
-    extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::BAR_OFF + 8);
+    static_assert(CIN % 16 == 0 && M % 16 == 0 && MSTORE <= M && L::ONES < 16, "channel padding");
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);  // operands, products
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
     constexpr int chunks_per_img = kImg / kWgradRows;
     const int img = blockIdx.x / chunks_per_img;
     const int rbase = (blockIdx.x % chunks_per_img) * kWgradRows;
     const int tid = threadIdx.x, warp = tid >> 5;
-    // raw rows: x rows rbase - 1 .. rbase + kWgradRows (zero-filled outside the image), dz rows
-    // rbase .. rbase + kWgradRows - 1
-    for (int i = tid; i < (kWgradRows + 2) * L::P * XCH; i += kWgradThreads) {
-        const int kc = i % XCH, c = (i / XCH) % L::P, hr = i / (XCH * L::P);
-        const int gr = rbase + hr - 1;
-        const bool in = gr >= 0 && gr < kImg;
-        cp_async16(smem + L::XR_OFF + hr * L::XROW + raw_off<CIN>(c, kc),
-                   x + ((int64_t)(img * kImg + (in ? gr : 0)) * kImg + c) * CIN + kc * 8, in ? 16u : 0u);
-    }
-    for (int i = tid; i < kWgradRows * L::P * ZCH; i += kWgradThreads) {
-        const int kc = i % ZCH, c = (i / ZCH) % L::P, hr = i / (ZCH * L::P);
-        cp_async16(smem + L::ZR_OFF + hr * L::ZROW + raw_off<M>(c, kc),
-                   dz + ((int64_t)(img * kImg + rbase + hr) * kImg + c) * M + kc * 8, 16u);
-    }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(L::TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        mbar_init(mbar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid == 32) {
+        bulk_mbar_init(bar, 1);
+        bulk_mbar_init(bar + 1, 1);
     }
-    // rows 9 CIN .. AROWS - 1 of A: the ones row, then zeros; written once
-    {
-        constexpr int first_group = (9 * CIN) / 8, groups = L::AROWS / 8 - first_group;
-        for (int i = tid; i < groups * (L::P / 8) * 8; i += kWgradThreads) {
-            const int row = first_group * 8 + (i / ((L::P / 8) * 8)) * 8 + (i % 8);
-            const int pg = (i / 8) % (L::P / 8);
-            const unsigned one = row == 9 * CIN ? 0x3F803F80u : 0u;  // bf16 1.0 pairs
-            *reinterpret_cast<uint4*>(smem + (row >> 3) * L::SBO + pg * 128 + (row & 7) * 16) =
-                make_uint4(one, one, one, one);
-        }
+    // the ones plane, the zero column of the copies for dx = 0 and 2, the rows outside the image
+    for (int i = tid; i < L::HR * kImg; i += kWgradThreads)
+        *reinterpret_cast<uint4*>(smem + L::ONES * L::PLANE + i * 16) = make_uint4(0x3F80u, 0u, 0u, 0u);  // bf16 1.0
+    const int hlo = rbase == 0 ? 1 : 0, hhi = rbase + kWgradRows == kImg ? L::HR - 1 : L::HR;
+    for (int i = tid; i < L::HR * L::CH * 2; i += kWgradThreads) {
+        const int side = i & 1, kc = (i >> 1) % L::CH, hr = (i >> 1) / L::CH;
+        *reinterpret_cast<uint4*>(smem + (2 * side * L::CH + kc) * L::PLANE + (hr * kImg + side * (kImg - 1)) * 16) =
+            make_uint4(0u, 0u, 0u, 0u);
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int i = tid; i < 3 * L::CH * kImg; i += kWgradThreads) {
+        uint4* pl = reinterpret_cast<uint4*>(smem + (i / kImg) * L::PLANE) + i % kImg;
+        if (hlo == 1) pl[0] = make_uint4(0u, 0u, 0u, 0u);
+        if (hhi == L::HR - 1) pl[(L::HR - 1) * kImg] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    constexpr uint32_t idesc = umma_idesc_bf16(128, M);
-    bool ok = true;
-    uint32_t phase = 0;
-#pragma unroll 1
-    for (int lr = 0; lr < kWgradRows && ok; ++lr) {
-        // A core matrices: (tap t, channel block kc, pixel group pg) = transpose of the 8 x 8 block
-        // x[pixels 8 pg + j shifted by the tap][channels 8 kc + i] (zero outside the image).
-        // Consecutive threads take consecutive pixel groups: conflict-free raw reads (padding) and
-        // canonical writes (128 bytes apart).
-        for (int i = tid; i < 9 * XCH * (L::P / 8); i += kWgradThreads) {
-            const int pg = i % (L::P / 8), kc = (i / (L::P / 8)) % XCH, t = i / ((L::P / 8) * XCH);
-            const unsigned char* src = smem + L::XR_OFF + (lr + t / 3) * L::XROW;
-            uint4 v[8], o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int gc = 8 * pg + j + t % 3 - 1;
-                v[j] = (gc >= 0 && gc < kImg) ? *reinterpret_cast<const uint4*>(src + raw_off<CIN>(gc, kc))
-                                              : make_uint4(0u, 0u, 0u, 0u);
-            }
-            transpose8x8_bf16(v, o);
-            const int r0 = t * CIN + kc * 8;
-            uint4* dst = reinterpret_cast<uint4*>(smem + (r0 >> 3) * L::SBO + pg * 128);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) dst[k] = o[k];
+    if (warp == 1) {
+        const int lane = tid & 31;
+        const int nrow = hhi - hlo;
+        if (lane == 0)
+            bulk_expect(bar, (uint32_t)(nrow * L::CH * (3 * kImg - 2) * 16 + (M / 8) * L::BPLANE));
+        __syncwarp();
+        for (int i = lane; i < M / 8; i += 32)
+            bulk_g2s(smem + L::B_OFF + i * L::BPLANE, dz + (((int64_t)img * (M / 8) + i) * kPix + rbase * kImg) * 8,
+                     L::BPLANE, bar);
+        // dx = 1: the rows of a chunk in one copy; dx = 0 and 2: 63 pixels of every row
+        for (int i = lane; i < L::CH; i += 32)
+            bulk_g2s(smem + (L::CH + i) * L::PLANE + hlo * kImg * 16,
+                     x + (((int64_t)img * L::CH + i) * kPix + (rbase + hlo - 1) * kImg) * 8, nrow * kImg * 16, bar);
+        for (int i = lane; i < 2 * nrow * L::CH; i += 32) {
+            const int side = i & 1, kc = (i >> 1) % L::CH, hr = hlo + (i >> 1) / L::CH;
+            const __nv_bfloat16* src = x + (((int64_t)img * L::CH + kc) * kPix + (rbase + hr - 1) * kImg + side) * 8;
+            bulk_g2s(smem + (2 * side * L::CH + kc) * L::PLANE + (hr * kImg + 1 - side) * 16, src, (kImg - 1) * 16, bar);
         }
-        // B core matrices: (channel block mc, pixel group pg) = transpose of dz[pixels][channels]
-        for (int i = tid; i < ZCH * (L::P / 8); i += kWgradThreads) {
-            const int pg = i % (L::P / 8), mc = i / (L::P / 8);
-            const unsigned char* src = smem + L::ZR_OFF + lr * L::ZROW;
-            uint4 v[8], o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const uint4*>(src + raw_off<M>(8 * pg + j, mc));
-            transpose8x8_bf16(v, o);
-            uint4* dst = reinterpret_cast<uint4*>(smem + L::B_OFF + mc * L::SBO + pg * 128);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) dst[k] = o[k];
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
+    }
+    if (tid == 0) {
+        if (bulk_wait(bar, 0, kMmaWaitLimit)) {
+            constexpr uint32_t idesc = umma_idesc_bf16(128, M, true);
             const uint32_t base = smem_u32(smem);
 #pragma unroll 1
-            for (int tile = 0; tile < L::TILES; ++tile)
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll 1
+                for (int lr = 0; lr < kWgradRows; ++lr)
 #pragma unroll
-                for (int s = 0; s < L::P / 16; ++s) {
-                    const uint32_t a = base + tile * (128 / 8) * L::SBO + 2 * s * 128;
-                    const uint32_t b = base + L::B_OFF + 2 * s * 128;
-                    umma_bf16(tmem + tile * M, umma_desc(a, 128, L::SBO), umma_desc(b, 128, L::SBO), idesc,
-                              (lr > 0 || s > 0) ? 1u : 0u);
-                }
-            umma_commit(mbar);
+                    for (int s = 0; s < kImg / 16; ++s) {
+                        const uint32_t a = base + ((lr + dy) * kImg + 16 * s) * 16;
+                        const uint32_t b = base + L::B_OFF + (lr * kImg + 16 * s) * 16;
+                        umma_bf16(tmem + dy * M, umma_desc(a, 128, L::PLANE), umma_desc(b, 128, L::BPLANE), idesc,
+                                  (lr > 0 || s > 0) ? 1u : 0u);
+                    }
+            umma_commit(bar + 1);
         }
-        // the operands are rewritten for the next row only after these MMAs have read them
-        bool done = false;
-        for (int it = 0; it < kMmaWaitLimit && !done; ++it) done = mbar_try_wait(mbar, phase);
-        phase ^= 1u;
-        if (!done) {
-            ok = false;
-            if ((tid & 31) == 0) atomicOr(status, kStatusMmaTimeout);
-        }
-        tc_fence_after();
-        __syncthreads();
     }
-    if (ok) {
+    __syncwarp();
+    const bool done = bulk_wait(bar + 1, 0, kMmaWaitLimit);
+    tc_fence_after();
+    if (done) {
         float* pw = part_w + (int64_t)blockIdx.x * (MSTORE * 9 * CIN);
 #pragma unroll 1
-        for (int tile = 0; tile < L::TILES; ++tile) {
-            const int r = tile * 128 + tid;  // this thread's accumulator row
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + tile * M;
+        for (int dy = 0; dy < 3; ++dy) {
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + dy * M;
             float v[32];
             if constexpr (M == 32) tmem_ld32(taddr, v);
             else tmem_ld16(taddr, v);
-            if (r < 9 * CIN) {
-                const int t = r / CIN, k = r % CIN;
+            if (tid < 3 * CIN) {  // accumulator row tid: column offset tid / CIN, channel tid % CIN
+                const int t = 3 * dy + tid / CIN, k = tid % CIN;
 #pragma unroll
                 for (int m = 0; m < MSTORE; ++m) pw[(m * 9 + t) * CIN + k] = v[m];
-            } else if (r == 9 * CIN) {
+            } else if (tid == 3 * CIN && dy == 0) {
 #pragma unroll
                 for (int m = 0; m < MSTORE; ++m) part_b[(int64_t)blockIdx.x * MSTORE + m] = v[m];
             }
         }
+    } else if ((tid & 31) == 0) {
+        atomicOr(status, kStatusMmaTimeout);
     }
     tc_fence_before();
     __syncthreads();
