@@ -31,6 +31,7 @@ constexpr int kDzP[kLayers] = {32, 32, 32, 32, 16};    // stored channels of eac
 template <class T>
 __global__ void pack_input_kernel(const T* __restrict__ st, int64_t img_stride, int n, float4 mean, float4 inv,
                                   __nv_bfloat16* __restrict__ a0) {
+    dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)n * kPix) return;
     const int64_t img = i / kPix, p = i % kPix;
@@ -48,6 +49,7 @@ __global__ void loss_kernel(const float* __restrict__ y, const T* __restrict__ c
                             const double* __restrict__ fine_r, int n, float4 oscale, float inv_count,
                             __nv_bfloat16* __restrict__ dz4, float* __restrict__ part) {
     __shared__ float red[256];
+    dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     float se = 0.0f;
     if (i < (int64_t)n * kPix) {
@@ -97,6 +99,7 @@ __device__ __forceinline__ void store_bf16_weight(const LayerParams& L, int e, f
 __global__ void adam_kernel(const NetParams N, float* __restrict__ P, const float* __restrict__ G,
                             float* __restrict__ Mo, float* __restrict__ Ve, float lr, float b1, float b2, float c1,
                             float c2, float eps) {
+    dependency_wait();
     const LayerParams& L = N.l[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.nw + L.cout) return;
@@ -113,6 +116,7 @@ __global__ void adam_kernel(const NetParams N, float* __restrict__ P, const floa
 
 // bf16 copies of the parameters (after set_params)
 __global__ void weights_bf16_kernel(const NetParams N, const float* __restrict__ P) {
+    dependency_wait();
     const LayerParams& L = N.l[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < L.nw) store_bf16_weight(L, e, P[L.off + e]);
@@ -207,6 +211,22 @@ struct sbp_cnn {
 
 namespace {
 
+// Launch that may begin while the stream's previous kernel drains (dependency_wait in the kernels).
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 template <int CIN, int COUT, int EPI>
 cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     constexpr int bytes = ConvTcLayout<CIN, COUT>::BYTES;
@@ -218,8 +238,7 @@ cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
         configured = true;
     }
     a.status = c->status;
-    conv3x3_tc_kernel<CIN, COUT, EPI><<<n * (kImg / kBand), kConvThreads, bytes, c->st()>>>(a);
-    return cudaGetLastError();
+    return launch_after(conv3x3_tc_kernel<CIN, COUT, EPI>, n * (kImg / kBand), kConvThreads, bytes, c->st(), a);
 }
 
 NetParams net_params(const sbp_cnn* c) {
@@ -254,11 +273,12 @@ cudaError_t wgrad(const sbp_cnn* c, int n, int layer, const __nv_bfloat16* x, co
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    wgrad_tc_kernel<CIN, M, MSTORE><<<parts, kWgradThreads, bytes, c->st()>>>(x, dz, c->part_w, c->part_b, c->status);
+    const cudaError_t e =
+        launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->status);
+    if (e != cudaSuccess) return e;
     const int nw = MSTORE * 9 * CIN, nb = MSTORE;
-    wgrad_reduce_kernel<<<(nw + nb + 31) / 32, 32 * kReduceSplit, 0, c->st()>>>(
-        c->part_w, c->part_b, parts, nw, nb, c->G + c->w_off[layer], c->G + c->b_off[layer]);
-    return cudaGetLastError();
+    return launch_after(wgrad_reduce_kernel, (nw + nb + 31) / 32, 32 * kReduceSplit, 0, c->st(), c->part_w, c->part_b, parts,
+                        nw, nb, c->G + c->w_off[layer], c->G + c->b_off[layer]);
 }
 
 sbp_status check_batch(const sbp_cnn* c, int n) {
@@ -276,12 +296,11 @@ sbp_status forward(sbp_cnn* c, int n, const void* state, int dtype, int64_t img_
     const int64_t total = (int64_t)n * kPix;
     const int blocks = (int)((total + 255) / 256);
     if (dtype == SBP_F64)
-        pack_input_kernel<double><<<blocks, 256, 0, c->st()>>>(static_cast<const double*>(state), img_stride, n,
-                                                               c->in_mean, c->in_inv, c->a[0]);
+        SBP_TRY_CUDA(launch_after(pack_input_kernel<double>, blocks, 256, 0, c->st(), static_cast<const double*>(state),
+                                  img_stride, n, c->in_mean, c->in_inv, c->a[0]));
     else
-        pack_input_kernel<float><<<blocks, 256, 0, c->st()>>>(static_cast<const float*>(state), img_stride, n,
-                                                              c->in_mean, c->in_inv, c->a[0]);
-    SBP_TRY_CUDA(cudaGetLastError());
+        SBP_TRY_CUDA(launch_after(pack_input_kernel<float>, blocks, 256, 0, c->st(), static_cast<const float*>(state),
+                                  img_stride, n, c->in_mean, c->in_inv, c->a[0]));
     for (int l = 0; l < kLayers; ++l) {
         ConvArgs a{};
         a.x = c->a[l];
@@ -323,12 +342,11 @@ sbp_status backward(sbp_cnn* c, int n, const void* coarse, int dtype, int64_t im
     const int blocks = (int)((total + 255) / 256);
     const float inv_count = 1.0f / float(total * 4);
     if (dtype == SBP_F64)
-        loss_kernel<double><<<blocks, 256, 0, c->st()>>>(c->y, static_cast<const double*>(coarse), img_stride, fine_r,
-                                                         n, c->out_scale, inv_count, c->dz[4], c->part_loss);
+        SBP_TRY_CUDA(launch_after(loss_kernel<double>, blocks, 256, 0, c->st(), c->y, static_cast<const double*>(coarse),
+                                  img_stride, fine_r, n, c->out_scale, inv_count, c->dz[4], c->part_loss));
     else
-        loss_kernel<float><<<blocks, 256, 0, c->st()>>>(c->y, static_cast<const float*>(coarse), img_stride, fine_r,
-                                                        n, c->out_scale, inv_count, c->dz[4], c->part_loss);
-    SBP_TRY_CUDA(cudaGetLastError());
+        SBP_TRY_CUDA(launch_after(loss_kernel<float>, blocks, 256, 0, c->st(), c->y, static_cast<const float*>(coarse),
+                                  img_stride, fine_r, n, c->out_scale, inv_count, c->dz[4], c->part_loss));
     SBP_TRY_CUDA((wgrad<32, 16, 8>(c, n, 4, c->a[4], c->dz[4])));
     SBP_TRY_CUDA(conv_input_gradient<16>(c, n, 4));
     for (int l = 3; l >= 1; --l) {
@@ -534,9 +552,8 @@ sbp_status sbp_cnn_train_step(sbp_cnn* c, int n, const void* d_coarse, int dtype
     c->adam_t += 1;
     const float c1 = float(1.0 / (1.0 - std::pow(double(b1), c->adam_t)));
     const float c2 = float(1.0 / (1.0 - std::pow(double(b2), c->adam_t)));
-    adam_kernel<<<dim3((kMaxLayerParams + 255) / 256, kLayers), 256, 0, c->st()>>>(net_params(c), c->P, c->G, c->Mo, c->Ve,
-                                                                                  lr, b1, b2, c1, c2, eps);
-    SBP_TRY_CUDA(cudaGetLastError());
+    SBP_TRY_CUDA(launch_after(adam_kernel, dim3((kMaxLayerParams + 255) / 256, kLayers), 256, 0, c->st(), net_params(c), c->P,
+                              c->G, c->Mo, c->Ve, lr, b1, b2, c1, c2, eps));
     return SBP_OK;
 }
 

@@ -27,7 +27,7 @@ namespace cnn {
 
 constexpr int kImg = 64;           // image side: the coarse grid
 constexpr int kPix = kImg * kImg;  // pixels per image
-constexpr int kBand = 8;           // image rows per CTA of the convolution kernel
+constexpr int kBand = 4;           // image rows per CTA of the convolution kernel
 constexpr int kConvThreads = 256;  // 8 warps: two accumulator tiles of 128 positions at a time
 constexpr int kWgradThreads = 128; // 4 warps: one accumulator row of a 128-row tile per thread
 constexpr int kWgradRows = 4;      // image rows per CTA in the weight-gradient kernel
@@ -103,6 +103,16 @@ __device__ __forceinline__ void umma_commit(uint64_t* mbar) {
                  : "memory");
 }
 
+// Programmatic dependent launch (the kernels are launched with it, see launch_after in cnn.cu): a
+// kernel may start while its predecessor in the stream drains.  dependency_wait returns once every
+// earlier kernel has completed and its writes are visible; only then does a kernel let its own
+// successor start, so what a successor does before its wait (barriers, TMEM, zero padding, the
+// weights, which the optimiser's kernel two or more launches before wrote) sees finished work.
+__device__ __forceinline__ void dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -150,8 +160,8 @@ struct ConvTcLayout {
     static constexpr int NP = COUT < 16 ? 16 : COUT;         // N of the MMA (multiple of 16 for M = 128)
     static constexpr int HR = kBand + 2;                     // halo rows
     static constexpr int PITCH = kImg + 1;
-    static constexpr int TILES = (kBand * PITCH + 127) / 128;  // M = 128 accumulator tiles (5)
-    static constexpr int TMEM_COLS = TILES * NP <= 128 ? 128 : 256;
+    static constexpr int TILES = (kBand * PITCH + 127) / 128;  // M = 128 accumulator tiles (3)
+    static constexpr int TMEM_COLS = TILES * NP <= 64 ? 64 : 128;
     static constexpr int POS = TILES * 128 + 2 * PITCH + 2;  // positions the operands can reach
     static constexpr int CH = CIN / 8;                       // 16-byte channel chunks per pixel
     static constexpr int PLANE = POS * 16;                   // bytes of one chunk's positions
@@ -185,17 +195,22 @@ struct ConvArgs {
 
 // 3x3 convolution with zero padding as an implicit GEMM on the tcgen05 tensor cores:
 // out[p][n] = sum over taps t and input channels k of x[p + off(t)][k] * w[n][t][k],
-// off(t) = (t / 3 - 1, t % 3 - 1).  One CTA of 256 threads computes kBand = 8 image rows for all
+// off(t) = (t / 3 - 1, t % 3 - 1).  One CTA of 256 threads computes kBand = 4 image rows for all
 // output channels (N = COUT, at least 16): bulk copies bring the band's rows (1 KB per row and
 // chunk) and the layer's weights (one block) into shared memory, one thread issues the 9 x CIN / 16
-// MMAs (K = 16 each) of each of the 5 accumulator tiles and commits every tile to its own mbarrier,
+// MMAs (K = 16 each) of each of the 3 accumulator tiles and commits every tile to its own mbarrier,
 // and warp w reads lanes 32 (w % 4) .. of tiles w / 4, w / 4 + 2, ... -- one position per thread, all
 // channels -- while the later tiles are still being multiplied:
 //   EPI_GELU   z = acc + bias -> zout (f32, if kept), gelu(z) -> yout (bf16)   (hidden layers)
 //   EPI_LINEAR acc + bias -> zout (f32, [pixel][8])                            (output layer)
 //   EPI_APPLY  as EPI_LINEAR, and coarse + y * out_scale -> out (f64 planes)
 //   EPI_DGELU  acc * gelu'(zprev) -> yout (bf16)                       (gradient of a hidden layer)
-// Bound by memory (32 -> 32 layer, 64 images: 67 MB with pre-activations, 34 MB without).
+// The band's copies, products and epilogue follow one another within a CTA, so what hides them is the
+// number of CTAs on an SM: four of 4 rows (51 KB, 128 TMEM columns) against two of 8 rows, although
+// 4 rows fill only 68% of their accumulator rows (8 rows: 81%): an apply pass of 512 states takes
+// 1.03 ms against 1.26 (16 rows, one CTA: 1.65).  The tensor pipe is the next bound (an M = 128,
+// N = 32 product takes 64 cycles, 13 us of a layer on 64 images), then memory (34 MB a layer, 67 MB
+// with pre-activations).
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs A) {
     using L = ConvTcLayout<CIN, COUT>;
@@ -231,14 +246,14 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    if (tid == 32) {
+        bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * kImg * 16 + 9 * L::B_TAP));
+        bulk_g2s(smem + L::B_OFF, A.w, 9 * L::B_TAP, bar);
+    }
+    dependency_wait();
     if (warp == 1) {
-        const int lane = tid & 31;
-        if (lane == 0) {
-            bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * kImg * 16 + 9 * L::B_TAP));
-            bulk_g2s(smem + L::B_OFF, A.w, 9 * L::B_TAP, bar);
-        }
         __syncwarp();
-        for (int i = lane; i < (hhi - hlo) * L::CH; i += 32) {
+        for (int i = tid & 31; i < (hhi - hlo) * L::CH; i += 32) {
             const int kc = i % L::CH, hr = hlo + i / L::CH;
             bulk_g2s(smem + kc * L::PLANE + (1 + hr * L::PITCH) * 16,
                      A.x + (((int64_t)img * L::CH + kc) * kPix + (r0 + hr - 1) * kImg) * 8, kImg * 16, bar);
@@ -362,7 +377,7 @@ struct WgradTcLayout {
 // For each row offset dy the GEMM D[(dx, k)][m] = sum over p of A[(dx, k)][p] * B[m][p] has the
 // 3 CIN (column offset, channel) pairs as its rows (M = 128 with the ones row and dropped rows), the
 // dz channels as N and the pixels as K; both operands are MN-major, as the chunk-major rows lie in
-// memory, so the bulk copies put them in place and one thread issues all 3 x kWgradRows x 4 MMAs
+// memory, so the bulk copies put them in place (one a plane) and one thread issues all 3 x kWgradRows x 4 MMAs
 // (K = 16) into three accumulators.  A row offset is a start offset of A; the column offsets are
 // three copies of the rows (an MMA's row groups lie one stride apart).
 // M = channels of dz as stored (16 or 32), MSTORE = rows of the layer's weight tensor (<= M).
@@ -391,61 +406,62 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
         bulk_mbar_init(bar, 1);
         bulk_mbar_init(bar + 1, 1);
     }
-    // the ones plane, the zero column of the copies for dx = 0 and 2, the rows outside the image
+    // the ones plane
     for (int i = tid; i < L::HR * kImg; i += kWgradThreads)
         *reinterpret_cast<uint4*>(smem + L::ONES * L::PLANE + i * 16) = make_uint4(0x3F80u, 0u, 0u, 0u);  // bf16 1.0
     const int hlo = rbase == 0 ? 1 : 0, hhi = rbase + kWgradRows == kImg ? L::HR - 1 : L::HR;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    dependency_wait();
+    // The copies: dz a chunk at a time, and the rows of x a chunk at a time for each dx, shifted by
+    // one position to the right (dx = 0, without the last pixel) or left (dx = 2, without the first)
+    if (tid == 32) bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * 3 * kImg * 16 - 2 * L::CH * 16 + (M / 8) * L::BPLANE));
+    if (warp == 1) {
+        const int lane = tid & 31;
+        __syncwarp();
+        for (int i = lane; i < M / 8; i += 32)
+            bulk_g2s(smem + L::B_OFF + i * L::BPLANE, dz + (((int64_t)img * (M / 8) + i) * kPix + rbase * kImg) * 8,
+                     L::BPLANE, bar);
+        for (int i = lane; i < 3 * L::CH; i += 32) {
+            const int dx = i / L::CH, kc = i % L::CH;
+            const __nv_bfloat16* src = x + (((int64_t)img * L::CH + kc) * kPix + (rbase + hlo - 1) * kImg + (dx == 2)) * 8;
+            bulk_g2s(smem + i * L::PLANE + (hlo * kImg + (dx == 0)) * 16, src, ((hhi - hlo) * kImg - (dx != 1)) * 16, bar);
+        }
+    }
+    const bool loaded = bulk_wait(bar, 0, kMmaWaitLimit);
+    // the column that a shifted copy took from the row beside it is zero padding, and so are the
+    // rows outside the image
     for (int i = tid; i < L::HR * L::CH * 2; i += kWgradThreads) {
         const int side = i & 1, kc = (i >> 1) % L::CH, hr = (i >> 1) / L::CH;
         *reinterpret_cast<uint4*>(smem + (2 * side * L::CH + kc) * L::PLANE + (hr * kImg + side * (kImg - 1)) * 16) =
             make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int i = tid; i < 3 * L::CH * kImg; i += kWgradThreads) {
-        uint4* pl = reinterpret_cast<uint4*>(smem + (i / kImg) * L::PLANE) + i % kImg;
-        if (hlo == 1) pl[0] = make_uint4(0u, 0u, 0u, 0u);
-        if (hhi == L::HR - 1) pl[(L::HR - 1) * kImg] = make_uint4(0u, 0u, 0u, 0u);
-    }
+    if (hlo == 1 || hhi == L::HR - 1)
+        for (int i = tid; i < 3 * L::CH * kImg; i += kWgradThreads) {
+            uint4* pl = reinterpret_cast<uint4*>(smem + (i / kImg) * L::PLANE) + i % kImg;
+            if (hlo == 1) pl[0] = make_uint4(0u, 0u, 0u, 0u);
+            if (hhi == L::HR - 1) pl[(L::HR - 1) * kImg] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    // what the threads wrote becomes visible to the tensor core's proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before();
     __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    if (warp == 1) {
-        const int lane = tid & 31;
-        const int nrow = hhi - hlo;
-        if (lane == 0)
-            bulk_expect(bar, (uint32_t)(nrow * L::CH * (3 * kImg - 2) * 16 + (M / 8) * L::BPLANE));
-        __syncwarp();
-        for (int i = lane; i < M / 8; i += 32)
-            bulk_g2s(smem + L::B_OFF + i * L::BPLANE, dz + (((int64_t)img * (M / 8) + i) * kPix + rbase * kImg) * 8,
-                     L::BPLANE, bar);
-        // dx = 1: the rows of a chunk in one copy; dx = 0 and 2: 63 pixels of every row
-        for (int i = lane; i < L::CH; i += 32)
-            bulk_g2s(smem + (L::CH + i) * L::PLANE + hlo * kImg * 16,
-                     x + (((int64_t)img * L::CH + i) * kPix + (rbase + hlo - 1) * kImg) * 8, nrow * kImg * 16, bar);
-        for (int i = lane; i < 2 * nrow * L::CH; i += 32) {
-            const int side = i & 1, kc = (i >> 1) % L::CH, hr = hlo + (i >> 1) / L::CH;
-            const __nv_bfloat16* src = x + (((int64_t)img * L::CH + kc) * kPix + (rbase + hr - 1) * kImg + side) * 8;
-            bulk_g2s(smem + (2 * side * L::CH + kc) * L::PLANE + (hr * kImg + 1 - side) * 16, src, (kImg - 1) * 16, bar);
-        }
-    }
-    if (tid == 0) {
-        if (bulk_wait(bar, 0, kMmaWaitLimit)) {
-            constexpr uint32_t idesc = umma_idesc_bf16(128, M, true);
-            const uint32_t base = smem_u32(smem);
+    if (tid == 0 && loaded) {
+        constexpr uint32_t idesc = umma_idesc_bf16(128, M, true);
+        const uint32_t base = smem_u32(smem);
 #pragma unroll 1
-            for (int dy = 0; dy < 3; ++dy)
+        for (int dy = 0; dy < 3; ++dy)
 #pragma unroll 1
-                for (int lr = 0; lr < kWgradRows; ++lr)
+            for (int lr = 0; lr < kWgradRows; ++lr)
 #pragma unroll
-                    for (int s = 0; s < kImg / 16; ++s) {
-                        const uint32_t a = base + ((lr + dy) * kImg + 16 * s) * 16;
-                        const uint32_t b = base + L::B_OFF + (lr * kImg + 16 * s) * 16;
-                        umma_bf16(tmem + dy * M, umma_desc(a, 128, L::PLANE), umma_desc(b, 128, L::BPLANE), idesc,
-                                  (lr > 0 || s > 0) ? 1u : 0u);
-                    }
-            umma_commit(bar + 1);
-        }
+                for (int s = 0; s < kImg / 16; ++s) {
+                    const uint32_t a = base + ((lr + dy) * kImg + 16 * s) * 16;
+                    const uint32_t b = base + L::B_OFF + (lr * kImg + 16 * s) * 16;
+                    umma_bf16(tmem + dy * M, umma_desc(a, 128, L::PLANE), umma_desc(b, 128, L::BPLANE), idesc,
+                              (lr > 0 || s > 0) ? 1u : 0u);
+                }
+        umma_commit(bar + 1);
     }
     __syncwarp();
     const bool done = bulk_wait(bar + 1, 0, kMmaWaitLimit);
@@ -489,6 +505,7 @@ __global__ void __launch_bounds__(32 * kReduceSplit) wgrad_reduce_kernel(const f
                                                                        int nw, int nb, float* __restrict__ gw,
                                                                        float* __restrict__ gb) {
     __shared__ float sums[kReduceSplit][32];
+    dependency_wait();
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + lane;
     const bool is_w = e < nw;
