@@ -3,30 +3,33 @@
 // Compiled with -fmad=false: results are bit-identical to the reference's row path
 // (xi) and column path (eta) in the same dtype.
 //
-// Aligned arrays (rows and batch stride multiples of 16 bytes, 16-byte aligned base pointers)
-// take the bulk-staged kernels: one tile per CTA, every input row segment of the tile (with its
-// halo or closure region) brought into shared memory by one cp.async.bulk copy that completes
-// on an mbarrier, so a CTA has its whole tile in flight at once and no thread spends
-// instructions on the loads.  Row tiles: kXiBulkRows rows x 128 vectors of 16 bytes (256 f64 or
-// 512 f32 outputs per row), each thread one 16-byte output vector per row.  Column tiles:
-// kEtaBulkRows rows x 1 KB of adjacent columns, each thread one column over its share of the
-// rows with the D-tap window in a register ring.  Other arrays take the kernels below.
+// One tile per CTA, every input row segment of the tile (with its halo or closure region) brought
+// into shared memory by one cp.async.bulk copy that completes on an mbarrier, so a CTA has its
+// whole tile in flight at once and no thread spends instructions on the loads.  Rows need not
+// start on 16-byte boundaries (odd lengths, offset pointers): a segment is widened to 16-byte
+// boundaries, which stays inside the array except at its first and last bytes, where the copy is
+// narrowed instead and a lane fetches the few elements left over (fetch_row).
 //
-// Row direction: a CTA stages kXiRows row segments (plus halo) in shared memory, with 16-byte
-// loads when the rows are 16-byte aligned; each thread
-// then reads its window with 16-byte vector loads and produces 16/sizeof(T) consecutive
-// outputs (2 f64 or 4 f32) per row, stored as one 16-byte vector.  Boundary-closure outputs
-// (first/last M of the row) read global memory directly.
+// Row tiles: up to kXiRows rows x 4 KB.  A thread's outputs are one 16-byte vector of the row in
+// memory (a column is counted from the 16-byte boundary at or before its row's start), so window loads
+// from shared memory and stores are 16 bytes wide on every row, whatever its alignment; outputs
+// of the boundary closures and of the vectors that a row's ends cut are taken one by one
+// afterwards, with the closure coefficients gathered from global memory.
 //
-// Column direction: one thread per 16 bytes of adjacent columns (2 f64 or 4 f32; one column
-// where the rows are not 16-byte aligned) marches down a chunk of rows with the D-tap windows
-// of its columns held in registers (fully unrolled ring, so no register moves), every row one
-// 16-byte load and one 16-byte store coalesced across the warp; rows inside the boundary
-// closures use the M x N blocks.  The reference's fused / unfused column split falls on a
-// multiple of 8 (f64) or 16 (f32) columns, so a thread's columns are all on the same side.
+// Arrays whose rows all start on 16-byte boundaries take instantiations (ALIGNED) in which that is
+// known: the bookkeeping of the general form costs 6% on 4 fields of 4096 x 4096.
+//
+// Column tiles: TR rows x TC adjacent columns, each thread one column over its share of the rows with
+// the D-tap window in a register ring.  The reference's fused / unfused column split falls on a
+// multiple of 8 (f64) or 16 (f32) columns.
+//
+// Bound by memory: one read and one write of the field.  Upwind9, 4 fields of 1021 x 1533 f64 (rows off
+// the 16-byte boundaries): 26 us each direction and kind, from 41 (row) and 69 (column) with a scalar load per
+// element; 64 x 64 f64 Upwind4: 10.8 to 5.3 (row) and 6.4 to 4.6 us (column).
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "bulk_copy.cuh"
 #include "op_apply.h"
@@ -37,8 +40,9 @@ namespace sbp {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kEtaRows = 64;  // rows per column chunk: enough CTAs for even waves on 4096^2 fields
-constexpr int kXiRows = 1;
+constexpr int kBulkWait = 1 << 22;  // mbarrier polls before a tile gives up
+// Tiles whose staged rows did not arrive within kBulkWait polls; their outputs are not written.
+__device__ unsigned g_bulk_timeouts = 0;
 
 template <class T>
 struct Vec;
@@ -51,295 +55,255 @@ struct Vec<float> {
     using type = float4;
 };
 
+// Closure-block rows (start blocks) in global memory: the row kernel's lanes read different rows of
+// them, which constant memory would serialise.
 template <int OP, int KIND, class T>
-__global__ void __launch_bounds__(kThreads)
-    op_xi_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t nbatch, int64_t bstride,
-                 T idx, bool vec_ok) {
-    constexpr int M = OpShape<OP>::M, H = OpShape<OP>::H;
-    constexpr int K = 16 / sizeof(T);           // outputs per thread
-    constexpr int PAD = ((H + K - 1) / K) * K;  // left/right halo, multiple of the vector width
-    constexpr int SEG = kThreads * K;
-    constexpr int NV = (K + 2 * PAD) / K;  // vectors in one thread's window
-    constexpr int BW = SEG + 2 * PAD;      // buffer width of one row
-    using V = typename Vec<T>::type;
-    __shared__ __align__(16) T buf[kXiRows * BW];
+struct GatherCoef;
+#define SBP_GATHER(OP, TAG, KINDV, KINDN, T, LIT, SUF)                                                          \
+    static __device__ const T g_##TAG##_##KINDN##_START_##SUF[] = {SBPC_##TAG##_##KINDN##_START(LIT)};           \
+    template <>                                                                                                 \
+    struct GatherCoef<OP, KINDV, T> {                                                                           \
+        __device__ __forceinline__ static T start(int i) { return __ldg(g_##TAG##_##KINDN##_START_##SUF + i); } \
+    };
+#define SBP_GATHER2(OP, TAG, KINDV, KINDN)                    \
+    SBP_GATHER(OP, TAG, KINDV, KINDN, double, SBPC_LIT_F64, D) \
+    SBP_GATHER(OP, TAG, KINDV, KINDN, float, SBPC_LIT_F32, F)
+SBP_GATHER2(UPWIND4, UPWIND4, DIFF, DIFF)
+SBP_GATHER2(UPWIND4H2, UPWIND4H2, DIFF, DIFF)
+SBP_GATHER2(UPWIND9, UPWIND9, DIFF, DIFF)
+SBP_GATHER2(UPWIND9H2, UPWIND9H2, DIFF, DIFF)
+SBP_GATHER2(SBP4, SBP4, DIFF, DIFF)
+SBP_GATHER2(SBP8, SBP8, DIFF, DIFF)
+SBP_GATHER2(UPWIND4, UPWIND4, DISS, DISS)
+SBP_GATHER2(UPWIND4H2, UPWIND4H2, DISS, DISS)
+SBP_GATHER2(UPWIND9, UPWIND9, DISS, DISS)
+SBP_GATHER2(UPWIND9H2, UPWIND9H2, DISS, DISS)
+#undef SBP_GATHER
+#undef SBP_GATHER2
 
-    const int nseg = (nx + SEG - 1) / SEG;
-    const int nrg = (ny + kXiRows - 1) / kXiRows;
-    const int64_t items = nbatch * (int64_t)nrg * nseg;
-    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        const int seg = (int)(it % nseg);
-        const int64_t rr = it / nseg;
-        const int row0 = (int)(rr % nrg) * kXiRows;
-        const int64_t b = rr / nrg;
-        const int nrows = min(kXiRows, ny - row0);
-        const int s0 = seg * SEG;
-        const int base = s0 - PAD;  // column of buf[row][0]
-        const int c_lo = base < 0 ? 0 : base;
-        const int c_hi = min(nx, s0 + SEG + PAD);
-        // every load of the kXiRows rows is issued before the barrier
-        for (int r = 0; r < nrows; ++r) {
-            const T* src = in + b * bstride + (int64_t)(row0 + r) * nx;
-            T* bb = buf + r * BW;
-            if (vec_ok) {
-                // c_lo and c_hi are multiples of K (or nx, itself a multiple of K)
-                for (int c = c_lo + K * threadIdx.x; c < c_hi; c += K * kThreads)
-                    *reinterpret_cast<V*>(bb + c - base) = __ldg(reinterpret_cast<const V*>(src + c));
-            } else {
-                for (int c = c_lo + threadIdx.x; c < c_hi; c += kThreads) bb[c - base] = __ldg(src + c);
+// sum_unfused (sbp_ops.cuh) with gathered closure coefficients: the same sum in the same order.
+template <int OP, int KIND, class T, class P>
+__device__ __forceinline__ T sum_gathered(int i, int n, P&& p) {
+    constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N, H = OpShape<OP>::H;
+    using C = GatherCoef<OP, KIND, T>;
+    if (i >= M && i < n - M) return diag_unfused<OP, KIND, T>([&](int d) { return p(i - H + d); });
+    const bool right = i >= n - M;
+    const int b = right ? n - N : 0;
+    auto coef = [&](int k) {
+        const T v = C::start(right ? (n - 1 - i) * N + (N - 1 - k) : i * N + k);
+        return right && KIND == DIFF ? -v : v;
+    };
+    T t = coef(0) * p(b);
+#pragma unroll
+    for (int k = 1; k < N; ++k) t = t + coef(k) * p(b + k);
+    return t;
+}
+
+// Elements of a row's first element past the 16-byte boundary at or before it.
+template <class T>
+__device__ __forceinline__ int parity_of(const T* p) {
+    return (int)((reinterpret_cast<uintptr_t>(p) & 15) / sizeof(T));
+}
+
+// The extent of the whole input array in memory.
+struct Extent {
+    uintptr_t begin, end;
+};
+
+// Bytes that the bulk copy of `w` elements at `src` takes, and its first byte: widened to 16-byte
+// boundaries, or narrowed at an end where that would leave the array.
+template <class T>
+__device__ __forceinline__ uint32_t row_span(const T* src, int w, const Extent& A, uintptr_t& first) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(src), b = a + (uintptr_t)w * sizeof(T);
+    uintptr_t lo = a & ~(uintptr_t)15, hi = (b + 15) & ~(uintptr_t)15;
+    if (lo < A.begin) lo += 16;
+    if (hi > A.end) hi -= 16;
+    first = lo;
+    return hi > lo ? (uint32_t)(hi - lo) : 0u;
+}
+
+// Fetches `nrows` row segments, `w(r)` elements at `src(r)` into `dst(r)` (16-byte aligned; element 0
+// lands parity_of(src) elements in), by the calling warp.  Announces the bytes on `bar` (count 1)
+// after the elements that the copies leave out have been written.
+template <class T, class SRC, class W, class DST>
+__device__ __forceinline__ void fetch_rows(int nrows, const SRC& src, const W& w, const DST& dst, const Extent& A,
+                                           uint64_t* bar) {
+    const int lane = threadIdx.x & 31;
+    uint32_t bytes = 0;
+    for (int r = lane; r < nrows; r += 32) {
+        uintptr_t first;
+        const T* s = src(r);
+        const int n = w(r);
+        const uint32_t b = row_span(s, n, A, first);
+        bytes += b;
+        const uintptr_t a = reinterpret_cast<uintptr_t>(s), last = first + b;
+        if (first > a || last < a + (uintptr_t)n * sizeof(T)) {
+            T* d = dst(r) + parity_of(s);
+            for (int k = 0; k < n; ++k) {
+                const uintptr_t e = a + (uintptr_t)k * sizeof(T);
+                if (e >= first && e < last) k = (int)((last - a) / sizeof(T)) - 1;  // copied in bulk
+                else d[k] = s[k];
             }
         }
-        __syncthreads();
-
-        const int c0 = s0 + K * threadIdx.x;
-        for (int r = 0; r < nrows && c0 < nx; ++r) {
-            const T* src = in + b * bstride + (int64_t)(row0 + r) * nx;
-            T* dst = out + b * bstride + (int64_t)(row0 + r) * nx;
-            const T* rbuf = buf + r * BW;
-            T o[K];
-            const bool interior = c0 >= M && c0 + K - 1 < nx - M;
-            if (interior) {
-                T w[K + 2 * PAD];
-                const V* bv = reinterpret_cast<const V*>(rbuf + K * threadIdx.x);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) reinterpret_cast<V*>(w)[v] = bv[v];
-                // w[j] holds column c0 - PAD + j
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-                    o[j] = diag_unfused<OP, KIND, T>([&](int d) { return w[j + d + PAD - H]; }) * idx;
-            } else {
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-                    if (c0 + j < nx)
-                        o[j] = sum_unfused<OP, KIND, T>(c0 + j, nx, [&](int kk) { return __ldg(src + kk); }) * idx;
-            }
-            if (vec_ok && c0 + K <= nx) {
-                *reinterpret_cast<V*>(dst + c0) = *reinterpret_cast<V*>(o);
-            } else {
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-                    if (c0 + j < nx) dst[c0 + j] = o[j];
-            }
-        }
-        __syncthreads();
+    }
+    bytes = __reduce_add_sync(0xffffffffu, bytes);
+    __syncwarp();
+    if (lane == 0) bulk_expect(bar, bytes);
+    __syncwarp();
+    for (int r = lane; r < nrows; r += 32) {
+        uintptr_t first;
+        const T* s = src(r);
+        const uint32_t b = row_span(s, w(r), A, first);
+        if (b)
+            bulk_g2s(reinterpret_cast<unsigned char*>(dst(r)) + (first - (reinterpret_cast<uintptr_t>(s) & ~(uintptr_t)15)),
+                     reinterpret_cast<const void*>(first), b, bar);
     }
 }
 
-template <int OP, int KIND, class T>
-__global__ void __launch_bounds__(kThreads)
-    op_eta_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t nbatch, int64_t bstride,
-                  T idx, int simd) {
-    constexpr int M = OpShape<OP>::M, D = OpShape<OP>::D, H = OpShape<OP>::H;
-    const int ncb = (nx + kThreads - 1) / kThreads;
-    const int nrc = (ny + kEtaRows - 1) / kEtaRows;
-    const int64_t items = nbatch * (int64_t)ncb * nrc;
-    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        const int cb = (int)(it % ncb);
-        const int64_t r1_ = it / ncb;
-        const int rc = (int)(r1_ % nrc);
-        const int64_t b = r1_ / nrc;
-        const int col = cb * kThreads + threadIdx.x;
-        if (col >= nx) continue;
-        const T* src = in + b * bstride + col;
-        T* dst = out + b * bstride + col;
-        const bool fused = col < simd;
-        const int y0 = rc * kEtaRows, y1 = min(ny, y0 + kEtaRows);
-        auto at = [&](int r) { return __ldg(src + (int64_t)r * nx); };
-        // closure rows in this chunk
-        for (int r = y0; r < y1 && r < M; ++r) dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
-        for (int r = max(y0, ny - M); r < y1; ++r)
-            dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
-        // interior rows: register ring
-        const int i0 = max(y0, M), i1 = min(y1, ny - M);
-        if (i0 >= i1) continue;
-        T w[D];
-#pragma unroll
-        for (int k = 0; k < D - 1; ++k) w[k] = at(i0 - H + k);
-        int r = i0;
-        for (; r + D <= i1; r += D) {
-#pragma unroll
-            for (int u = 0; u < D; ++u) {
-                w[(u + D - 1) % D] = at(r + u + H);
-                T f = T(0);
-                if (fused) {
-#pragma unroll
-                    for (int k = 0; k < D; ++k) f = fma_rn(w[(u + k) % D], Coef<OP, KIND, T>::diag(k), f);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < D; ++k) f = f + Coef<OP, KIND, T>::diag(k) * w[(u + k) % D];
-                }
-                dst[(int64_t)(r + u) * nx] = f * idx;
-            }
-        }
-        for (; r < i1; ++r) dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
-    }
-}
-
-// Column direction, K = 16 / sizeof(T) adjacent columns per thread (see the file comment).
-// Requires nx and bstride multiples of K and 16-byte aligned arrays.
-template <int OP, int KIND, class T>
-__global__ void __launch_bounds__(kThreads)
-    op_eta_vec_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t nbatch, int64_t bstride,
-                      T idx, int simd) {
-    constexpr int M = OpShape<OP>::M, D = OpShape<OP>::D, H = OpShape<OP>::H;
-    constexpr int K = 16 / sizeof(T);
-    using V = typename Vec<T>::type;
-    const int ngroups = nx / K;
-    const int ncb = (ngroups + kThreads - 1) / kThreads;
-    const int nrc = (ny + kEtaRows - 1) / kEtaRows;
-    const int64_t items = nbatch * (int64_t)ncb * nrc;
-    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        const int cb = (int)(it % ncb);
-        const int64_t r1_ = it / ncb;
-        const int rc = (int)(r1_ % nrc);
-        const int64_t b = r1_ / nrc;
-        const int grp = cb * kThreads + threadIdx.x;
-        if (grp >= ngroups) continue;
-        const int col0 = grp * K;
-        const T* src = in + b * bstride + col0;
-        T* dst = out + b * bstride + col0;
-        const bool fused = col0 < simd;  // simd is a multiple of K: all K columns agree
-        const int y0 = rc * kEtaRows, y1 = min(ny, y0 + kEtaRows);
-        auto row_vec = [&](int r) { return __ldg(reinterpret_cast<const V*>(src + (int64_t)r * nx)); };
-        auto closure_row = [&](int r) {
-            T o[K];
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-                o[j] = sum_column<OP, KIND, T>(fused, r, ny, [&](int rr) { return __ldg(src + (int64_t)rr * nx + j); }) *
-                       idx;
-            *reinterpret_cast<V*>(dst + (int64_t)r * nx) = *reinterpret_cast<V*>(o);
-        };
-        for (int r = y0; r < y1 && r < M; ++r) closure_row(r);
-        for (int r = max(y0, ny - M); r < y1; ++r) closure_row(r);
-        const int i0 = max(y0, M), i1 = min(y1, ny - M);
-        if (i0 >= i1) continue;
-        V w[D];
-#pragma unroll
-        for (int k = 0; k < D - 1; ++k) w[k] = row_vec(i0 - H + k);
-        int r = i0;
-        for (; r + D <= i1; r += D) {
-#pragma unroll
-            for (int u = 0; u < D; ++u) {
-                w[(u + D - 1) % D] = row_vec(r + u + H);
-                T o[K];
-#pragma unroll
-                for (int j = 0; j < K; ++j) {
-                    T f = T(0);
-                    if (fused) {
-#pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            f = fma_rn(reinterpret_cast<const T*>(&w[(u + k) % D])[j], Coef<OP, KIND, T>::diag(k), f);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            f = f + Coef<OP, KIND, T>::diag(k) * reinterpret_cast<const T*>(&w[(u + k) % D])[j];
-                    }
-                    o[j] = f * idx;
-                }
-                *reinterpret_cast<V*>(dst + (int64_t)(r + u) * nx) = *reinterpret_cast<V*>(o);
-            }
-        }
-        for (; r < i1; ++r) closure_row(r);
-    }
-}
-
-constexpr int kBulkWait = 1 << 22;  // mbarrier polls before a tile gives up
-// Tiles whose staged rows did not arrive within kBulkWait polls; their outputs are not written.
-__device__ unsigned g_bulk_timeouts = 0;
-
-constexpr int kXiBulkRows = 16;
+constexpr int kXiRows = 16;  // most rows of a row tile
 template <class T>
-constexpr int xi_bulk_cols() { return 128 * (16 / (int)sizeof(T)); }
+constexpr int xi_cols() { return 128 * (16 / (int)sizeof(T)); }
 template <class T>
-constexpr int xi_bulk_pitch() { return xi_bulk_cols<T>() + 32; }  // covers the halo, closures and alignment
+constexpr int xi_pitch() { return xi_cols<T>() + 32; }  // covers the halo, closures and alignment
 template <class T>
-constexpr size_t xi_bulk_smem() { return (size_t)kXiBulkRows * xi_bulk_pitch<T>() * sizeof(T) + 16; }
+constexpr size_t xi_smem(int rows) { return (size_t)rows * xi_pitch<T>() * sizeof(T) + 16; }
 
-// Row direction, bulk-staged tile (see the file comment).  Requires nx and bstride multiples of
-// K = 16 / sizeof(T) and 16-byte aligned arrays.
-template <int OP, int KIND, class T>
+// Row direction (see the file comment): `tr` rows per tile, 2^lpr threads per row.  u counts elements
+// from the 16-byte boundary at or before a row's start; tile cb covers u in [cb TC, cb TC + TC).
+// vec_out: output rows have the alignment of the input rows, so vectors are stored whole.
+template <int OP, int KIND, class T, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
-    op_xi_bulk_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx) {
+    op_xi_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int ncb, int tr,
+                 int lpr, bool vec_out, Extent A) {
     constexpr int M = OpShape<OP>::M, H = OpShape<OP>::H;
     constexpr int K = 16 / sizeof(T);
-    constexpr int TC = xi_bulk_cols<T>(), P = xi_bulk_pitch<T>(), TR = kXiBulkRows;
+    constexpr int TC = xi_cols<T>(), P = xi_pitch<T>();
     constexpr int PAD = ((H + K - 1) / K) * K;
     constexpr int NV = (K + 2 * PAD) / K;
     using V = typename Vec<T>::type;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* buf = reinterpret_cast<T*>(smem_raw);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)TR * P * sizeof(T));
-    const int ncb = (nx + TC - 1) / TC, nrg = (ny + TR - 1) / TR;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)tr * P * sizeof(T));
+    const int nrg = (ny + tr - 1) / tr;
     int64_t it = blockIdx.x;
     const int cb = (int)(it % ncb);
     it /= ncb;
     const int rg = (int)(it % nrg);
-    const int64_t b = it / nrg;
-    const int c0 = cb * TC, c1 = min(nx, c0 + TC);
-    const int y0 = rg * TR, nrows = min(TR, ny - y0);
-    int lo, hi;
-    region_of<OP>(c0, c1, nx, lo, hi);
-    lo -= lo % K;                              // 16-byte aligned segment start
-    hi = min(nx, (hi + K - 1) / K * K);        // and a whole number of 16-byte vectors
-    const uint32_t row_bytes = (uint32_t)(hi - lo) * (uint32_t)sizeof(T);
-    const T* src = in + b * bstride + (int64_t)y0 * nx + lo;
+    const int64_t off = (it / nrg) * bstride + (int64_t)rg * tr * nx;  // the tile's first row
+    const int nrows = min(tr, ny - rg * tr), u0 = cb * TC;
+    const T* src = in + off;
+    T* dst = out + off;
+    auto row_parity = [&](int r) { return ALIGNED ? 0 : parity_of(src + (int64_t)r * nx); };
+    // columns [lo, hi) of row r that the tile's outputs read (aligned: whole vectors of them)
+    int lo_a = 0, hi_a = 0;
+    if constexpr (ALIGNED) {
+        region_of<OP>(u0, min(nx, u0 + TC), nx, lo_a, hi_a);
+        lo_a &= ~(K - 1);
+        hi_a = min(nx, (hi_a + K - 1) & ~(K - 1));
+    }
+    auto seg = [&](int r, int& lo, int& hi) {
+        lo = lo_a;
+        hi = hi_a;
+        if constexpr (!ALIGNED) {
+            const int par = row_parity(r), c0 = max(0, u0 - par), c1 = min(nx, u0 + TC - par);
+            if (c0 < c1) region_of<OP>(c0, c1, nx, lo, hi);
+        }
+    };
     if (threadIdx.x == 0) bulk_mbar_init(bar, 1);
     __syncthreads();
     if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) bulk_expect(bar, row_bytes * (uint32_t)nrows);
-        for (int r = threadIdx.x; r < nrows; r += 32) bulk_g2s(buf + r * P, src + (int64_t)r * nx, row_bytes, bar);
+        if constexpr (ALIGNED) {
+            const uint32_t row_bytes = (uint32_t)(hi_a - lo_a) * (uint32_t)sizeof(T);
+            if (threadIdx.x == 0) bulk_expect(bar, row_bytes * (uint32_t)nrows);
+            for (int r = threadIdx.x; r < nrows; r += 32)
+                bulk_g2s(buf + r * P, src + (int64_t)r * nx + lo_a, row_bytes, bar);
+        } else {
+            int lo, hi;
+            fetch_rows<T>(
+                nrows,
+                [&](int r) {
+                    seg(r, lo, hi);
+                    return src + (int64_t)r * nx + lo;
+                },
+                [&](int r) {
+                    seg(r, lo, hi);
+                    return hi - lo;
+                },
+                [&](int r) { return buf + r * P; }, A, bar);
+        }
     }
     if (!bulk_wait(bar, 0, kBulkWait)) {
         if (threadIdx.x == 0) atomicAdd(&g_bulk_timeouts, 1u);
         return;
     }
-    const int sub = threadIdx.x / 128, v = threadIdx.x % 128;
-    const int c = c0 + K * v;  // first of this thread's K outputs; buf column 0 is input column lo
-    if (c >= c1) return;
-    const bool interior = c >= M && c + K - 1 < nx - M;
-    for (int r = sub; r < nrows; r += 2) {
-        const T* rb = buf + r * P;
-        T* dst = out + b * bstride + (int64_t)(y0 + r) * nx;
-        T o[K];
-        if (interior) {
+    const int v = threadIdx.x & ((1 << lpr) - 1);
+    for (int r = threadIdx.x >> lpr; r < nrows; r += kThreads >> lpr) {
+        const int par = row_parity(r);
+        int lo, hi;
+        seg(r, lo, hi);
+        const int su = (lo + par) & ~(K - 1);  // u of the segment's first staged element
+        for (int u = u0 + K * v; u < u0 + TC; u += K << lpr) {
+            const int c = u - par;
+            if (c < M || c + K - 1 >= nx - M) continue;
             T w[K + 2 * PAD];  // w[j] holds column c - PAD + j
-            const V* bv = reinterpret_cast<const V*>(rb + (c - PAD - lo));
+            const V* bv = reinterpret_cast<const V*>(buf + r * P + (u - PAD - su));
 #pragma unroll
             for (int q = 0; q < NV; ++q) reinterpret_cast<V*>(w)[q] = bv[q];
+            T o[K];
 #pragma unroll
             for (int j = 0; j < K; ++j)
                 o[j] = diag_unfused<OP, KIND, T>([&](int d) { return w[j + d + PAD - H]; }) * idx;
-        } else {
+            T* d = dst + (int64_t)r * nx + c;
+            if (vec_out) {
+                *reinterpret_cast<V*>(d) = *reinterpret_cast<V*>(o);
+            } else {
 #pragma unroll
-            for (int j = 0; j < K; ++j)
-                o[j] = sum_unfused<OP, KIND, T>(c + j, nx, [&](int kk) { return rb[kk - lo]; }) * idx;
+                for (int j = 0; j < K; ++j) d[j] = o[j];
+            }
         }
-        *reinterpret_cast<V*>(dst + c) = *reinterpret_cast<V*>(o);
+    }
+    // the ends of the rows: columns whose vector is not interior, one output per thread
+    constexpr int E = M + K - 1;
+    const bool any_left = u0 < E + K, any_right = u0 + TC > nx - E;
+    if (!any_left && !any_right) return;
+    for (int i = threadIdx.x; i < nrows * 2 * E; i += kThreads) {
+        const int r = i / (2 * E), k = i % (2 * E);
+        const int c = k < E ? k : nx - 1 - (k - E);
+        if (k < E ? c >= nx - E : c < 0) continue;  // the two ends meet on short rows: the right one takes it
+        const int par = row_parity(r), u = c + par;
+        if (u < u0 || u >= u0 + TC) continue;
+        const int cv = (u & ~(K - 1)) - par;
+        if (cv >= M && cv + K - 1 < nx - M) continue;  // done above
+        int lo, hi;
+        seg(r, lo, hi);
+        const T* rb = buf + r * P + (par - ((lo + par) & ~(K - 1)));  // column 0 of the row
+        dst[(int64_t)r * nx + c] = sum_gathered<OP, KIND, T>(c, nx, [&](int kk) { return rb[kk]; }) * idx;
     }
 }
 
-constexpr int kEtaBulkRows = 48;
-template <int OP, class T>
-constexpr int eta_bulk_region() {  // input rows a column tile can need (region_of's extent)
+template <int OP, int TR>
+constexpr int eta_region() {  // input rows a column tile can need (region_of's extent)
     constexpr int M = OpShape<OP>::M, N = OpShape<OP>::N, H = OpShape<OP>::H;
-    constexpr int a = kEtaBulkRows + H + (H > M - 1 ? H : M - 1);
+    constexpr int a = TR + H + (H > M - 1 ? H : M - 1);
     return a > N ? a : N;
 }
-template <int OP, class T>
-constexpr size_t eta_bulk_smem() { return (size_t)eta_bulk_region<OP, T>() * 1024 + 16; }
+template <class T, int TC, bool ALIGNED>
+constexpr int eta_pitch() { return TC + (ALIGNED ? 0 : 2 * (16 / (int)sizeof(T))); }  // room for the widened ends
+template <int OP, class T, int TR, int TC, bool ALIGNED>
+constexpr size_t eta_smem() { return (size_t)eta_region<OP, TR>() * eta_pitch<T, TC, ALIGNED>() * sizeof(T) + 16; }
 
-// Column direction, bulk-staged tile (see the file comment).  Same requirements as the row tile.
-template <int OP, int KIND, class T>
+// Column direction (see the file comment).
+template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
-    op_eta_bulk_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx,
-                       int simd) {
+    op_eta_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int simd,
+                  Extent A) {
     constexpr int M = OpShape<OP>::M, D = OpShape<OP>::D, H = OpShape<OP>::H;
-    constexpr int TC = 1024 / sizeof(T), TR = kEtaBulkRows;
-    constexpr int GROUPS = kThreads / TC;  // row groups (2 in f64, 1 in f32)
+    constexpr int K = 16 / sizeof(T), P = eta_pitch<T, TC, ALIGNED>();
+    constexpr int GROUPS = kThreads / TC;  // row groups
     constexpr int RG = TR / GROUPS;        // rows of one thread
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* buf = reinterpret_cast<T*>(smem_raw);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)eta_bulk_region<OP, T>() * 1024);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)eta_region<OP, TR>() * P * sizeof(T));
     const int ncb = (nx + TC - 1) / TC, nrc = (ny + TR - 1) / TR;
     int64_t it = blockIdx.x;  // vertically adjacent tiles are adjacent in launch order (shared halos in L2)
     const int rc = (int)(it % nrc);
@@ -349,14 +313,20 @@ __global__ void __launch_bounds__(kThreads)
     const int y0 = rc * TR, y1 = min(ny, y0 + TR), c0 = cb * TC, tw = min(TC, nx - c0);
     int lo, hi;
     region_of<OP>(y0, y1, ny, lo, hi);
-    const int nrows = hi - lo;
-    const uint32_t row_bytes = (uint32_t)tw * (uint32_t)sizeof(T);
     const T* src = in + b * bstride + (int64_t)lo * nx + c0;
     if (threadIdx.x == 0) bulk_mbar_init(bar, 1);
     __syncthreads();
     if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) bulk_expect(bar, row_bytes * (uint32_t)nrows);
-        for (int r = threadIdx.x; r < nrows; r += 32) bulk_g2s(buf + r * TC, src + (int64_t)r * nx, row_bytes, bar);
+        if constexpr (ALIGNED) {
+            const int nrows = hi - lo;
+            const uint32_t row_bytes = (uint32_t)tw * (uint32_t)sizeof(T);
+            if (threadIdx.x == 0) bulk_expect(bar, row_bytes * (uint32_t)nrows);
+            for (int r = threadIdx.x; r < nrows; r += 32) bulk_g2s(buf + r * P, src + (int64_t)r * nx, row_bytes, bar);
+        } else {
+            fetch_rows<T>(
+                hi - lo, [&](int r) { return src + (int64_t)r * nx; }, [&](int) { return tw; },
+                [&](int r) { return buf + r * P; }, A, bar);
+        }
     }
     if (!bulk_wait(bar, 0, kBulkWait)) {
         if (threadIdx.x == 0) atomicAdd(&g_bulk_timeouts, 1u);
@@ -367,7 +337,9 @@ __global__ void __launch_bounds__(kThreads)
     const int col = c0 + j;
     const bool fused = col < simd;
     T* dst = out + b * bstride + col;
-    auto at = [&](int r) { return buf[(r - lo) * TC + j]; };
+    // row r of the array starts (p0 + (r - lo) nx) mod K elements past a 16-byte boundary
+    const int p0 = parity_of(src), step = nx & (K - 1);
+    auto at = [&](int r) { return buf[(r - lo) * P + (ALIGNED ? 0 : (p0 + (r - lo) * step) & (K - 1)) + j]; };
     const int ra = y0 + g * RG, rb = min(y1, ra + RG);
     for (int r = ra; r < rb && r < M; ++r) dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
     for (int r = max(ra, ny - M); r < rb; ++r) dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
@@ -395,81 +367,55 @@ __global__ void __launch_bounds__(kThreads)
     for (; r < i1; ++r) dst[(int64_t)r * nx] = sum_column<OP, KIND, T>(fused, r, ny, at) * idx;
 }
 
-int g_num_sms = 0;
+constexpr int kSms = 148;
 
-int num_sms() {
-    if (g_num_sms == 0) {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        g_num_sms = n;
+// Column tiles of 48 rows x 1 KB stream the largest share of a field per halo row; while they would
+// leave SMs without a tile (a 64 x 64 field is two of them), 16 rows x 32 columns do the work with
+// two rows per thread instead of 24 to 48.
+template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
+cudaError_t launch_eta(const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride, const Extent& A,
+                       cudaStream_t st) {
+    constexpr size_t smem = eta_smem<OP, T, TR, TC, ALIGNED>();
+    static bool configured = false;  // per instantiation: the attribute belongs to the function
+    if (!configured && smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(op_eta_kernel<OP, KIND, T, TR, TC, ALIGNED>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        configured = true;
     }
-    return g_num_sms;
+    const T idx = inv_spacing<T>(OpShape<OP>::h2, ny);
+    const int simd = (int)(simd_lanes<T>() * (nx / simd_lanes<T>()));
+    const int64_t items = nbatch * ((ny + TR - 1) / TR) * ((nx + TC - 1) / TC);
+    op_eta_kernel<OP, KIND, T, TR, TC, ALIGNED>
+        <<<(unsigned)items, kThreads, smem, st>>>(in, out, (int)ny, (int)nx, bstride, idx, simd, A);
+    return cudaGetLastError();
 }
 
-template <int OP, int KIND, class T>
+template <int OP, int KIND, class T, bool ALIGNED>
 cudaError_t launch_t(int dir, const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride,
                      cudaStream_t st) {
-    // One work item per CTA (the grid-stride loops only matter beyond this cap): the block
-    // scheduler then overlaps one CTA's loads with another's arithmetic, which the measured
-    // throughput prefers to a persistent grid that loops load -> compute -> store.
-    const int blocks_cap = 1 << 30;
-    (void)num_sms;
     constexpr int K = 16 / sizeof(T);
-    const bool aligned = (nx % K == 0) && (bstride % K == 0) && (reinterpret_cast<uintptr_t>(in) % 16 == 0) &&
-                         (reinterpret_cast<uintptr_t>(out) % 16 == 0);
-    if (aligned) {
-        // bulk-staged tiles, one per CTA
-        if (dir == 0) {
-            const T idx = inv_spacing<T>(OpShape<OP>::h2, nx);
-            constexpr int TC = xi_bulk_cols<T>();
-            const int64_t items = nbatch * ((ny + kXiBulkRows - 1) / kXiBulkRows) * ((nx + TC - 1) / TC);
-            op_xi_bulk_kernel<OP, KIND, T><<<(unsigned)items, kThreads, xi_bulk_smem<T>(), st>>>(
-                in, out, (int)ny, (int)nx, bstride, idx);
-        } else {
-            const T idx = inv_spacing<T>(OpShape<OP>::h2, ny);
-            const int simd = (int)(simd_lanes<T>() * (nx / simd_lanes<T>()));
-            constexpr int TC = 1024 / sizeof(T);
-            constexpr size_t smem = eta_bulk_smem<OP, T>();
-            static bool configured = false;  // per instantiation: the attribute belongs to the function
-            if (!configured) {
-                const cudaError_t e = cudaFuncSetAttribute(op_eta_bulk_kernel<OP, KIND, T>,
-                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e != cudaSuccess) return e;
-                configured = true;
-            }
-            const int64_t items = nbatch * ((ny + kEtaBulkRows - 1) / kEtaBulkRows) * ((nx + TC - 1) / TC);
-            op_eta_bulk_kernel<OP, KIND, T><<<(unsigned)items, kThreads, smem, st>>>(in, out, (int)ny, (int)nx, bstride,
-                                                                                     idx, simd);
-        }
-        return cudaGetLastError();
+    const uintptr_t a = reinterpret_cast<uintptr_t>(in);
+    const Extent A{a, a + ((uintptr_t)(nbatch - 1) * bstride + (uintptr_t)ny * nx) * sizeof(T)};
+    if (dir == 1) {
+        constexpr int TR = 48, TC = 1024 / sizeof(T);
+        if (nbatch * ((ny + TR - 1) / TR) * ((nx + TC - 1) / TC) >= kSms)
+            return launch_eta<OP, KIND, T, TR, TC, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st);
+        return launch_eta<OP, KIND, T, 16, 32, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st);
     }
-    if (dir == 0) {
-        const T idx = inv_spacing<T>(OpShape<OP>::h2, nx);
-        const int64_t nseg = (nx + kThreads * K - 1) / (kThreads * K);
-        const int64_t items = nbatch * ((ny + kXiRows - 1) / kXiRows) * nseg;
-        const int grid = (int)(items < blocks_cap ? items : blocks_cap);
-        const bool vec_ok = (nx % K == 0) && (bstride % K == 0) && (reinterpret_cast<uintptr_t>(out) % 16 == 0) &&
-                            (reinterpret_cast<uintptr_t>(in) % 16 == 0);
-        op_xi_kernel<OP, KIND, T><<<grid, kThreads, 0, st>>>(in, out, (int)ny, (int)nx, nbatch, bstride, idx, vec_ok);
-    } else {
-        const T idx = inv_spacing<T>(OpShape<OP>::h2, ny);
-        const int simd = (int)(simd_lanes<T>() * (nx / simd_lanes<T>()));
-        constexpr int K = 16 / sizeof(T);
-        const bool vec_ok = (nx % K == 0) && (bstride % K == 0) && (reinterpret_cast<uintptr_t>(in) % 16 == 0) &&
-                            (reinterpret_cast<uintptr_t>(out) % 16 == 0);
-        if (vec_ok) {
-            const int64_t items = nbatch * ((nx / K + kThreads - 1) / kThreads) * ((ny + kEtaRows - 1) / kEtaRows);
-            const int grid = (int)(items < blocks_cap ? items : blocks_cap);
-            op_eta_vec_kernel<OP, KIND, T><<<grid, kThreads, 0, st>>>(in, out, (int)ny, (int)nx, nbatch, bstride, idx,
-                                                                      simd);
-        } else {
-            const int64_t items = nbatch * ((nx + kThreads - 1) / kThreads) * ((ny + kEtaRows - 1) / kEtaRows);
-            const int grid = (int)(items < blocks_cap ? items : blocks_cap);
-            op_eta_kernel<OP, KIND, T><<<grid, kThreads, 0, st>>>(in, out, (int)ny, (int)nx, nbatch, bstride, idx,
-                                                                  simd);
-        }
-    }
+    constexpr int TC = xi_cols<T>();
+    const int64_t ncb = (nx + (ALIGNED ? 0 : K - 1) + TC - 1) / TC;
+    // 16 rows a tile, or 4 where that would leave SMs without a tile; as many threads per row as its
+    // vectors need, so that narrow fields take several rows at once
+    int tr = kXiRows;
+    if (nbatch * ((ny + tr - 1) / tr) * ncb < kSms) tr = 4;
+    int lpr = 7;
+    while (lpr > 3 && (K << (lpr - 1)) >= nx + K - 1) --lpr;
+    const bool vec_out = (a - reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+    const T idx = inv_spacing<T>(OpShape<OP>::h2, nx);
+    const int64_t items = nbatch * ((ny + tr - 1) / tr) * ncb;
+    op_xi_kernel<OP, KIND, T, ALIGNED><<<(unsigned)items, kThreads, xi_smem<T>(tr), st>>>(
+        in, out, (int)ny, (int)nx, bstride, idx, (int)ncb, tr, lpr, vec_out, A);
     return cudaGetLastError();
 }
 
@@ -478,8 +424,14 @@ cudaError_t launch_kind(int dir, int kind, const void* in, void* out, int64_t ny
                         int64_t bstride, cudaStream_t st) {
     const T* i = static_cast<const T*>(in);
     T* o = static_cast<T*>(out);
-    if (kind == DIFF) return launch_t<OP, DIFF, T>(dir, i, o, ny, nx, nbatch, bstride, st);
-    if constexpr (OpShape<OP>::upwind) return launch_t<OP, DISS, T>(dir, i, o, ny, nx, nbatch, bstride, st);
+    constexpr int K = 16 / sizeof(T);
+    const bool aligned = nx % K == 0 && bstride % K == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
+    auto launch = [&](auto k) {
+        return aligned ? launch_t<OP, decltype(k)::value, T, true>(dir, i, o, ny, nx, nbatch, bstride, st)
+                       : launch_t<OP, decltype(k)::value, T, false>(dir, i, o, ny, nx, nbatch, bstride, st);
+    };
+    if (kind == DIFF) return launch(std::integral_constant<int, DIFF>{});
+    if constexpr (OpShape<OP>::upwind) return launch(std::integral_constant<int, DISS>{});
     return cudaErrorInvalidValue;
 }
 

@@ -1,0 +1,50 @@
+"""The operator kernels on rows that do not start on 16-byte boundaries: odd lengths, input and output
+pointers at every element offset (equal and unequal), batches with a gap between them, the least and
+tile-edge lengths of both tile shapes.  Bit-identical to the oracle, as every operator result; the
+bytes around the output stay as they were."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+FNS = {"diffxi": (0, 0), "diffeta": (1, 0), "dissxi": (0, 1), "disseta": (1, 1)}
+SHAPES = [(16, 16), (17, 19), (33, 31), (47, 65), (49, 129), (20, 255), (18, 257), (16, 513), (130, 1027)]
+
+
+@pytest.mark.parametrize("op", [0, 2, 4, 5])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_alignments(orc, op, dtype):
+    from summationbyparts_b200 import _capi
+    np_t, t_t = (np.float64, torch.float64) if dtype == "f64" else (np.float32, torch.float32)
+    rng = np.random.default_rng(10 * op + len(dtype))
+    offsets = [(0, 0), (1, 1), (1, 0), (0, 1)] if dtype == "f64" else [(0, 0), (1, 1), (2, 2), (3, 3), (1, 2), (3, 0)]
+    for k, (ny, nx) in enumerate(SHAPES):
+        nb, gap = (1, 0) if k % 2 else (3, k)
+        stride = ny * nx + gap
+        a = rng.uniform(-1, 1, (nb, ny, nx)).astype(np_t)
+        refs = {}
+        for name, (direction, kind) in FNS.items():
+            if kind == 0 or op in (0, 2):
+                refs[name] = [orc.op_apply(op, orc.XI if direction == 0 else orc.ETA,
+                                           orc.DIFF if kind == 0 else orc.DISS, a[b]) for b in range(nb)]
+        for oi, oo in offsets:
+            total = (nb - 1) * stride + ny * nx
+            src = torch.full((total + 8,), float("nan"), dtype=t_t, device="cuda")
+            for b in range(nb):
+                src[oi + b * stride:oi + b * stride + ny * nx] = torch.from_numpy(a[b].ravel()).cuda()
+            for name, ref in refs.items():
+                dst = torch.full((total + 8,), 7.0, dtype=t_t, device="cuda")
+                size = src.element_size()
+                _capi.check(getattr(_capi.lib, "sbp_" + name)(
+                    op, _capi.F64 if dtype == "f64" else _capi.F32, src.data_ptr() + oi * size,
+                    dst.data_ptr() + oo * size, ny, nx, nb, stride,
+                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+                out = dst.cpu().numpy()
+                want = np.full(total + 8, 7.0, dtype=np_t)
+                for b in range(nb):
+                    want[oo + b * stride:oo + b * stride + ny * nx] = ref[b].ravel()
+                assert out.tobytes() == want.tobytes(), (name, ny, nx, oi, oo)
