@@ -135,7 +135,9 @@ class _Library:
     def __getattr__(self, name):
         if _Library._handle is None:
             _Library._handle = _load()
-        return getattr(_Library._handle, name)
+        f = getattr(_Library._handle, name)
+        setattr(self, name, f)  # later lookups find it on the instance
+        return f
 
 
 lib = _Library()

@@ -23,36 +23,44 @@ from . import _capi
 UPWIND4, UPWIND4H2, UPWIND9, UPWIND9H2, SBP4_ID, SBP8_ID = range(6)
 
 
-def _dtype_code(t) -> int:
+_DTYPES: dict = {}  # torch dtype -> C dtype code, filled on first use (torch is imported lazily)
+
+
+def _setup():
     import torch
 
-    if t.dtype == torch.float64:
-        return _capi.F64
-    if t.dtype == torch.float32:
-        return _capi.F32
-    raise TypeError(f"unsupported dtype {t.dtype}")
+    _DTYPES.update({torch.float64: _capi.F64, torch.float32: _capi.F32})
+    global _raw_stream
+    # handle of the current stream of a device; the public call builds a Stream object each time
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+        lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def _launch(fn, op_id: int, prev, fut) -> None:
-    import torch
-
-    if prev.shape != fut.shape:
-        raise ValueError(f"prev {tuple(prev.shape)} and fut {tuple(fut.shape)} must have the same shape")
-    if prev.dtype != fut.dtype:
+    if not _DTYPES:
+        _setup()
+    shape, dtype = prev.shape, prev.dtype
+    if shape != fut.shape:
+        raise ValueError(f"prev {tuple(shape)} and fut {tuple(fut.shape)} must have the same shape")
+    if dtype != fut.dtype:
         raise ValueError("prev and fut must have the same dtype")
     if not (prev.is_cuda and fut.is_cuda):
         raise ValueError("prev and fut must be CUDA tensors")
     if not (prev.is_contiguous() and fut.is_contiguous()):
         raise ValueError("prev and fut must be contiguous")
-    if prev.dim() == 2:
-        nb, (ny, nx) = 1, prev.shape
-    elif prev.dim() == 3:
-        nb, ny, nx = prev.shape
+    rank = len(shape)
+    if rank == 2:
+        nb, (ny, nx) = 1, shape
+    elif rank == 3:
+        nb, ny, nx = shape
     else:
         raise ValueError("expected (ny, nx) or (batch, ny, nx)")
-    stream = torch.cuda.current_stream(prev.device).cuda_stream
-    _capi.check(fn(op_id, _dtype_code(prev), prev.data_ptr(), fut.data_ptr(), ny, nx, nb, ny * nx,
-                   ctypes.c_void_p(stream)))
+    code = _DTYPES.get(dtype)
+    if code is None:
+        raise TypeError(f"unsupported dtype {dtype}")
+    status = fn(op_id, code, prev.data_ptr(), fut.data_ptr(), ny, nx, nb, ny * nx, _raw_stream(prev.device.index))
+    if status:
+        _capi.check(status)
 
 
 class SbpOperator1dInfo:
