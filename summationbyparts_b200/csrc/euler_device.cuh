@@ -72,6 +72,7 @@ struct InstanceDev {
     // the free-stream pressure and 1 / (gamma - 1).
     double vk_b[5], vk_u[5], vk_f[5];
     double v_pinf, v_igm1;
+    int v_regular;  // every vortex has a radius (1 / r*^2 is finite)
 };
 
 // pressure (euler/src/lib.rs:478-480)
@@ -138,8 +139,8 @@ __device__ inline void vortex_point(const InstanceDev& I, double gamma, double t
 }
 
 // vortex_point<true> for gamma = 1.4 with the instance constants precomputed on the host
-// (InstanceDev::vk_*) and no division: the boundary data of compensated-f32 systems, whose f64
-// SAT terms need not follow the reference's operation order (values differ in the last bits).
+// (InstanceDev::vk_*) and no division: the boundary data of the SATs (values differ from the
+// reference's in the last bits).
 __device__ inline void vortex_point_fast(const InstanceDev& I, double t, double x, double y, double q[4]) {
     const double p_inf = I.v_pinf, igm1 = I.v_igm1;
     const double e_inf = p_inf * igm1 + 0.5;  // rho_inf = u_inf = 1, v_inf = 0
@@ -173,59 +174,6 @@ __device__ inline void vortex_point_fast(const InstanceDev& I, double t, double 
             q[3] += en - e_inf;
         }
     }
-}
-
-// SAT_characteristic (euler/src/lib.rs:1150-1252) at one edge point, f64:
-// k += hi*tau * T * ((L + sign|L|) o (T^-1 (y - z))).
-__device__ inline void sat_point(double gamma, const double y[4], const double z[4], double hi, double sign,
-                                 double tau, double detj, double detj_d_dx, double detj_d_dy, double k[4]) {
-    const double rho = y[0], rhou = y[1], rhov = y[2], e = y[3];
-    const double kx_ = detj_d_dx / detj;
-    const double ky_ = detj_d_dy / detj;
-    const double r = hypot(kx_, ky_);
-    const double kx = kx_ / r, ky = ky_ / r;
-    const double u = rhou / rho, v = rhov / rho;
-    const double theta = kx * u + ky * v;
-    const double p = pressure<double>(gamma, rho, rhou, rhov, e);
-    const double c = sqrt(gamma * p / rho);
-    const double phi2 = (gamma - 1.0) * (u * u + v * v) / 2.0;
-    const double SQRT_2 = 1.41421356237309504880;
-    const double alpha = rho / (SQRT_2 * c);
-    const double phi2_c2 = (phi2 + c * c) / (gamma - 1.0);
-    const double T[4][4] = {
-        {1.0, 0.0, alpha, alpha},
-        {u, ky, alpha * (u + kx * c), alpha * (u - kx * c)},
-        {v, -kx, alpha * (v + ky * c), alpha * (v - ky * c)},
-        {phi2 / (gamma - 1.0), rho * (ky * u - kx * v), alpha * (phi2_c2 + c * theta), alpha * (phi2_c2 - c * theta)},
-    };
-    const double U = kx_ * u + ky_ * v;
-    const double hyp = hypot(kx_, ky_);
-    const double L[4] = {U, U, U + c * hyp, U - c * hyp};
-    const double beta = 1.0 / (2.0 * c * c);
-    const double TI[4][4] = {
-        {1.0 - phi2 / (c * c), (gamma - 1.0) * u / (c * c), (gamma - 1.0) * v / (c * c), -(gamma - 1.0) / (c * c)},
-        {-(ky * u - kx * v) / rho, ky / rho, -kx / rho, 0.0},
-        {beta * (phi2 - c * theta), beta * (kx * c - (gamma - 1.0) * u), beta * (ky * c - (gamma - 1.0) * v),
-         beta * (gamma - 1.0)},
-        {beta * (phi2 + c * theta), -beta * (kx * c + (gamma - 1.0) * u), -beta * (ky * c + (gamma - 1.0) * v),
-         beta * (gamma - 1.0)},
-    };
-    const double res[4] = {rho - z[0], rhou - z[1], rhov - z[2], e - z[3]};
-    double TIres[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int row = 0; row < 4; ++row)
-#pragma unroll
-        for (int col = 0; col < 4; ++col) TIres[row] += TI[row][col] * res[col];
-    double LTIres[4];
-#pragma unroll
-    for (int row = 0; row < 4; ++row) LTIres[row] = (L[row] + sign * fabs(L[row])) * TIres[row];
-    double TLTIres[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int row = 0; row < 4; ++row)
-#pragma unroll
-        for (int col = 0; col < 4; ++col) TLTIres[row] += T[row][col] * LTIres[col];
-#pragma unroll
-    for (int comp = 0; comp < 4; ++comp) k[comp] += hi * tau * TLTIres[comp];
 }
 
 // Knuth's TwoSum: s + e == a + b exactly (round-to-nearest, no FMA involved).

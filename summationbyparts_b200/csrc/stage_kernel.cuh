@@ -14,7 +14,7 @@
 // store their k in the edge-k buffer instead; the edge kernel (sat_kernel, launched right after
 // on the same stream) adds the characteristic SATs in the order north, south, east, west
 // (SAT_characteristics, euler/src/lib.rs:1002-1013) and does their update.  The SAT of one
-// point is a long dependent f64 chain (vortex data, two hypot, a dozen divisions); evaluated by
+// point is a long dependent f64 chain (vortex data, roots, reciprocals); evaluated by
 // a few threads of a tile it held the whole CTA at the next barrier, in a launch of its own it
 // runs one thread per edge point.
 //
@@ -77,13 +77,12 @@ struct StageArgs {
     T* new_hi;               // new state (stage 3)
     T* new_lo;
     T* kedge;                // k of block-edge points, 4 per point (edge_index order per block)
-    const double* egeo;      // compensated f32: edge geometry, kEdgeGeo per point (edge_geo_kernel)
+    const double* egeo;      // edge geometry, kEdgeGeo per point (edge_geo_kernel)
     const int4* mg;          // MultiGrid segments (block, start, end, -) of all block sides
     const EvalDev* eval;     // expression programs of SBP_BC_EVAL sides
     double* evz;             // SBP_BC_EVAL data of the launch's edge points (eval_kernel), 4 per point
     const T* met;            // metric planes in T
     const T* jinv;           // f64: 1 / J planes (BlockDev::r_off)
-    const double* met64;     // metric planes in f64 (SAT terms)
     const float* rinf;       // compensated f32, upwind: free-stream dissipation planes (BlockDev::r_off)
     const double* xy;        // coordinates
     double gamma;
@@ -110,78 +109,11 @@ constexpr int region_extent(int T, int H, int M, int N) {
 __device__ __forceinline__ int tile_rows(const int4& td) { return td.w >> 16; }
 __device__ __forceinline__ int tile_cols(const int4& td) { return td.w & 0xffff; }
 
-// Characteristic SAT of one edge point (euler/src/lib.rs:1150-1252), f64, written row by row
-// so no 4x4 matrix is ever live.  Same operations in the same order as the reference.
-__device__ __forceinline__ void sat_point_rows(double gamma, const double y[4], const double z[4], double hi,
-                                               double sign, double tau, double detj, double detj_d_dx,
-                                               double detj_d_dy, double k[4]) {
-    const double rho = y[0], rhou = y[1], rhov = y[2], e = y[3];
-    const double kx_ = detj_d_dx / detj;
-    const double ky_ = detj_d_dy / detj;
-    const double r = hypot(kx_, ky_);
-    const double kx = kx_ / r, ky = ky_ / r;
-    const double u = rhou / rho, v = rhov / rho;
-    const double theta = kx * u + ky * v;
-    const double p = pressure<double>(gamma, rho, rhou, rhov, e);
-    const double c = sqrt(gamma * p / rho);
-    const double phi2 = (gamma - 1.0) * (u * u + v * v) / 2.0;
-    const double alpha = rho / (1.41421356237309504880 * c);
-    const double phi2_c2 = (phi2 + c * c) / (gamma - 1.0);
-    const double U = kx_ * u + ky_ * v;
-    const double hyp = hypot(kx_, ky_);
-    const double beta = 1.0 / (2.0 * c * c);
-    const double cc = c * c, gm1 = gamma - 1.0;
-    const double r0 = rho - z[0], r1 = rhou - z[1], r2 = rhov - z[2], r3 = e - z[3];
-    double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-    t0 += (1.0 - phi2 / cc) * r0;
-    t0 += (gm1 * u / cc) * r1;
-    t0 += (gm1 * v / cc) * r2;
-    t0 += (-gm1 / cc) * r3;
-    t1 += (-(ky * u - kx * v) / rho) * r0;
-    t1 += (ky / rho) * r1;
-    t1 += (-kx / rho) * r2;
-    t1 += 0.0 * r3;
-    t2 += (beta * (phi2 - c * theta)) * r0;
-    t2 += (beta * (kx * c - gm1 * u)) * r1;
-    t2 += (beta * (ky * c - gm1 * v)) * r2;
-    t2 += (beta * gm1) * r3;
-    t3 += (beta * (phi2 + c * theta)) * r0;
-    t3 += (-beta * (kx * c + gm1 * u)) * r1;
-    t3 += (-beta * (ky * c + gm1 * v)) * r2;
-    t3 += (beta * gm1) * r3;
-    const double L0 = U, L2 = U + c * hyp, L3 = U - c * hyp;
-    const double l0 = (L0 + sign * fabs(L0)) * t0;
-    const double l1 = (L0 + sign * fabs(L0)) * t1;
-    const double l2 = (L2 + sign * fabs(L2)) * t2;
-    const double l3 = (L3 + sign * fabs(L3)) * t3;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    s0 += 1.0 * l0;
-    s0 += 0.0 * l1;
-    s0 += alpha * l2;
-    s0 += alpha * l3;
-    s1 += u * l0;
-    s1 += ky * l1;
-    s1 += (alpha * (u + kx * c)) * l2;
-    s1 += (alpha * (u - kx * c)) * l3;
-    s2 += v * l0;
-    s2 += (-kx) * l1;
-    s2 += (alpha * (v + ky * c)) * l2;
-    s2 += (alpha * (v - ky * c)) * l3;
-    s3 += (phi2 / gm1) * l0;
-    s3 += (rho * (ky * u - kx * v)) * l1;
-    s3 += (alpha * (phi2_c2 + c * theta)) * l2;
-    s3 += (alpha * (phi2_c2 - c * theta)) * l3;
-    const double ht = hi * tau;
-    k[0] += ht * s0;
-    k[1] += ht * s1;
-    k[2] += ht * s2;
-    k[3] += ht * s3;
-}
-
-// sat_point_rows with five reciprocals in place of its divisions and sqrt(kx^2 + ky^2) in place
-// of hypot (no overflow at these magnitudes): the SAT of compensated-f32 systems, still f64, whose
-// last bits need not follow the reference's operation order.
-__device__ __forceinline__ void sat_point_fast(double gamma, const double y[4], const double z[4], double hi,
+// Characteristic SAT of one edge point (SAT_characteristic, euler/src/lib.rs:1150-1252), f64:
+// k += hi tau T ((L + sign |L|) o (T^-1 (y - z))), written row by row so no 4x4 matrix is ever
+// live, with five reciprocals in place of the reference's divisions and sqrt(kx^2 + ky^2) in place of
+// hypot (no overflow at these magnitudes).  igm1 = 1 / (gamma - 1).
+__device__ __forceinline__ void sat_point(double gamma, const double y[4], const double z[4], double hi,
                                                double sign, double tau, double detj, double detj_d_dx,
                                                double detj_d_dy, double igm1, double k[4]) {
     const double rho = y[0], rhou = y[1], rhov = y[2], e = y[3];
@@ -416,32 +348,23 @@ __device__ __forceinline__ double absolute_state(const StageArgs<T>& A, const Bl
 struct EdgeGeo {
     double x, y, m[5];
 };
-// Compensated-f32 systems gather the geometry of their block-edge points once into one contiguous
-// 64-byte record per point (slot e_off + edge_index: x, y, detJ, the 4 metric terms, padding;
-// edge_geo_kernel), which the edge kernel reads instead of seven scattered sectors (the first and
-// last columns of a block are nx elements apart).
+// A schedule gathers the geometry of its block-edge points once into one contiguous 64-byte record per
+// point (slot e_off + edge_index: x, y, detJ, the 4 metric terms, padding; edge_geo_kernel), which
+// the SATs read instead of seven scattered sectors (the first and last columns of a block are nx
+// elements apart).
 constexpr int kEdgeGeo = 8;
-template <class T>
-__device__ __forceinline__ EdgeGeo edge_geo(const StageArgs<T>& A, const BlockDev& B, int pt) {
-    const int64_t np = B.npad;
-    const double* m64 = A.met64 + B.m_off;
-    const double* xy = A.xy + B.x_off;
-    EdgeGeo g;
-    g.x = xy[pt];
-    g.y = xy[np + pt];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) g.m[c] = m64[c * np + pt];
-    return g;
+__device__ __forceinline__ EdgeGeo edge_record(const double* p) {
+    const double2* gp = reinterpret_cast<const double2*>(p);
+    const double2 g0 = gp[0], g1 = gp[1], g2 = gp[2], g3 = gp[3];
+    return EdgeGeo{g0.x, g0.y, {g1.x, g1.y, g2.x, g2.y, g3.x}};
 }
 
-// SATs of one block-edge point in the reference's order N, S, E, W; k updated in place.
+// Sum of the SATs of one block-edge point in the reference's order N, S, E, W, added to kv.
 template <class T>
 __device__ __forceinline__ void sat_edge(const StageArgs<T>& A, const InstanceDev& I, const BlockDev& B, int eidx, int row,
                                       int col, const EdgeGeo& geo, const double yv[4], double kv[4]) {
     const int nx = B.nx, ny = B.ny;
     const bool on[4] = {row == ny - 1, row == 0, col == nx - 1, col == 0};
-    // compensated-f32 systems: division-free SAT arithmetic and vortex data (gamma = 1.4)
-    constexpr bool FAST = sizeof(T) == 4;
     const double cst = A.stage == kStageK ? A.ctime : (A.stage == 0 ? 0.0 : (A.stage == 3 ? 1.0 : 0.5));
     const double stime = cst == 0.0 ? I.time : I.time + I.dt * cst;
     for (int d = 0; d < 4; ++d) {
@@ -449,7 +372,7 @@ __device__ __forceinline__ void sat_edge(const StageArgs<T>& A, const InstanceDe
         double zv[4];
         const int kind = B.bc_kind[d];
         if (kind == BC_VORTEX) {
-            if (FAST && A.gamma == 1.4)
+            if (A.gamma == 1.4 && (sizeof(T) == 4 || I.v_regular))
                 vortex_point_fast(I, stime, geo.x, geo.y, zv);
             else
                 vortex_point<true>(I, A.gamma, stime, geo.x, geo.y, zv);
@@ -517,10 +440,7 @@ __device__ __forceinline__ void sat_edge(const StageArgs<T>& A, const InstanceDe
         const double hi = ns ? B.hi_eta : B.hi_xi;
         const double ddx = ns ? geo.m[3] : geo.m[1];
         const double ddy = ns ? geo.m[4] : geo.m[2];
-        if constexpr (FAST)
-            sat_point_fast(A.gamma, yv, zv, hi, sign, tau, geo.m[0], ddx, ddy, I.v_igm1, kv);
-        else
-            sat_point_rows(A.gamma, yv, zv, hi, sign, tau, geo.m[0], ddx, ddy, kv);
+        sat_point(A.gamma, yv, zv, hi, sign, tau, geo.m[0], ddx, ddy, I.v_igm1, kv);
     }
 }
 
@@ -1064,39 +984,11 @@ __global__ void __launch_bounds__(kSatThreads, 4) sat_kernel(const StageArgs<T> 
         yv[cc] = absolute_state<T>(A, B, cc, qs[cc]);
         kv[cc] = double(A.kedge[slot + cc]);
     }
-    EdgeGeo geo;
-    if (sizeof(T) == 4 && A.egeo) {
-        const double2* gp = reinterpret_cast<const double2*>(A.egeo + kEdgeGeo * (B.e_off + edge_index(row, col, nx, ny)));
-        const double2 g0 = gp[0], g1 = gp[1], g2 = gp[2], g3 = gp[3];
-        geo.x = g0.x;
-        geo.y = g0.y;
-        geo.m[0] = g1.x;
-        geo.m[1] = g1.y;
-        geo.m[2] = g2.x;
-        geo.m[3] = g2.y;
-        geo.m[4] = g3.x;
-    } else {
-        geo = edge_geo(A, B, pt);
-    }
-    sat_edge<T>(A, I, B, i, row, col, geo, yv, kv);
+    const EdgeGeo geo = edge_record(A.egeo + kEdgeGeo * (B.e_off + edge_index(row, col, nx, ny)));
+    double sv[4] = {0.0, 0.0, 0.0, 0.0};
+    sat_edge<T>(A, I, B, i, row, col, geo, yv, sv);
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) rk_update<T, COMP>(A, qoff + cc * np + pt, qs[cc], T(kv[cc]), cb, ca);
-}
-
-// Edge geometry of a group's edge points (edges[i] = block, row, col) at their slots.
-template <class T>
-__global__ void edge_geo_kernel(const StageArgs<T> A, const int4* __restrict__ edges, int nedges, double* __restrict__ geo) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nedges) return;
-    const int4 ed = edges[i];
-    const BlockDev& B = A.blocks[ed.x];
-    const EdgeGeo g = edge_geo(A, B, ed.y * B.nx + ed.z);
-    double* o = geo + kEdgeGeo * (B.e_off + edge_index(ed.y, ed.z, B.nx, B.ny));
-    o[0] = g.x;
-    o[1] = g.y;
-#pragma unroll
-    for (int c = 0; c < 5; ++c) o[2 + c] = g.m[c];
-    o[7] = 0.0;
+    for (int cc = 0; cc < 4; ++cc) rk_update<T, COMP>(A, qoff + cc * np + pt, qs[cc], T(kv[cc] + sv[cc]), cb, ca);
 }
 
 // Expression boundary data (SBP_BC_EVAL sides) of a stage launch's edge points (edges[i] =

@@ -81,6 +81,23 @@ size_t stage_smem_host(int prec, int opx, int opy, bool upw, int ty) {
     return (size_t)tile_smem(ty, upw, prec == 0 ? 8 : 4, (ox.D - 1) / 2, ox.M, ox.N, (oy.D - 1) / 2, oy.M, oy.N);
 }
 
+// Edge geometry of a group's edge points (edges[i] = block, row, col) at their slots.
+__global__ void edge_geo_kernel(const BlockDev* __restrict__ blocks, const double* __restrict__ met64,
+                                const double* __restrict__ xy, const int4* __restrict__ edges, int nedges,
+                                double* __restrict__ geo) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nedges) return;
+    const int4 ed = edges[i];
+    const BlockDev& B = blocks[ed.x];
+    const int64_t np = B.npad, pt = (int64_t)ed.y * B.nx + ed.z;
+    double* o = geo + kEdgeGeo * (B.e_off + edge_index(ed.y, ed.z, B.nx, B.ny));
+    o[0] = xy[B.x_off + pt];
+    o[1] = xy[B.x_off + np + pt];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) o[2 + c] = met64[B.m_off + c * np + pt];
+    o[7] = 0.0;
+}
+
 struct Group {
     int opx, opy;
     bool upw;
@@ -159,7 +176,7 @@ struct sbp_system {
     double* d_sums = nullptr;
     unsigned long long* d_speeds = nullptr;
     void* kedge = nullptr;   // k of block-edge points between the stage and the edge kernel
-    double* egeo = nullptr;   // compensated f32: edge geometry (kEdgeGeo per point, edge_geo_kernel)
+    double* egeo = nullptr;   // edge geometry (kEdgeGeo per point, edge_geo_kernel)
     int64_t nedge = 0;
     int4* d_mg = nullptr;    // MultiGrid segments of all block sides
     EvalDev* d_eval = nullptr;  // expression programs of SBP_BC_EVAL sides
@@ -310,6 +327,9 @@ void set_reference(InstanceDev& I, double gamma) {
     const double m = I.mach, p_inf = 1.0 / (gamma * m * m);
     I.v_pinf = p_inf;
     I.v_igm1 = 1.0 / (gamma - 1.0);
+    I.v_regular = 1;
+    for (int k = 0; k < I.nvort; ++k)
+        if (!(I.rstar[k] * I.rstar[k] > 0.0)) I.v_regular = 0;
     for (int k = 0; k < 5; ++k) {
         const double rs2 = I.rstar[k] * I.rstar[k];
         I.vk_f[k] = rs2 > 0.0 ? 1.0 / rs2 : 0.0;
@@ -340,7 +360,6 @@ StageArgs<T> stage_args(sbp_system* s, int stage, const Group& g) {
     a.new_lo = static_cast<T*>(s->prev_lo);
     a.met = s->prec == 0 ? reinterpret_cast<const T*>(s->met64) : reinterpret_cast<const T*>(s->met32);
     a.jinv = s->prec == 0 ? reinterpret_cast<const T*>(s->jinv64) : nullptr;
-    a.met64 = s->met64;
     a.rinf = s->rinf;
     a.xy = s->xy;
     a.kedge = static_cast<T*>(s->kedge);
@@ -609,12 +628,10 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
             SBP_TRY_CUDA(cudaMemcpyAsync(g.d_edges, edges[gi].data(), g.nedges * sizeof(int4),
                                          cudaMemcpyHostToDevice, s->stream));
             if (s->has_eval) SBP_TRY_CUDA(cudaMalloc(&g.d_evz, (size_t)g.nedges * 4 * sizeof(double)));
-            if (s->prec == 1) {
-                // the geometry of the group's edge points for the edge kernel (time-independent)
-                StageArgs<float> a = stage_args<float>(s, 0, g);
-                edge_geo_kernel<float><<<(g.nedges + 127) / 128, 128, 0, s->stream>>>(a, g.d_edges, g.nedges, s->egeo);
-                SBP_TRY_CUDA(cudaGetLastError());
-            }
+            // the geometry of the group's edge points for their SATs (time-independent)
+            edge_geo_kernel<<<(g.nedges + 127) / 128, 128, 0, s->stream>>>(s->d_blocks, s->met64, s->xy, g.d_edges,
+                                                                           g.nedges, s->egeo);
+            SBP_TRY_CUDA(cudaGetLastError());
         }
     }
     SBP_TRY_CUDA(cudaStreamSynchronize(s->stream));
@@ -1049,9 +1066,7 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
     e = e ?: alloc((void**)&s->d_sums, (size_t)nblocks * (1 + kNormParts) * sizeof(double));
     e = e ?: alloc((void**)&s->d_speeds, 2 * nblocks * sizeof(unsigned long long));
     e = e ?: alloc(&s->kedge, 4 * s->nedge * ts);
-    if (s->prec == 1) {
-        e = e ?: alloc((void**)&s->egeo, kEdgeGeo * s->nedge * sizeof(double));
-    }
+    e = e ?: alloc((void**)&s->egeo, kEdgeGeo * s->nedge * sizeof(double));
     e = e ?: alloc((void**)&s->d_mg, (mg_host.size() + 1) * sizeof(int4));
     e = e ?: alloc((void**)&s->d_eval, sizeof(EvalDev));
     if (e != cudaSuccess) return fail(cuda_status(e, "device allocation"));
