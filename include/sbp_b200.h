@@ -262,12 +262,14 @@ sbp_status sbp_system_error(sbp_system* sys, double* per_instance);
 sbp_status sbp_system_h2_err(sbp_system* sys, int block, const double* q, double* err);
 
 /* Tile schedule: output tiles of ty x tx points per CTA, `threads` threads per CTA
- * (0 = keep), for every operator group; clears the autotuner's per-group choices.
+ * (0 = keep), for every operator group; clears the autotuner's per-group choices.  Until it is
+ * called, a system too small to fill the GPU takes the fused form of the stage kernel (tiles of
+ * 8 x 16 or 16 x 32 points, the SATs in the stage launches); f64 results do not depend on the form.
  * sbp_system_autotune searches, per operator group, the tile rows (16, 32) and the width of the
  * stage kernel's grid (as many persistent CTAs per SM as fit, one per SM, or one CTA per tile),
  * timing whole RK4 steps on the current state (state and time are restored) by coordinate
  * descent over the groups, and keeps the fastest; it returns the tile shape of the group with
- * the most points. */
+ * the most points.  It starts from the current schedule, a small system's fused form included. */
 sbp_status sbp_system_set_tiles(sbp_system* sys, int ty, int tx, int threads);
 sbp_status sbp_system_autotune(sbp_system* sys, int* ty, int* tx, int* threads);
 /* Schedule of one operator group: tile rows, persistent CTAs per SM (-1 = as many as fit,
@@ -305,7 +307,7 @@ sbp_status sbp_system_advance_tableau(sbp_system* sys, int tableau, int64_t nste
 sbp_status sbp_system_advance_adaptive(sbp_system* sys, double dt, double* guess_dt, double maxerr);
 
 /* Kernel launches per RK4 step: per operator pair and stage a stage kernel and an edge (SAT)
- * kernel, plus the time update. */
+ * kernel, plus the time update; four per operator pair in the fused form of small systems. */
 int sbp_system_launches_per_step(const sbp_system* sys);
 
 /* Per-kernel measurement.  A system's blocks are scheduled in groups, one per operator pair

@@ -4,8 +4,10 @@
 namespace sbp {
 // prec 0 = f64, 1 = f32 compensated; ty = tile rows (16 or 32); sc = RK stage class (0: stage 0,
 // 1: stages 1 and 2, 2: stage 3), which only the compensated 32-row kernel is specialised on.
+// ty | kTileFused: the fused form with the SATs (8 or 16 rows; pairs of one family).
 // Returns the kernel entry (a __global__ function pointer usable with cudaLaunchKernel) or
 // nullptr if not built.
+constexpr int kTileFused = 64;
 const void* stage_kernel_ptr(int prec, int opx, int opy, bool upw, int ty, int sc);
 
 const void* stage_ptr_f64_u4(int opx, int opy, bool upw, int ty, int sc);

@@ -11,7 +11,7 @@ namespace sbp {
 // 16-row tiles: stage_kernel; 32-row tiles: the 2 x 2 micro-tile kernel.
 #define CASE(OX, OY, UPW)                                                                          \
     if (opx == OX && opy == OY && upw == UPW) {                                                     \
-        if (ty == 16) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, float, UPW, true, 16>); \
+        if (ty == 16) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, float, UPW, true, 16, false>); \
         if (ty == kVecRows) return vec_entry<OX, OY, UPW>(sc);   \
     }
 

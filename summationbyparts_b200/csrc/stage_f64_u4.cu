@@ -6,25 +6,40 @@ namespace sbp {
 
 #define CASE(OX, OY, UPW, TYV)                                   \
     if (opx == OX && opy == OY && upw == UPW && ty == TYV)        \
-        return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, TYV>);
+        return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, TYV, false>);
+
+// the fused form
+#define FUSED(OX, OY, UPW)                                                                                          \
+    if (opx == OX && opy == OY && upw == UPW && ty == (8 | kTileFused))                                             \
+        return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 8, true>);                   \
+    if (opx == OX && opy == OY && upw == UPW && ty == (16 | kTileFused))                                            \
+        return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 16, true>);
 
 const void* stage_ptr_f64_u4(int opx, int opy, bool upw, int ty, int sc) {
     (void)sc;  // the f64 kernels take the stage at run time
     CASE(UPWIND4, UPWIND4, true, 16)
+    FUSED(UPWIND4, UPWIND4, true)
     CASE(UPWIND4, UPWIND4, true, 32)
     CASE(UPWIND4, UPWIND4, false, 16)
+    FUSED(UPWIND4, UPWIND4, false)
     CASE(UPWIND4, UPWIND4, false, 32)
     CASE(UPWIND4H2, UPWIND4H2, true, 16)
+    FUSED(UPWIND4H2, UPWIND4H2, true)
     CASE(UPWIND4H2, UPWIND4H2, true, 32)
     CASE(UPWIND4H2, UPWIND4H2, false, 16)
+    FUSED(UPWIND4H2, UPWIND4H2, false)
     CASE(UPWIND4H2, UPWIND4H2, false, 32)
     CASE(UPWIND4, UPWIND4H2, true, 16)
+    FUSED(UPWIND4, UPWIND4H2, true)
     CASE(UPWIND4, UPWIND4H2, true, 32)
     CASE(UPWIND4, UPWIND4H2, false, 16)
+    FUSED(UPWIND4, UPWIND4H2, false)
     CASE(UPWIND4, UPWIND4H2, false, 32)
     CASE(UPWIND4H2, UPWIND4, true, 16)
+    FUSED(UPWIND4H2, UPWIND4, true)
     CASE(UPWIND4H2, UPWIND4, true, 32)
     CASE(UPWIND4H2, UPWIND4, false, 16)
+    FUSED(UPWIND4H2, UPWIND4, false)
     CASE(UPWIND4H2, UPWIND4, false, 32)
     return nullptr;
 }

@@ -9,8 +9,8 @@ namespace sbp {
 
 #define CASE(OX, OY, UPW)                                                                           \
     if (opx == OX && opy == OY && upw == UPW) {                                                      \
-        if (ty == 16) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 16>); \
-        if (ty == 32) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 32>); \
+        if (ty == 16) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 16, false>); \
+        if (ty == 32) return reinterpret_cast<const void*>(&stage_kernel<OX, OY, double, UPW, false, 32, false>); \
     }
 
 const void* stage_ptr_f64_xsb(int opx, int opy, bool upw, int ty, int sc) {

@@ -87,6 +87,11 @@ struct StageArgs {
     const double* xy;        // coordinates
     double gamma;
     unsigned* status;
+    // fused form, stage 3 of a step: CTAs of all groups (0: the launch advances no time), their counter,
+    // and the instances to advance
+    int time_ctas, ninst;
+    unsigned* time_done;
+    const int* active;
 };
 
 // Stage index of the k-only mode: the launch computes k = RHS(u_in) (SATs included) into u_out
@@ -282,50 +287,6 @@ __device__ __forceinline__ void rk_update_ops(const StageArgs<T>& A, int64_t e, 
     }
 }
 
-// This stage's RK4 update of one component at element e (see the header comment), operands
-// read from global memory.  `qv` is the stage input at the point (the step-start state in
-// stage 0); cb, ca: this stage's B and A tableau entries times dt (ca unused in stage 3).
-template <class T, bool COMP>
-__device__ __forceinline__ void rk_update(const StageArgs<T>& A, int64_t e, T qv, T kc, double cb, double ca) {
-    if (A.stage == kStageK) {
-        A.u_out[e] = kc;
-        return;
-    }
-    if constexpr (!COMP) {
-        const T cbt = T(cb);
-        if (A.stage == 0) {
-            A.acc_hi[e] = qv + cbt * kc;
-            A.u_out[e] = qv + T(ca) * kc;
-        } else if (A.stage < 3) {
-            const T av = A.acc_hi[e];
-            const T pv = __ldg(A.prev_hi + e);
-            A.acc_hi[e] = av + cbt * kc;
-            A.u_out[e] = pv + T(ca) * kc;
-        } else {
-            A.new_hi[e] = A.acc_hi[e] + cbt * kc;
-        }
-    } else {
-        // compensated form: see rk_update_staged
-        const float cbf = float(cb);
-        const float kf = float(kc);
-        if (A.stage == 0) {
-            A.u_out[e] = T(float(qv) + float(ca) * kf);
-            A.acc_hi[e] = T(cbf * kf);
-        } else if (A.stage < 3) {
-            const float pv = float(__ldg(A.prev_hi + e));
-            A.u_out[e] = T(pv + float(ca) * kf);
-            A.acc_hi[e] = T(float(A.acc_hi[e]) + cbf * kf);
-        } else {
-            const float d = float(A.acc_hi[e]) + cbf * kf;
-            float hi = float(A.prev_hi[e]);
-            float lo = float(A.prev_lo[e]);
-            comp_add(hi, lo, d);
-            A.new_hi[e] = T(hi);
-            A.new_lo[e] = T(lo);
-        }
-    }
-}
-
 // Element of a block's edge opposite to side d (north -> the block's south row, ...) at position
 // k along that edge: the point whose state a neighbour's side-d SAT reads.
 __device__ __forceinline__ int opposite_edge_point(int d, int k, int gnx, int gny) {
@@ -359,23 +320,46 @@ __device__ __forceinline__ EdgeGeo edge_record(const double* p) {
     return EdgeGeo{g0.x, g0.y, {g1.x, g1.y, g2.x, g2.y, g3.x}};
 }
 
-// Sum of the SATs of one block-edge point in the reference's order N, S, E, W, added to kv.
+// The sides of a block on which an edge point lies (at most two of N, S, E, W, in that order; -1: none),
+// and the vortex data at the point if one of them takes those: what its SATs need beside the state.
+struct SatSides {
+    int d[2];
+    double z[4];
+};
 template <class T>
-__device__ __forceinline__ void sat_edge(const StageArgs<T>& A, const InstanceDev& I, const BlockDev& B, int eidx, int row,
-                                      int col, const EdgeGeo& geo, const double yv[4], double kv[4]) {
-    const int nx = B.nx, ny = B.ny;
-    const bool on[4] = {row == ny - 1, row == 0, col == nx - 1, col == 0};
+__device__ __forceinline__ SatSides sat_sides(const StageArgs<T>& A, const InstanceDev& I, const BlockDev& B, int row,
+                                              int col, const EdgeGeo& geo) {
     const double cst = A.stage == kStageK ? A.ctime : (A.stage == 0 ? 0.0 : (A.stage == 3 ? 1.0 : 0.5));
     const double stime = cst == 0.0 ? I.time : I.time + I.dt * cst;
-    for (int d = 0; d < 4; ++d) {
-        if (!on[d]) continue;
+    const int ns = row == B.ny - 1 ? NORTH : (row == 0 ? SOUTH : -1);
+    const int ew = col == B.nx - 1 ? EAST : (col == 0 ? WEST : -1);
+    SatSides s{};
+    s.d[0] = ns >= 0 ? ns : ew;
+    s.d[1] = ns >= 0 ? ew : -1;
+    if ((s.d[0] >= 0 && B.bc_kind[s.d[0]] == BC_VORTEX) || (s.d[1] >= 0 && B.bc_kind[s.d[1]] == BC_VORTEX)) {
+        if (A.gamma == 1.4 && (sizeof(T) == 4 || I.v_regular))
+            vortex_point_fast(I, stime, geo.x, geo.y, s.z);
+        else
+            vortex_point<true>(I, A.gamma, stime, geo.x, geo.y, s.z);
+    }
+    return s;
+}
+
+// Sum of the SATs of one block-edge point in the reference's order N, S, E, W, added to kv.
+template <class T>
+__device__ __forceinline__ void sat_apply(const StageArgs<T>& A, const InstanceDev& I, const BlockDev& B, int eidx, int row,
+                                          int col, const EdgeGeo& geo, const SatSides& side, const double yv[4],
+                                          double kv[4]) {
+    const int nx = B.nx, ny = B.ny;
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        const int d = k == 0 ? side.d[0] : side.d[1];
+        if (d < 0) continue;
         double zv[4];
         const int kind = B.bc_kind[d];
         if (kind == BC_VORTEX) {
-            if (A.gamma == 1.4 && (sizeof(T) == 4 || I.v_regular))
-                vortex_point_fast(I, stime, geo.x, geo.y, zv);
-            else
-                vortex_point<true>(I, A.gamma, stime, geo.x, geo.y, zv);
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) zv[cc] = side.z[cc];
         } else if (kind == BC_EVAL) {
             // BoundaryCharacteristic::Eval (euler/src/lib.rs:853-863): the expressions at the stage
             // time, evaluated for this edge point by eval_kernel just before
@@ -665,10 +649,85 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
 }
+// Programmatic dependent launch: returns once every earlier kernel of the chain has completed and
+// its writes are visible; only then may the kernel's own successor start.
+__device__ __forceinline__ void dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <int OPX, int OPY, class T, bool UPW, bool COMP, int TY>
-__global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 : 2) stage_kernel(const StageArgs<T> A) {
+// The SAT threads of the fused form: the tiles of the CTA in the order of the stencil threads, one edge
+// point per thread, its SAT terms into ssat (slot: tile column on a horizontal edge, TX + tile row on a
+// vertical one).  Two barriers per tile with the stencil threads: terms ready, terms used.
+template <int MX, int MY, class T, int TY>
+__device__ __forceinline__ void sat_tiles(const StageArgs<T>& A, double* __restrict__ ssat) {
+    constexpr int TX = tile_tx(TY);
+    const int lane = threadIdx.x - kStageThreads;
+    bool waited = false;
+    for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
+        const int4 td = A.tiles[t];
+        const BlockDev& B = A.blocks[td.x];
+        const int nx = B.nx, ny = B.ny, y0 = td.y, x0 = td.z, th = tile_rows(td), tw = tile_cols(td);
+        if ((x0 < MX && x0 + tw > nx - MX) || (y0 < MY && y0 + th > ny - MY)) return;  // as the stencil threads
+        const bool top = y0 == 0, bot = y0 + th == ny, left = x0 == 0, right = x0 + tw == nx;
+        const int nh = top || bot ? tw : 0, nv = left || right ? th : 0;
+        int row = -1, col = -1;
+        if (lane < nh) {
+            row = top ? 0 : ny - 1;
+            col = x0 + lane;
+        } else if (lane < nh + nv) {
+            row = y0 + lane - nh;
+            col = left ? 0 : nx - 1;
+            if (nh && row == (top ? 0 : ny - 1)) row = -1;  // the corner is in the row
+        }
+        const InstanceDev& I = A.inst[B.instance];
+        EdgeGeo geo{};
+        SatSides side{};
+        if (row >= 0) {
+            geo = edge_record(A.egeo + kEdgeGeo * (B.e_off + edge_index(row, col, nx, ny)));
+            side = sat_sides(A, I, B, row, col, geo);
+        }
+        if (!waited) {
+            dependency_wait();
+            waited = true;
+        }
+        if (row >= 0) {
+            const T* q = A.u_in + B.q_off + row * nx + col;
+            double yv[4], sv[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) yv[cc] = absolute_state<T>(A, B, cc, q[cc * (int64_t)B.npad]);
+            sat_apply<T>(A, I, B, 0, row, col, geo, side, yv, sv);
+            const int slot = row == 0 || row == ny - 1 ? col - x0 : TX + row - y0;
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) ssat[4 * slot + cc] = sv[cc];
+        }
+        __syncthreads();
+        __syncthreads();
+    }
+    if (!waited) dependency_wait();
+}
+
+// Threads of the fused form that evaluate the SATs: one per edge point of a tile, which lies on at
+// most one horizontal and one vertical block edge.
+__host__ __device__ constexpr int sat_threads(int ty) { return ty + tile_tx(ty) <= 32 ? 32 : 64; }
+
+// Barrier of the kStageThreads stencil threads (all threads where there are no others).
+__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStageThreads) : "memory"); }
+
+// SATF: the fused form for systems that leave SMs without work (see fused_rows in system.cu).  The
+// SATs of a tile's edge points are evaluated in the same launch by threads of their own, beside the
+// stencils, instead of an edge kernel after it, and the last CTA of stage 3 advances the instance
+// times: a step is four launches instead of nine.
+// The stage launches of a step after its first are dependent ones: what does not depend on the stage
+// input -- the metric rows, the edge geometry, the vortex boundary data -- is fetched and evaluated
+// before the predecessor has finished, and a kernel lets its successor start only after its own
+// wait, so that such early work sees the finished step before it.
+//   Measured, us per step, separate -> fused: one 64 x 64 Upwind4 block 64 -> 21 (f64), 64 -> 21
+// (compensated); six Upwind9 blocks of 37,310 points 70 -> 39 and 68 -> 35.
+template <int OPX, int OPY, class T, bool UPW, bool COMP, int TY, bool SATF>
+__global__ void __launch_bounds__(kStageThreads + (SATF ? sat_threads(TY) : 0),
+                                  SATF || (TY == 32 && sizeof(T) == 8) ? 1 : 2) stage_kernel(const StageArgs<T> A) {
     using G = TileGeom<OPX, OPY, TY, T>;
     using V = typename PairOf<T>::type;
     constexpr int TX = G::TX, MR = G::MR, MC = G::MC, XA = G::XA, YA = G::YA, RP = G::RP, EP = G::EP, RH = G::RH;
@@ -682,6 +741,10 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
     T* rx = rq + 4 * RH * RP;                // [2][TY][RP]: raw xi metrics of the tile rows
     T* re = rx + 2 * TY * RP;                // [2][RH][EP]: raw eta metrics of the tile columns
     T* fl = re + 2 * RH * EP;                // fluxes of one direction: [UPW ? 8 : 4] xi or eta arrays
+    // SATF: the SAT terms of the tile's edge points, one row of points then one column
+    double* ssat = reinterpret_cast<double*>(smem_raw + tile_smem(TY, UPW, sizeof(T), OpShape<OPX>::H, OpShape<OPX>::M,
+                                                                  OpShape<OPX>::N, OpShape<OPY>::H, OpShape<OPY>::M,
+                                                                  OpShape<OPY>::N));
     const T gamma = T(A.gamma);
     const int tid = threadIdx.x;
     const int comp = tid >> 6, gx = tid & 7, gy = (tid >> 3) & 7;  // stencil phases
@@ -690,7 +753,8 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
     // Starts the asynchronous copies of one tile's raw rows: every row of the region's state planes,
     // the xi metrics of the tile rows and the eta metrics of the tile columns, a warp per row, in
     // 16-byte pieces widened to 16-byte boundaries (a plane's padding holds the overhang).
-    auto fetch = [&](const int4 td) {
+    // what: 1 = metrics, 2 = state, 3 = both.
+    auto fetch = [&](const int4 td, int what) {
         const BlockDev& B = A.blocks[td.x];
         const int nx = B.nx, np = B.npad, y0 = td.y, x0 = td.z;
         const int th = tile_rows(td), tw = tile_cols(td);
@@ -705,10 +769,12 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
             {
                 const int e = ((off + lx0) & ~(AL - 1)) + lane * AL;
                 if (e < off + lx1) {
+                    if (what & 2) {
 #pragma unroll
-                    for (int pl = 0; pl < 4; ++pl) cp_async16(rq + (pl * RH + r) * RP + lane * AL, q + pl * np + e);
+                        for (int pl = 0; pl < 4; ++pl) cp_async16(rq + (pl * RH + r) * RP + lane * AL, q + pl * np + e);
+                    }
                     const int tr = ly0 + r - y0;
-                    if (tr >= 0 && tr < th) {
+                    if ((what & 1) && tr >= 0 && tr < th) {
 #pragma unroll
                         for (int pl = 0; pl < 2; ++pl)
                             cp_async16(rx + (pl * TY + tr) * RP + lane * AL, mt + (1 + pl) * np + e);
@@ -716,7 +782,7 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 }
             }
             const int e = ((off + x0) & ~(AL - 1)) + lane * AL;
-            if (e < off + x0 + tw) {
+            if ((what & 1) && e < off + x0 + tw) {
 #pragma unroll
                 for (int pl = 0; pl < 2; ++pl) cp_async16(re + (pl * RH + r) * EP + lane * AL, mt + (3 + pl) * np + e);
             }
@@ -724,7 +790,20 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
     };
     static_assert(RP <= 32 * AL && EP <= 32 * AL, "one 16-byte piece per lane");
 
-    if (blockIdx.x < A.ntiles) fetch(A.tiles[blockIdx.x]);
+    if constexpr (SATF) {
+        if (tid >= kStageThreads) {
+            sat_tiles<MX, MY, T, TY>(A, ssat);
+            return;
+        }
+    }
+    if (blockIdx.x < A.ntiles) {
+        const int4 td = A.tiles[blockIdx.x];
+        fetch(td, 1);
+        dependency_wait();
+        fetch(td, 2);
+    } else {
+        dependency_wait();
+    }
 
     for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
         const int4 td = A.tiles[t];
@@ -754,8 +833,40 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
             return;
         }
         const bool xi_pre = left_cl || right_cl, eta_pre = top_cl || bot_cl;
+        // Operands of the update pass for this thread's points (coalesced: consecutive threads take
+        // consecutive columns); the fused form, which has the registers, loads them here, the other just
+        // before they are used:
+        // 1 / J, the free-stream plane, and up to three state arrays.
+        constexpr int NOP = COMP ? 3 : 2;
+        T jinv[PPT], rv[PPT], op[NOP][PPT][CPT];
+        int pe[PPT];  // element of the point in a plane (-1: not in the tile)
+        const int uc = PTS >= kStageThreads ? 0 : (tid / PTS) * CPT;  // first component
+        const T* src[3] = {A.stage == 0 ? A.u_in + qoff : A.acc_hi + qoff, A.prev_hi + qoff, A.prev_lo + qoff};
+        const int nsrc = A.stage == kStageK ? 0 : (A.stage == 0 ? 1 : (A.stage < 3 ? 2 : (COMP ? 3 : 1)));
+        const T* ji = COMP ? A.met + B.m_off : A.jinv + roff;
+        auto load_operands = [&]() {
+#pragma unroll
+            for (int i = 0; i < PPT; ++i) {
+                const int p = tid % (PTS < kStageThreads ? PTS : kStageThreads) + i * kStageThreads;
+                const int ur = p / TX, ux = p % TX;
+                pe[i] = ur < th && ux < tw ? (y0 + ur) * nx + x0 + ux : -1;
+                jinv[i] = T(1);
+                rv[i] = T(0);
+                if (pe[i] >= 0) {
+                    jinv[i] = __ldg(ji + pe[i]);
+                    if constexpr (COMP && UPW) rv[i] = __ldg(A.rinf + roff + pe[i]);
+#pragma unroll
+                    for (int a = 0; a < NOP; ++a)
+#pragma unroll
+                        for (int cc = 0; cc < CPT; ++cc)
+                            op[a][i][cc] = a < nsrc ? src[a][(uc + cc) * np + pe[i]] : T(0);
+                }
+            }
+        };
+        if constexpr (SATF) load_operands();
+
         cp_async_wait_all();
-        __syncthreads();
+        tile_sync();
 
         // ---------------- xi fluxes of the tile rows, widened by the xi halo ----------------
         {
@@ -776,7 +887,7 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 }
             }
         }
-        __syncthreads();
+        tile_sync();
 
         // the next tile, its block descriptor brought near for fetch
         const int tn = t + (int)gridDim.x;
@@ -815,12 +926,12 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 if (right_cl) closure_part<OPX, UPW, true, PARTS, 0>(part, ld, o);
                 else closure_part<OPX, UPW, false, PARTS, 0>(part, ld, o);
             }
-            __syncthreads();
+            tile_sync();
             if (own) {
 #pragma unroll
                 for (int i = 0; i < CNT; ++i) fl[(cc * MX + part * CNT + i) * TY + r] = o[i];
             }
-            __syncthreads();
+            tile_sync();
             if (active) {
 #pragma unroll
                 for (int j = 0; j < MC; ++j) {
@@ -832,7 +943,7 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 }
             }
         }
-        __syncthreads();
+        tile_sync();
 
         // ---------------- eta fluxes of the tile columns, widened by the eta halo ----------------
         for (int p = tid; p < (ly1 - ly0) * TX; p += kStageThreads) {
@@ -851,20 +962,10 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 }
             }
         }
-        __syncthreads();
+        tile_sync();
         // the raw rows are no longer needed: the next tile's copies run from here on
-        if (tn < A.ntiles) fetch(ntd);
+        if (tn < A.ntiles) fetch(ntd, 3);
 
-        // Operands of the update pass for this thread's points (coalesced: consecutive threads take
-        // consecutive columns), loaded before the eta sums so that their latency is hidden:
-        // 1 / J, the free-stream plane, and up to three state arrays.
-        constexpr int NOP = COMP ? 3 : 2;
-        T jinv[PPT], rv[PPT], op[NOP][PPT][CPT];
-        int pe[PPT];  // element of the point in a plane (-1: not in the tile)
-        const int uc = PTS >= kStageThreads ? 0 : (tid / PTS) * CPT;  // first component
-        const T* src[3] = {A.stage == 0 ? A.u_in + qoff : A.acc_hi + qoff, A.prev_hi + qoff, A.prev_lo + qoff};
-        const int nsrc = A.stage == kStageK ? 0 : (A.stage == 0 ? 1 : (A.stage < 3 ? 2 : (COMP ? 3 : 1)));
-        const T* ji = COMP ? A.met + B.m_off : A.jinv + roff;
         // ---------------- eta sums ----------------
         if (active) {
             const T* ec = fl + comp * YA + (r0 + G::YL - HY) * TX;
@@ -883,12 +984,12 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 if (bot_cl) closure_part<OPY, UPW, true, PARTS, 0>(part, ld, o);
                 else closure_part<OPY, UPW, false, PARTS, 0>(part, ld, o);
             }
-            __syncthreads();
+            tile_sync();
             if (own) {
 #pragma unroll
                 for (int i = 0; i < CNT; ++i) fl[(cc * MY + part * CNT + i) * TX + col] = o[i];
             }
-            __syncthreads();
+            tile_sync();
             if (active) {
 #pragma unroll
                 for (int u = 0; u < MR; ++u) {
@@ -900,7 +1001,7 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 }
             }
         }
-        __syncthreads();
+        tile_sync();
         // the sums through shared memory to the update pass
         if (active) {
 #pragma unroll
@@ -914,24 +1015,9 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 if constexpr (MC == 4) o[TX / 4 + (gx ^ 4)] = {s[2], s[3]};
             }
         }
-#pragma unroll
-        for (int i = 0; i < PPT; ++i) {
-            const int p = tid % (PTS < kStageThreads ? PTS : kStageThreads) + i * kStageThreads;
-            const int ur = p / TX, ux = p % TX;
-            pe[i] = ur < th && ux < tw ? (y0 + ur) * nx + x0 + ux : -1;
-            jinv[i] = T(1);
-            rv[i] = T(0);
-            if (pe[i] >= 0) {
-                jinv[i] = __ldg(ji + pe[i]);
-                if constexpr (COMP && UPW) rv[i] = __ldg(A.rinf + roff + pe[i]);
-#pragma unroll
-                for (int a = 0; a < NOP; ++a)
-#pragma unroll
-                    for (int cc = 0; cc < CPT; ++cc)
-                        op[a][i][cc] = a < nsrc ? src[a][(uc + cc) * np + pe[i]] : T(0);
-            }
-        }
-        __syncthreads();
+        if constexpr (!SATF) load_operands();
+        if constexpr (SATF) __syncthreads();  // the SAT terms are there
+        else tile_sync();
 
         // ---------------- update pass ----------------
         // Interior points finish; points on a block edge store k for the edge kernel.
@@ -947,14 +1033,42 @@ __global__ void __launch_bounds__(kStageThreads, TY == 32 && sizeof(T) == 8 ? 1 
                 T k = fl[(uc + cc) * PTS + ur * TX + G::epos(ux)] * jinv[i];
                 if constexpr (COMP && UPW) k = fma_rn(I.ref.q[uc + cc], rv[i], k);
                 const int64_t e = qoff + (uc + cc) * np + pe[i];
-                if (edge) A.kedge[4 * (eoff + edge_index(row, col, nx, ny)) + uc + cc] = k;
-                else rk_update_ops<T, COMP>(A, e, cb, ca, k, op[0][i][cc], op[1][i][cc], COMP ? op[NOP - 1][i][cc] : T(0));
+                if (edge) {
+                    if constexpr (SATF) {
+                        const int slot = row == 0 || row == ny - 1 ? ux : TX + ur;
+                        k = T(double(k) + ssat[4 * slot + uc + cc]);
+                    } else {
+                        A.kedge[4 * (eoff + edge_index(row, col, nx, ny)) + uc + cc] = k;
+                        continue;
+                    }
+                }
+                rk_update_ops<T, COMP>(A, e, cb, ca, k, op[0][i][cc], op[1][i][cc], COMP ? op[NOP - 1][i][cc] : T(0));
             }
         }
-        // Every thread is done with the flux buffer before the next tile's fluxes.
-        __syncthreads();
+        // Every thread is done with the flux buffer (and the SAT terms) before the next tile's.
+        if constexpr (SATF) __syncthreads();
+        else tile_sync();
     }
     if (bad) atomicOr(A.status, bad);
+    if constexpr (SATF) {
+        // stage 3: the last CTA of the step's groups advances the times of the active instances; the SAT
+        // threads have read them before the last barrier
+        if (A.time_ctas > 0) {
+            __shared__ bool last;
+            tile_sync();
+            if (tid == 0) {
+                __threadfence();
+                last = atomicAdd(A.time_done, 1u) == (unsigned)A.time_ctas - 1u;
+            }
+            tile_sync();
+            if (last) {
+                InstanceDev* inst = const_cast<InstanceDev*>(A.inst);
+                for (int i = tid; i < A.ninst; i += kStageThreads)
+                    if (A.active[i]) inst[i].time = inst[i].time + inst[i].dt;
+                if (tid == 0) *A.time_done = 0u;
+            }
+        }
+    }
 }
 
 // Edge kernel: one thread per block-edge point of a stage launch's blocks (edges[i] = block,
@@ -972,11 +1086,14 @@ __global__ void __launch_bounds__(kSatThreads, 4) sat_kernel(const StageArgs<T> 
     const int nx = B.nx, ny = B.ny;
     const int64_t np = B.npad, qoff = B.q_off;
     const int64_t slot = 4 * (B.e_off + edge_index(row, col, nx, ny));
-    const double cb = A.stage < 4 ? I.cb[A.stage] : 0.0;
-    const double ca = A.stage < 3 ? I.ca[A.stage] : 0.0;
+    const T cb = T(A.stage < 4 ? I.cb[A.stage] : 0.0);
+    const T ca = T(A.stage < 3 ? I.ca[A.stage] : 0.0);
     const int pt = row * nx + col;
     const T* q = A.u_in + qoff;
-    double yv[4], kv[4];
+    const EdgeGeo geo = edge_record(A.egeo + kEdgeGeo * (B.e_off + edge_index(row, col, nx, ny)));
+    const SatSides side = sat_sides(A, I, B, row, col, geo);
+    dependency_wait();
+    double yv[4], kv[4], sv[4] = {0.0, 0.0, 0.0, 0.0};
     T qs[4];  // the stored stage input (a deviation in the compensated form)
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc) {
@@ -984,11 +1101,19 @@ __global__ void __launch_bounds__(kSatThreads, 4) sat_kernel(const StageArgs<T> 
         yv[cc] = absolute_state<T>(A, B, cc, qs[cc]);
         kv[cc] = double(A.kedge[slot + cc]);
     }
-    const EdgeGeo geo = edge_record(A.egeo + kEdgeGeo * (B.e_off + edge_index(row, col, nx, ny)));
-    double sv[4] = {0.0, 0.0, 0.0, 0.0};
-    sat_edge<T>(A, I, B, i, row, col, geo, yv, sv);
+    sat_apply<T>(A, I, B, i, row, col, geo, side, yv, sv);
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) rk_update<T, COMP>(A, qoff + cc * np + pt, qs[cc], T(kv[cc] + sv[cc]), cb, ca);
+    for (int cc = 0; cc < 4; ++cc) {
+        // the operands of the update pass of stage_kernel
+        const int64_t e = qoff + cc * np + pt;
+        T o0 = qs[cc], o1 = T(0), o2 = T(0);
+        if (A.stage != 0 && A.stage != kStageK) {
+            o0 = A.acc_hi[e];
+            if (COMP || A.stage < 3) o1 = A.prev_hi[e];
+            if (COMP && A.stage == 3) o2 = A.prev_lo[e];
+        }
+        rk_update_ops<T, COMP>(A, e, cb, ca, T(kv[cc] + sv[cc]), o0, o1, o2);
+    }
 }
 
 // Expression boundary data (SBP_BC_EVAL sides) of a stage launch's edge points (edges[i] =
@@ -997,6 +1122,7 @@ __global__ void __launch_bounds__(kSatThreads, 4) sat_kernel(const StageArgs<T> 
 template <class T>
 __global__ void __launch_bounds__(kSatThreads) eval_kernel(const StageArgs<T> A, const int4* __restrict__ edges,
                                                            int nedges) {
+    dependency_wait();
     const int i = blockIdx.x * kSatThreads + threadIdx.x;
     if (i >= nedges) return;
     const int4 ed = edges[i];

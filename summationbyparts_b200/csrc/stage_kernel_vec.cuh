@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) stage_kernel_vec(const Stage
     }
     // RK operand arrays (stage_operands): stage 0 u_in; stages 1, 2 acc_hi, prev_hi; stage 3 also prev_lo
     constexpr int NSRC = SC + 1;
+    dependency_wait();
     const float* src[3] = {SC == 0 ? A.u_in : A.acc_hi, A.prev_hi, A.prev_lo};
 
     for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {

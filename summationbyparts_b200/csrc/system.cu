@@ -103,6 +103,7 @@ struct Group {
     bool upw;
     const void* fn[3];  // stage kernel per RK stage class (vec_stage_class); the same entry thrice
                         // for kernels that take the stage at run time
+    bool fused = false; // the SATs are part of the stage kernel (its fused form)
     int4* d_tiles = nullptr;
     int ntiles = 0;
     int4* d_edges = nullptr;  // (block, row, col) of every edge point of the group's blocks
@@ -122,6 +123,7 @@ struct TileChoice {
     int opx, opy;
     bool upw;
     int ty, ctas;
+    bool fused;
 };
 
 // One chunk of sbp_system_advance_host: the blocks [b0, b1) (whole instances), their own step
@@ -186,6 +188,7 @@ struct sbp_system {
     // schedule
     int TY = 16, TX = kTileX, threads = kStageThreads;
     std::vector<TileChoice> tile_choice;  // per operator group; groups not listed use (TY, -1)
+    bool tiles_auto = true;               // until a caller chooses: small systems take the fused form
     int tiles_gen = 0;                    // bumped whenever the tile schedule changes
     std::vector<int> active;
     std::vector<Group> groups;
@@ -372,31 +375,59 @@ StageArgs<T> stage_args(sbp_system* s, int stage, const Group& g) {
     return a;
 }
 
-sbp_status launch_group(sbp_system* s, int stage, const Group& g, cudaStream_t st, bool edges_too = true) {
-    if (g.ntiles == 0) return SBP_OK;
-    cudaError_t e;
-    const void* sat = s->prec == 0 ? sat_ptr_f64() : sat_ptr_f32();
-    const dim3 sat_grid((g.nedges + kSatThreads - 1) / kSatThreads);
+// Advance of the instance times by the fused stage kernels of a step (StageArgs::time_ctas).
+struct TimeAdvance {
+    int ctas = 0;
+    const int* active = nullptr;  // ninst flags, then the counter
+};
+
+template <class T>
+cudaError_t launch_group_t(sbp_system* s, int stage, const Group& g, cudaStream_t st, bool edges_too, bool dependent,
+                           const TimeAdvance& ta) {
+    StageArgs<T> a = stage_args<T>(s, stage, g);
+    if (g.fused && stage == 3 && ta.ctas > 0) {
+        a.time_ctas = ta.ctas;
+        a.ninst = s->ninst;
+        a.active = ta.active;
+        a.time_done = reinterpret_cast<unsigned*>(const_cast<int*>(ta.active) + s->ninst);
+    }
+    // A dependent launch may begin while the stream's previous kernel drains (dependency_wait).  Stage
+    // kernels are; edge kernels are not: their early CTAs cost the separate f64 stage kernel the tail of its
+    // launch (one 700 x 700 Upwind9 block 180 instead of 183 us a step, the f64 ensemble 2-3%).
+    auto launch = [&](const void* fn, int grid, int threads, void** args, size_t smem, bool dep) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = dep ? 1 : 0;
+        return cudaLaunchKernelExC(&cfg, fn, args);
+    };
+    void* args[] = {&a};
+    const int threads = s->threads + (g.fused ? sat_threads(g.ty) : 0);
+    cudaError_t e = launch(g.fn[vec_stage_class(stage)], g.grid, threads, args, g.smem, dependent);
+    if (g.fused || !edges_too) return e;
+    const int sat_grid = (g.nedges + kSatThreads - 1) / kSatThreads;
     int4* edges = g.d_edges;
     int nedges = g.nedges;
-    const void* evk = s->prec == 0 ? eval_ptr_f64() : eval_ptr_f32();
-    if (s->prec == 0) {
-        StageArgs<double> a = stage_args<double>(s, stage, g);
-        void* args[] = {&a};
-        e = cudaLaunchKernel(g.fn[vec_stage_class(stage)], dim3(g.grid), dim3(s->threads), args, g.smem, st);
-        void* sargs[] = {&a, &edges, &nedges};
-        if (e == cudaSuccess && edges_too && s->has_eval)
-            e = cudaLaunchKernel(evk, sat_grid, dim3(kSatThreads), sargs, 0, st);
-        if (e == cudaSuccess && edges_too) e = cudaLaunchKernel(sat, sat_grid, dim3(kSatThreads), sargs, 0, st);
-    } else {
-        StageArgs<float> a = stage_args<float>(s, stage, g);
-        void* args[] = {&a};
-        e = cudaLaunchKernel(g.fn[vec_stage_class(stage)], dim3(g.grid), dim3(s->threads), args, g.smem, st);
-        void* sargs[] = {&a, &edges, &nedges};
-        if (e == cudaSuccess && edges_too && s->has_eval)
-            e = cudaLaunchKernel(evk, sat_grid, dim3(kSatThreads), sargs, 0, st);
-        if (e == cudaSuccess && edges_too) e = cudaLaunchKernel(sat, sat_grid, dim3(kSatThreads), sargs, 0, st);
-    }
+    void* sargs[] = {&a, &edges, &nedges};
+    if (e == cudaSuccess && s->has_eval)
+        e = launch(s->prec == 0 ? eval_ptr_f64() : eval_ptr_f32(), sat_grid, kSatThreads, sargs, 0, false);
+    if (e == cudaSuccess) e = launch(s->prec == 0 ? sat_ptr_f64() : sat_ptr_f32(), sat_grid, kSatThreads, sargs, 0, false);
+    return e;
+}
+
+// One stage of one group: the stage kernel and, unless its form includes the SATs, the edge kernel.
+// dependent: the stream's previous operation is a kernel of this group's previous stage.
+sbp_status launch_group(sbp_system* s, int stage, const Group& g, cudaStream_t st, bool edges_too = true,
+                        bool dependent = false, const TimeAdvance& ta = {}) {
+    if (g.ntiles == 0) return SBP_OK;
+    const cudaError_t e = s->prec == 0 ? launch_group_t<double>(s, stage, g, st, edges_too, dependent, ta)
+                                       : launch_group_t<float>(s, stage, g, st, edges_too, dependent, ta);
     return cuda_status(e, "stage kernel launch");
 }
 
@@ -505,7 +536,7 @@ const Tableau* tableau_of(int id) {
 // Returns the starts followed by n.
 std::vector<int> tile_starts(int n, int T, int M) {
     std::vector<int> b;
-    const int e = (n - M) & ~1;
+    const int e = T > M ? (n - M) & ~1 : n - M;  // (tiles of M rows hold exactly the closure)
     bool moved = false;
     for (int x = 0; x < n; x += T) {
         if (x <= e) b.push_back(x);
@@ -517,10 +548,37 @@ std::vector<int> tile_starts(int n, int T, int M) {
     return b;
 }
 
+// The tile rows of the fused stage kernel for a system that leaves SMs without work, 0 where the other
+// forms are better.  The fused kernel evaluates the SATs beside the stencils, saves the edge and time
+// launches and overlaps successive stages, but runs one CTA an SM.  Measured per step (Upwind9 f64,
+// one vortex block; 8-row tiles, 16-row tiles, the separate form): 128^2 (128 tiles of 8 rows) 30,
+// 37, 60 us; 160^2 (200) 41, 37, 60; 350^2 (242 tiles of 16 rows) -, 64, 76; 400^2 (325) -, 88, 101;
+// 500^2 (512) -, 115, 111.  So 8 rows while their tiles fit the SMs at once, 16 rows up to three tiles
+// an SM.
+// The rule goes by all blocks of the system and not by the instances or the chunk at hand, so every
+// schedule of a system takes the same form.  Expression sides need their own kernel, and pairs of
+// operators of two families are not instantiated.
+int fused_rows(const sbp_system* s) {
+    if (!s->tiles_auto || s->has_eval) return 0;
+    for (int ty : {8, 16}) {
+        int64_t tiles = 0;
+        for (const BlockDev& B : s->hb) {
+            OpInfo ox, oy;
+            op_info(B.op_xi, ox);
+            op_info(B.op_eta, oy);
+            const bool upw = ox.upwind && oy.upwind && !s->force_trad;
+            if (!stage_kernel_ptr(s->prec, B.op_xi, B.op_eta, upw, ty | kTileFused, 0)) return 0;
+            tiles += (int64_t)(tile_starts(B.ny, ty, oy.M).size() - 1) * (tile_starts(B.nx, tile_tx(ty), ox.M).size() - 1);
+        }
+        if (tiles <= (ty == 8 ? 1 : 3) * (int64_t)s->num_sms) return ty;
+    }
+    return 0;
+}
+
 sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const int* d_active,
                             std::vector<Group>& groups, cudaGraph_t& graph_out, cudaGraphExec_t& gexec_out) {
     free_group_list(groups, graph_out, gexec_out);
-    const int TX = s->TX;
+    const int fused = fused_rows(s);
     for (int b = 0; b < s->nblocks; ++b) {
         const BlockDev& B = s->hb[b];
         if (!active[B.instance]) continue;
@@ -536,13 +594,16 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
             g.opx = B.op_xi;
             g.opy = B.op_eta;
             g.upw = upw;
-            g.ty = s->TY;
+            g.ty = fused ? fused : s->TY;
+            g.fused = fused != 0;
             for (const TileChoice& c : s->tile_choice)
                 if (c.opx == g.opx && c.opy == g.opy && c.upw == g.upw) {
                     g.ty = c.ty;
                     g.ctas = c.ctas;
+                    g.fused = c.fused;
                 }
-            for (int sc = 0; sc < 3; ++sc) g.fn[sc] = stage_kernel_ptr(s->prec, B.op_xi, B.op_eta, upw, g.ty, sc);
+            for (int sc = 0; sc < 3; ++sc)
+                g.fn[sc] = stage_kernel_ptr(s->prec, B.op_xi, B.op_eta, upw, g.ty | (g.fused ? kTileFused : 0), sc);
             if (!g.fn[0] || !g.fn[1] || !g.fn[2]) {
                 set_error("operator pair (xi %d, eta %d) is not built into the stage kernels", B.op_xi, B.op_eta);
                 return SBP_ERR_UNSUPPORTED;
@@ -565,7 +626,7 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
             if (groups[gi].opx == B.op_xi && groups[gi].opy == B.op_eta && groups[gi].upw == upw) break;
         group_of[b] = (int)gi;
         Group& g = groups[gi];
-        const int TY = g.ty;
+        const int TY = g.ty, TX = tile_tx(TY);
         const std::vector<int> ys = tile_starts(B.ny, TY, oy.M), xs = tile_starts(B.nx, TX, ox.M);
         for (size_t iy = 0; iy + 1 < ys.size(); ++iy)
             for (size_t ix = 0; ix + 1 < xs.size(); ++ix) {
@@ -588,13 +649,15 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
         Group& g = groups[gi];
         const int TY = g.ty;
         g.ntiles = (int)tiles[gi].size();
-        g.smem = stage_smem_host(s->prec, g.opx, g.opy, g.upw, TY);
+        const int TX = tile_tx(TY);
+        g.smem = stage_smem_host(s->prec, g.opx, g.opy, g.upw, TY) + (g.fused ? 4 * (TX + TY) * sizeof(double) : 0);
+        const int threads = s->threads + (g.fused ? sat_threads(TY) : 0);
         {
             OpInfo ox, oy;
             op_info(g.opx, ox);
             op_info(g.opy, oy);
             // every region fits the kernel's fixed shared-memory geometry
-            if (g.WX > region_extent(kTileX, (ox.D - 1) / 2, ox.M, ox.N) ||
+            if (g.WX > region_extent(TX, (ox.D - 1) / 2, ox.M, ox.N) ||
                 g.HY > region_extent(TY, (oy.D - 1) / 2, oy.M, oy.N)) {
                 set_error("internal: tile region exceeds the shared-memory geometry");
                 return SBP_ERR_INVALID_ARGUMENT;
@@ -608,12 +671,11 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
         for (int sc = 0; sc < 3; ++sc) {
             SBP_TRY_CUDA(cudaFuncSetAttribute(g.fn[sc], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
             int n = 0;
-            SBP_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, g.fn[sc], s->threads, g.smem));
+            SBP_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, g.fn[sc], threads, g.smem));
             per_sm = std::min(per_sm, n);
         }
         if (per_sm < 1) {
-            set_error("stage kernel cannot be resident with %d threads and %zu bytes shared memory", s->threads,
-                      g.smem);
+            set_error("stage kernel cannot be resident with %d threads and %zu bytes shared memory", threads, g.smem);
             return SBP_ERR_INVALID_ARGUMENT;
         }
         // persistent grid of up to `ctas` CTAs per SM, or one CTA per tile (ctas == 0)
@@ -657,6 +719,15 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
                 coupled = true;
         }
     }
+    // Fused kernels advance the times themselves, if every group has one.
+    TimeAdvance ta;
+    ta.active = d_active;
+    bool all_fused = !groups.empty();
+    for (const Group& g : groups) {
+        all_fused = all_fused && g.fused;
+        ta.ctas += g.grid;
+    }
+    if (!all_fused) ta.ctas = 0;
     // Capture one RK4 step.
     SBP_TRY_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     sbp_status rc = SBP_OK;
@@ -664,25 +735,26 @@ sbp_status build_step_graph(sbp_system* s, const std::vector<int>& active, const
         cudaEventRecord(s->ev_fork, s->stream);
         for (size_t gi = 0; gi < groups.size() && rc == SBP_OK; ++gi) {
             cudaStreamWaitEvent(s->side[gi], s->ev_fork, 0);
-            for (int stage = 0; stage < 4 && rc == SBP_OK; ++stage) rc = launch_group(s, stage, groups[gi], s->side[gi]);
+            for (int stage = 0; stage < 4 && rc == SBP_OK; ++stage)
+                rc = launch_group(s, stage, groups[gi], s->side[gi], true, stage > 0, ta);
             cudaEventRecord(s->ev[gi], s->side[gi]);
         }
         for (size_t gi = 0; gi < groups.size(); ++gi) cudaStreamWaitEvent(s->stream, s->ev[gi], 0);
     }
     for (int stage = 0; stage < 4 && rc == SBP_OK && (groups.size() == 1 || coupled); ++stage) {
         if (groups.size() == 1) {
-            rc = launch_group(s, stage, groups[0], s->stream);
+            rc = launch_group(s, stage, groups[0], s->stream, true, stage > 0, ta);
         } else {
             cudaEventRecord(s->ev_fork, s->stream);
             for (size_t gi = 0; gi < groups.size() && rc == SBP_OK; ++gi) {
                 cudaStreamWaitEvent(s->side[gi], s->ev_fork, 0);
-                rc = launch_group(s, stage, groups[gi], s->side[gi]);
+                rc = launch_group(s, stage, groups[gi], s->side[gi], true, false, ta);
                 cudaEventRecord(s->ev[gi], s->side[gi]);
             }
             for (size_t gi = 0; gi < groups.size(); ++gi) cudaStreamWaitEvent(s->stream, s->ev[gi], 0);
         }
     }
-    if (rc == SBP_OK) rc = cuda_status(time_update(s->d_inst, d_active, s->ninst, s->stream), "time update");
+    if (rc == SBP_OK && !all_fused) rc = cuda_status(time_update(s->d_inst, d_active, s->ninst, s->stream), "time update");
     cudaGraph_t graph = nullptr;
     cudaError_t ee = cudaStreamEndCapture(s->stream, &graph);
     if (rc != SBP_OK) {
@@ -703,6 +775,7 @@ sbp_status build_schedule(sbp_system* s) {
     SBP_TRY_CUDA(cudaStreamSynchronize(s->stream));
     free_groups(s);
     std::vector<int> act(s->active);
+    act.push_back(0);  // the fused kernels' counter
     SBP_TRY_CUDA(cudaMemcpyAsync(s->d_active, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     SBP_TRY(build_step_graph(s, s->active, s->d_active, s->groups, s->graph, s->gexec));
     s->sched_dirty = false;
@@ -755,7 +828,9 @@ sbp_status launch_rhs(sbp_system* s, const double* u_in, double* k_out, double c
         a.u_in = u_in;
         a.u_out = k_out;
         void* args[] = {&a};
-        SBP_TRY_CUDA(cudaLaunchKernel(g.fn[0], dim3(g.grid), dim3(s->threads), args, g.smem, st));  // f64: one entry
+        const int threads = s->threads + (g.fused ? sat_threads(g.ty) : 0);
+        SBP_TRY_CUDA(cudaLaunchKernel(g.fn[0], dim3(g.grid), dim3(threads), args, g.smem, st));  // f64: one entry
+        if (g.fused) continue;
         int4* edges = g.d_edges;
         int nedges = g.nedges;
         void* sargs[] = {&a, &edges, &nedges};
@@ -1040,7 +1115,7 @@ sbp_status sbp_system_create(int device, const sbp_block_desc* blocks, int nbloc
     cudaError_t e = cudaSuccess;
     e = e ?: alloc((void**)&s->d_blocks, nblocks * sizeof(BlockDev));
     e = e ?: alloc((void**)&s->d_inst, ninstances * sizeof(InstanceDev));
-    e = e ?: alloc((void**)&s->d_active, ninstances * sizeof(int));
+    e = e ?: alloc((void**)&s->d_active, (ninstances + 1) * sizeof(int));
     e = e ?: alloc(&s->prev_hi, s->nq * ts);
     e = e ?: alloc(&s->acc_hi, s->nq * ts);
     e = e ?: alloc(&s->uA, s->nq * ts);
@@ -1394,9 +1469,10 @@ sbp_status build_chunks(sbp_system* s, int want) {
         for (int b = ch.b0; b < ch.b1; ++b) ch.active[s->hb[b].instance] = 1;
         SBP_TRY_CUDA(cudaStreamCreateWithFlags(&ch.st, cudaStreamNonBlocking));
         SBP_TRY_CUDA(cudaEventCreateWithFlags(&ch.done, cudaEventDisableTiming));
-        SBP_TRY_CUDA(cudaMalloc((void**)&ch.d_active, s->ninst * sizeof(int)));
+        SBP_TRY_CUDA(cudaMalloc((void**)&ch.d_active, (s->ninst + 1) * sizeof(int)));
         SBP_TRY_CUDA(cudaMemcpyAsync(ch.d_active, ch.active.data(), s->ninst * sizeof(int), cudaMemcpyHostToDevice,
                                      s->stream));
+        SBP_TRY_CUDA(cudaMemsetAsync(ch.d_active + s->ninst, 0, sizeof(int), s->stream));  // the fused kernels' counter
         SBP_TRY(build_step_graph(s, ch.active, ch.d_active, ch.groups, ch.graph, ch.gexec));
     }
     s->chunk_gen = s->tiles_gen;
@@ -1616,6 +1692,7 @@ sbp_status sbp_system_set_tiles(sbp_system* sys, int ty, int tx, int threads) {
     sys->TX = tx;
     sys->threads = kStageThreads;
     sys->tile_choice.clear();
+    sys->tiles_auto = false;
     ++sys->tiles_gen;
     sys->sched_dirty = true;
     return SBP_OK;
@@ -1682,9 +1759,10 @@ sbp_status sbp_system_autotune(sbp_system* sys, int* ty, int* tx, int* threads) 
     // the operator groups of the schedule
     SBP_TRY(build_schedule(sys));
     std::vector<TileChoice> choice;
-    for (const Group& g : sys->groups) choice.push_back(TileChoice{g.opx, g.opy, g.upw, g.ty, g.ctas});
+    for (const Group& g : sys->groups) choice.push_back(TileChoice{g.opx, g.opy, g.upw, g.ty, g.ctas, g.fused});
     // Candidates per group: tile rows {16, 32} x grid {as many CTAs per SM as fit, one per SM,
-    // one CTA per tile}; coordinate descent over the groups (each group's choice timed with the
+    // one CTA per tile}, from the current schedule (a small system's fused form is left only for
+    // one that is faster); coordinate descent over the groups (each group's choice timed with the
     // others at their current choice), two sweeps.
     static const int kCand[][2] = {{16, -1}, {32, -1}, {16, 1}, {32, 1}, {16, 0}, {32, 0}};
     sys->tile_choice = choice;
@@ -1693,10 +1771,11 @@ sbp_status sbp_system_autotune(sbp_system* sys, int* ty, int* tx, int* threads) 
         bool changed = false;
         for (size_t gi = 0; gi < choice.size(); ++gi) {
             for (const auto& c : kCand) {
-                if (choice[gi].ty == c[0] && choice[gi].ctas == c[1]) continue;
+                if (!choice[gi].fused && choice[gi].ty == c[0] && choice[gi].ctas == c[1]) continue;
                 std::vector<TileChoice> trial = choice;
                 trial[gi].ty = c[0];
                 trial[gi].ctas = c[1];
+                trial[gi].fused = false;
                 sys->tile_choice = trial;
                 const float ms = time_step();
                 if (ms < 0.99f * best) {  // keep a change only for a clear gain
@@ -1898,9 +1977,15 @@ int sbp_system_launches_per_step(const sbp_system* sys) {
             auto p = std::make_pair(B.op_xi, B.op_eta);
             if (std::find(pairs.begin(), pairs.end(), p) == pairs.end()) pairs.push_back(p);
         }
-        return 8 * (int)pairs.size() + 1;
+        return fused_rows(sys) ? 4 * (int)pairs.size() : (sys->has_eval ? 12 : 8) * (int)pairs.size() + 1;
     }
-    return (sys->has_eval ? 12 : 8) * (int)sys->groups.size() + 1;
+    int n = 0;
+    bool all_fused = !sys->groups.empty();
+    for (const Group& g : sys->groups) {
+        n += g.fused ? 4 : (sys->has_eval ? 12 : 8);
+        all_fused = all_fused && g.fused;
+    }
+    return n + (all_fused ? 0 : 1);
 }
 
 }  // extern "C"

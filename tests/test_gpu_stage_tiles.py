@@ -46,3 +46,39 @@ def test_one_step(orc, op, ny, nx):
         assert np.abs(results[prec, ty] - ref).max() <= bar * np.abs(ref).max(), (prec, ty)
     # the f64 sums round the same way on every tile shape
     assert results["f64", 0].tobytes() == results["f64", 16].tobytes() == results["f64", 32].tobytes()
+
+
+@pytest.mark.parametrize("case", ["block", "multiblock", "ensemble"])
+def test_fused_form(case):
+    """The fused stage kernel (SATs and times in the stage launches: the default of small systems)
+    against the separate stage and edge kernels: the same f64 states and times bit for bit, after steps
+    of every instance and after ragged ones."""
+    from summationbyparts_b200 import workloads
+    from summationbyparts_b200.system import BlockSystem
+    if case == "block":  # 8-row tiles
+        blocks, vortices, dts = workloads.Config0().blocks(), [workloads.STANDARD_VORTEX], [workloads.Config0().dt]
+    elif case == "multiblock":  # 16-row tiles, coupled blocks
+        blocks = workloads.multiblock()
+        vortices, dts = [workloads.STANDARD_VORTEX], [workloads.multiblock_dt(blocks)]
+    else:  # two operator groups on their own streams
+        insts = [i for i in workloads.ensemble_instances(60, seed=1) if i.side <= 75][:6]
+        assert {i.op_id for i in insts} == {workloads.UPWIND4, workloads.UPWIND9}
+        blocks, vortices, dts = workloads.ensemble_blocks(insts), [i.vortex for i in insts], [i.dt for i in insts]
+    out = []
+    for tiles in (0, 16):
+        g = BlockSystem(blocks, len(dts), "f64", 1.4)
+        if tiles:
+            g.set_tiles(tiles, 32)
+        for k, (v, dt) in enumerate(zip(vortices, dts)):
+            g.set_vortex(v, k)
+            g.set_dt(dt, k)
+        g.init_vortex(0.0)
+        fused = g.launches_per_step() % 4 == 0
+        assert fused == (tiles == 0)
+        g.advance(3)
+        g.advance_instances([k % 3 for k in range(len(dts))])
+        out.append((np.concatenate([g.state(b).ravel() for b in range(len(blocks))]),
+                    [g.time(k) for k in range(len(dts))]))
+        g.close()
+    assert out[0][1] == out[1][1]
+    assert out[0][0].tobytes() == out[1][0].tobytes()
