@@ -1542,10 +1542,8 @@ sbp_status sbp_system_set_time(sbp_system* sys, int instance, double t) {
     clear_error();
     if (!sys || instance >= sys->ninst) return SBP_ERR_INVALID_ARGUMENT;
     cudaSetDevice(sys->device);
-    SBP_TRY(sync_times(sys));
-    for (int i = 0; i < sys->ninst; ++i)
-        if (instance < 0 || i == instance) sys->hi[i].time = t;
-    SBP_TRY(upload_instances(sys));
+    // written on the device, where the times are advanced: the host's copies are read back before every use
+    SBP_TRY_CUDA(time_set(sys->d_inst, instance, sys->ninst, t, sys->st()));
     SBP_TRY_CUDA(cudaStreamSynchronize(sys->st()));
     return SBP_OK;
 }

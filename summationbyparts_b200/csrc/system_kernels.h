@@ -67,6 +67,8 @@ struct StageCombination {
 cudaError_t combine_stages(const BlockDev* blocks, const InstanceDev* inst, int nblocks, const double* base,
                            double* out, const StageCombination& cm, int64_t max_points, cudaStream_t st);
 
+// time[instance] = t (instance < 0: all).
+cudaError_t time_set(InstanceDev* inst, int instance, int ninst, double t, cudaStream_t st);
 // time[i] += dt[i] for the instances whose flag is set.
 cudaError_t time_update(InstanceDev* inst, const int* active, int ninst, cudaStream_t st);
 
