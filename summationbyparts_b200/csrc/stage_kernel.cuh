@@ -436,18 +436,18 @@ __host__ __device__ constexpr int tile_mr(int ty) { return ty / 8; }
 __host__ __device__ constexpr int tile_mc(int ty) { return tile_tx(ty) / 8; }
 
 // Local column of column x is x - x0 + xi_lead: room for the H halo columns, and for the N - M
-// columns before the last M that an end-closure block reads; even, so that a column's parity and
-// the alignment of its pair do not depend on the tile.  Rows have the same without the evenness.
+// columns before the last M that an end-closure block reads; xi_lead - H is even, so that every
+// thread's window starts at a pair.  Rows have the same without the evenness.
 __host__ __device__ constexpr int lead_of(int H, int M, int N) { return H > N - M ? H : N - M; }
-__host__ __device__ constexpr int xi_lead(int H, int M, int N) { return (lead_of(H, M, N) + 1) & ~1; }
+__host__ __device__ constexpr int xi_lead(int H, int M, int N) { return H + ((lead_of(H, M, N) - H + 1) & ~1); }
 // 16-byte (f64) pairs of adjacent columns that one thread's xi window spans.
 __host__ __device__ constexpr int xi_window(int ty, int H, int M, int N) {
-    return (((xi_lead(H, M, N) - H) & 1) + tile_mc(ty) + 2 * H + 1) / 2;
+    return (tile_mc(ty) + 2 * H + 1) / 2;
 }
 // Column pairs of one xi row: every region column, and every thread's window.
 __host__ __device__ constexpr int xi_pairs(int ty, int H, int M, int N) {
     const int L = xi_lead(H, M, N), a = L + (tile_tx(ty) + H > N ? tile_tx(ty) + H : N);
-    const int b = tile_tx(ty) - tile_mc(ty) + 2 * ((L - H) / 2) + 2 * xi_window(ty, H, M, N);
+    const int b = tile_tx(ty) - tile_mc(ty) + L - H + 2 * xi_window(ty, H, M, N);
     return ((a > b ? a : b) + 1) / 2;
 }
 // Pair p of a row is at slot (p & 1) * S + (p >> 1): the 8 threads of one micro-row read pairs
@@ -556,7 +556,7 @@ __device__ __forceinline__ void xi_sums(const T* __restrict__ row, int gx, T acc
             w[2 * q + 1] = v.y;
         }
 #pragma unroll
-        for (int j = 0; j < G::MC; ++j) add_taps<OP, KIND, SIGN, 0>(w + (OFF & 1) + j, acc[u][j]);
+        for (int j = 0; j < G::MC; ++j) add_taps<OP, KIND, SIGN, 0>(w + j, acc[u][j]);
     }
 }
 
