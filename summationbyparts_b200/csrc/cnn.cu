@@ -191,6 +191,7 @@ void lagrange6(const double* xs, double x, double* w) {
 
 struct sbp_cnn {
     int device = 0;
+    int num_sms = 148;
     int max_batch = 0;
     cudaStream_t own = nullptr, user = nullptr;
     bool has_user = false;
@@ -238,7 +239,9 @@ cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
         configured = true;
     }
     a.status = c->status;
-    return launch_after(conv3x3_tc_kernel<CIN, COUT, EPI>, n * (kImg / kBand), kConvThreads, bytes, c->st(), a);
+    a.bands = n * (kImg / kBand);
+    const int grid = a.bands < 2 * c->num_sms ? a.bands : 2 * c->num_sms;
+    return launch_after(conv3x3_tc_kernel<CIN, COUT, EPI>, grid, kConvThreads, bytes, c->st(), a);
 }
 
 NetParams net_params(const sbp_cnn* c) {
@@ -386,6 +389,8 @@ sbp_status sbp_cnn_create(int device, int max_batch, unsigned long long seed, sb
     sbp_cnn* c = new sbp_cnn;
     c->device = device;
     c->max_batch = max_batch;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) c->num_sms = sms;
     auto fail = [&](sbp_status s) {
         for (void* p : c->allocs) cudaFree(p);
         if (c->own) cudaStreamDestroy(c->own);

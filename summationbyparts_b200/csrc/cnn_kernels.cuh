@@ -27,8 +27,9 @@ namespace cnn {
 
 constexpr int kImg = 64;           // image side: the coarse grid
 constexpr int kPix = kImg * kImg;  // pixels per image
-constexpr int kBand = 4;           // image rows per CTA of the convolution kernel
-constexpr int kConvThreads = 256;  // 8 warps: two accumulator tiles of 128 positions at a time
+constexpr int kBand = 4;           // image rows of one band of the convolution kernel
+constexpr int kConvGroups = 3;     // groups of four epilogue warps of the convolution kernel
+constexpr int kConvThreads = 64 + 128 * kConvGroups;  // a copy warp, a product warp, the epilogue warps
 constexpr int kWgradThreads = 128; // 4 warps: one accumulator row of a 128-row tile per thread
 constexpr int kWgradRows = 4;      // image rows per CTA in the weight-gradient kernel
 
@@ -103,6 +104,10 @@ __device__ __forceinline__ void umma_commit(uint64_t* mbar) {
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
+}
+
 // Programmatic dependent launch (the kernels are launched with it, see launch_after in cnn.cu): a
 // kernel may start while its predecessor in the stream drains.  dependency_wait returns once every
 // earlier kernel has completed and its writes are visible; only then does a kernel let its own
@@ -150,26 +155,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 constexpr unsigned kStatusMmaTimeout = 1u;
 constexpr int kMmaWaitLimit = 1 << 22;  // mbarrier polls before giving up
 
-// Shared-memory layout of the tcgen05 convolution (dynamic).  A band of kBand rows with one halo row
-// on each side is one sequence of positions per channel chunk: each image row is preceded by a zero
-// position, which pads it on the left and the row before it on the right, so pixel (r, c) of the
-// band is position 1 + (r + 1) kPitch + c and the operand of tap (dy, dx) is the output's sequence
-// shifted by dy kPitch + dx.  Output position f = r kPitch + c; c = 64 is computed and dropped.
+// Shared-memory layout of the tcgen05 convolution (dynamic): the weights, then kConvStages band stages.
+// A band of kBand rows with one halo row on each side is one sequence of positions per channel chunk:
+// each image row is preceded by a zero position, which pads it on the left and the row before it on
+// the right, so pixel (r, c) of the band is position 1 + (r + 1) kPitch + c and the operand of tap
+// (dy, dx) is the output's sequence shifted by dy kPitch + dx.  Output position f = r kPitch + c; c = 64
+// is computed and dropped.
+constexpr int kConvStages = 2;
+constexpr int kConvAccs = 8;  // accumulator tiles in flight between the products and the epilogue
 template <int CIN, int COUT>
 struct ConvTcLayout {
     static constexpr int NP = COUT < 16 ? 16 : COUT;         // N of the MMA (multiple of 16 for M = 128)
-    static constexpr int HR = kBand + 2;                     // halo rows
+    static constexpr int HR = kBand + 2;                     // rows with the halo
     static constexpr int PITCH = kImg + 1;
     static constexpr int TILES = (kBand * PITCH + 127) / 128;  // M = 128 accumulator tiles (3)
-    static constexpr int TMEM_COLS = TILES * NP <= 64 ? 64 : 128;
+    static constexpr int TMEM_COLS = kConvAccs * NP;         // 256 or 128 (a power of two)
     static constexpr int POS = TILES * 128 + 2 * PITCH + 2;  // positions the operands can reach
     static constexpr int CH = CIN / 8;                       // 16-byte channel chunks per pixel
     static constexpr int PLANE = POS * 16;                   // bytes of one chunk's positions
+    static constexpr int STAGE = CH * PLANE;
     static constexpr int B_TAP = NP * CIN * 2;               // weights of one tap: [chunk][NP][8]
-    static constexpr int B_OFF = CH * PLANE;
-    static constexpr int BAR_OFF = B_OFF + 9 * B_TAP;        // mbarriers: operands, one per tile
-    static constexpr int BYTES = BAR_OFF + 8 * (TILES + 1) + 8;
-    static_assert(PLANE % 16 == 0 && BAR_OFF % 8 == 0 && HR * PITCH + 1 <= POS, "layout");
+    static constexpr int X_OFF = 9 * B_TAP;
+    static constexpr int BAR_OFF = X_OFF + kConvStages * STAGE;
+    // mbarriers: weights; per stage full, empty; per accumulator tile full, empty
+    static constexpr int BYTES = BAR_OFF + 8 * (1 + 2 * kConvStages + 2 * kConvAccs) + 8;
+    static_assert(BAR_OFF % 8 == 0 && (TMEM_COLS & (TMEM_COLS - 1)) == 0 && HR * PITCH + 1 <= POS, "layout");
 };
 
 // Weights of a convolution as one contiguous block in the order of shared memory:
@@ -190,111 +200,155 @@ struct ConvArgs {
     int64_t img_stride;
     float4 oscale;
     double* out;
+    int bands;                 // bands of all images
     unsigned* status;
 };
 
 // 3x3 convolution with zero padding as an implicit GEMM on the tcgen05 tensor cores:
 // out[p][n] = sum over taps t and input channels k of x[p + off(t)][k] * w[n][t][k],
-// off(t) = (t / 3 - 1, t % 3 - 1).  One CTA of 256 threads computes kBand = 4 image rows for all
-// output channels (N = COUT, at least 16): bulk copies bring the band's rows (1 KB per row and
-// chunk) and the layer's weights (one block) into shared memory, one thread issues the 9 x CIN / 16
-// MMAs (K = 16 each) of each of the 3 accumulator tiles and commits every tile to its own mbarrier,
-// and warp w reads lanes 32 (w % 4) .. of tiles w / 4, w / 4 + 2, ... -- one position per thread, all
-// channels -- while the later tiles are still being multiplied:
+// off(t) = (t / 3 - 1, t % 3 - 1).  Two persistent CTAs per SM keep the layer's weights (one bulk copy)
+// and take bands of kBand image rows in turn; a CTA's warps work on different bands at once:
+//   warp 0     bulk copies of a band's rows into a free stage (1 KB per row and chunk)
+//   warp 1     zeroes a row outside the image, then one thread issues the 9 x CIN / 16 MMAs (K = 16
+//              each) of each of the band's 3 accumulator tiles into a free accumulator
+//   warps 2-13 take the finished tiles in turn, four warps a tile, warp w lanes 32 (w % 4) .. -- one
+//              position per thread, all channels -- and run the epilogue:
 //   EPI_GELU   z = acc + bias -> zout (f32, if kept), gelu(z) -> yout (bf16)   (hidden layers)
 //   EPI_LINEAR acc + bias -> zout (f32, [pixel][8])                            (output layer)
 //   EPI_APPLY  as EPI_LINEAR, and coarse + y * out_scale -> out (f64 planes)
 //   EPI_DGELU  acc * gelu'(zprev) -> yout (bf16)                       (gradient of a hidden layer)
-// The band's copies, products and epilogue follow one another within a CTA, so what hides them is the
-// number of CTAs on an SM: four of 4 rows (51 KB, 128 TMEM columns) against two of 8 rows, although
-// 4 rows fill only 68% of their accumulator rows (8 rows: 81%): an apply pass of 512 states takes
-// 1.03 ms against 1.26 (16 rows, one CTA: 1.65).  The tensor pipe is the next bound (an M = 128,
-// N = 32 product takes 64 cycles, 13 us of a layer on 64 images), then memory (34 MB a layer, 67 MB
-// with pre-activations).
+// What bounds it on 64 images: the start and the drain of the launch (about 8 us of the 20), then the
+// epilogue's issue slots and the tensor pipe (an M = 128, N = 32 product takes 64 cycles, 13 us of a
+// 32 -> 32 layer), then memory (34 MB a layer, 67 MB with pre-activations).  Measured, apply pass of 512
+// states / training step on 64: one CTA per band with copies, products and epilogue in sequence, 4
+// an SM 938 / 422 us; this form 743 / 374; one CTA an SM with 8-row bands 945 / 402; three an SM with
+// one stage 755 / 394; three copies of a band, one per column offset, with no accumulator row spent
+// on padding 829 / 378 (three times the L2 traffic).
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs A) {
+__global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvArgs A) {
     using L = ConvTcLayout<CIN, COUT>;
     static_assert(CIN % 16 == 0 && COUT % 8 == 0 && L::NP <= 32, "channel padding");
     extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + L::TILES + 1);
-    const int img = blockIdx.x / (kImg / kBand);
-    const int r0 = (blockIdx.x % (kImg / kBand)) * kBand;
-    const int tid = threadIdx.x, warp = tid >> 5;
-
+    uint64_t* wbar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+    uint64_t *full = wbar + 1, *empty = full + kConvStages, *afull = empty + kConvStages, *aempty = afull + kConvAccs;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(aempty + kConvAccs);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
-        // TILES accumulators of 128 lanes x NP f32 columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(L::TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 32)
-        for (int b = 0; b <= L::TILES; ++b) bulk_mbar_init(bar + b, 1);
-    // the zero positions between the rows, and the halo rows outside the image
-    for (int i = tid; i < (L::HR + 1) * L::CH; i += kConvThreads)
-        *reinterpret_cast<uint4*>(smem + (i % L::CH) * L::PLANE + (i / L::CH) * L::PITCH * 16) = make_uint4(0, 0, 0, 0);
-    const int hlo = r0 == 0 ? 1 : 0, hhi = r0 + kBand == kImg ? L::HR - 1 : L::HR;  // halo rows in the image
-    for (int i = tid; i < kImg * L::CH; i += kConvThreads) {
-        uint4* row = reinterpret_cast<uint4*>(smem + (i % L::CH) * L::PLANE) + 1 + i / L::CH;
-        if (hlo == 1) row[0] = make_uint4(0, 0, 0, 0);
-        if (hhi == L::HR - 1) row[(L::HR - 1) * L::PITCH] = make_uint4(0, 0, 0, 0);
+    if (tid == 32) {
+        bulk_mbar_init(wbar, 1);
+        for (int i = 0; i < kConvStages; ++i) {
+            bulk_mbar_init(full + i, 1);
+            bulk_mbar_init(empty + i, 1);
+        }
+        for (int i = 0; i < kConvAccs; ++i) {
+            bulk_mbar_init(afull + i, 1);
+            bulk_mbar_init(aempty + i, 4);
+        }
     }
-    // the zeros written through the generic proxy become visible to the tensor core's proxy
+    // the zero positions between the rows, which no copy touches
+    for (int i = tid; i < kConvStages * L::CH * (L::HR + 1); i += kConvThreads)
+        *reinterpret_cast<uint4*>(smem + L::X_OFF + (i / (L::HR + 1)) * L::PLANE + (i % (L::HR + 1)) * L::PITCH * 16) =
+            make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    if (tid == 32) {
-        bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * kImg * 16 + 9 * L::B_TAP));
-        bulk_g2s(smem + L::B_OFF, A.w, 9 * L::B_TAP, bar);
-    }
-    dependency_wait();
-    if (warp == 1) {
-        __syncwarp();
-        for (int i = tid & 31; i < (hhi - hlo) * L::CH; i += 32) {
-            const int kc = i % L::CH, hr = hlo + i / L::CH;
-            bulk_g2s(smem + kc * L::PLANE + (1 + hr * L::PITCH) * 16,
-                     A.x + (((int64_t)img * L::CH + kc) * kPix + (r0 + hr - 1) * kImg) * 8, kImg * 16, bar);
+    constexpr int kBands = kImg / kBand;  // bands of an image
+    bool ok = true;
+    if (warp == 0) {
+        if (lane == 0) {
+            bulk_expect(wbar, 9 * L::B_TAP);
+            bulk_g2s(smem, A.w, 9 * L::B_TAP, wbar);
         }
-    }
-    if (tid == 0) {
-        if (bulk_wait(bar, 0, kMmaWaitLimit)) {
-            constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP, false);
-            const uint32_t base = smem_u32(smem);
-#pragma unroll 1
-            for (int h = 0; h < L::TILES; ++h) {
-#pragma unroll 1
-                for (int t = 0; t < 9; ++t) {
-                    const uint32_t a = base + (h * 128 + (t / 3) * L::PITCH + t % 3) * 16;
-                    const uint32_t b = base + L::B_OFF + t * L::B_TAP;
-#pragma unroll
-                    for (int j = 0; j < CIN / 16; ++j)
-                        umma_bf16(tmem + h * L::NP, umma_desc(a + 2 * j * L::PLANE, L::PLANE, 128),
-                                  umma_desc(b + 2 * j * L::NP * 16, L::NP * 16, 128), idesc, t > 0 || j > 0);
-                }
-                umma_commit(bar + 1 + h);
+        dependency_wait();
+        int i = 0;
+        for (int band = blockIdx.x; band < A.bands && ok; band += gridDim.x, ++i) {
+            const int st = i % kConvStages, img = band / kBands, r0 = band % kBands * kBand;
+            if (i >= kConvStages) ok = bulk_wait(empty + st, (i / kConvStages - 1) & 1, kMmaWaitLimit);
+            const int hlo = r0 == 0 ? 1 : 0, rows = (r0 + kBand == kImg ? L::HR - 1 : L::HR) - hlo;
+            if (lane == 0 && ok) bulk_expect(full + st, (uint32_t)(L::CH * rows * kImg * 16));
+            __syncwarp();
+            for (int k = lane; k < rows * L::CH && ok; k += 32) {
+                const int kc = k % L::CH, hr = hlo + k / L::CH;
+                bulk_g2s(smem + L::X_OFF + st * L::STAGE + kc * L::PLANE + (1 + hr * L::PITCH) * 16,
+                         A.x + (((int64_t)img * L::CH + kc) * kPix + (r0 + hr - 1) * kImg) * 8, kImg * 16, full + st);
             }
         }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int h = warp >> 2; h < L::TILES; h += 2) {
-        const bool done = bulk_wait(bar + 1 + h, 0, kMmaWaitLimit);
-        tc_fence_after();
-        if (!done) {
-            if ((tid & 31) == 0) atomicOr(A.status, kStatusMmaTimeout);
-            break;
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP, false);
+        const uint32_t wbase = smem_u32(smem);
+        dependency_wait();
+        ok = bulk_wait(wbar, 0, kMmaWaitLimit);
+        int i = 0, j = 0;  // bands and accumulator tiles so far
+        for (int band = blockIdx.x; band < A.bands && ok; band += gridDim.x, ++i) {
+            const int st = i % kConvStages, r0 = band % kBands * kBand;
+            unsigned char* stage = smem + L::X_OFF + st * L::STAGE;
+            ok = bulk_wait(full + st, (i / kConvStages) & 1, kMmaWaitLimit);
+            if (!ok) break;
+            if (r0 == 0 || r0 + kBand == kImg) {
+                const int r = r0 == 0 ? 0 : L::HR - 1;
+                for (int k = lane; k < L::CH * kImg; k += 32)
+                    reinterpret_cast<uint4*>(stage + (k / kImg) * L::PLANE)[1 + r * L::PITCH + k % kImg] =
+                        make_uint4(0u, 0u, 0u, 0u);
+                // what the lanes wrote becomes visible to the tensor core's proxy
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
+            __syncwarp();
+            const uint32_t base = smem_u32(stage);
+            for (int h = 0; h < L::TILES && ok; ++h, ++j) {
+                const int acc = j % kConvAccs;
+                if (j >= kConvAccs) ok = bulk_wait(aempty + acc, (j / kConvAccs - 1) & 1, kMmaWaitLimit);
+                tc_fence_after();
+                if (lane == 0 && ok) {
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+                        const uint32_t a = base + (h * 128 + (t / 3) * L::PITCH + t % 3) * 16;
+                        const uint32_t b = wbase + t * L::B_TAP;
+#pragma unroll
+                        for (int kk = 0; kk < CIN / 16; ++kk)
+                            umma_bf16(tmem + acc * L::NP, umma_desc(a + 2 * kk * L::PLANE, L::PLANE, 128),
+                                      umma_desc(b + 2 * kk * L::NP * 16, L::NP * 16, 128), idesc, t > 0 || kk > 0);
+                    }
+                    if (h == L::TILES - 1) umma_commit(empty + st);
+                    umma_commit(afull + acc);
+                }
+                __syncwarp();
+            }
         }
-        float v[32];
-        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + h * L::NP;
-        if constexpr (L::NP == 32) tmem_ld32(taddr, v);
-        else tmem_ld16(taddr, v);
-        const int f = h * 128 + (tid & 127);  // this thread's position
-        const int r = f / L::PITCH, c = f % L::PITCH;
-        if (c < kImg && r < kBand) {
-            const int pix = (r0 + r) * kImg + c;
+    } else {
+        dependency_wait();
+        for (int t = (warp - 2) >> 2;; t += kConvGroups) {  // tile t of the CTA: tile t % TILES of its band t / TILES
+            const int band = blockIdx.x + t / L::TILES * gridDim.x, h = t % L::TILES;
+            if (band >= A.bands) break;
+            const int acc = t % kConvAccs, img = band / kBands;
+            const int f = h * 128 + (warp & 3) * 32 + lane, r = f / L::PITCH, c = f % L::PITCH;  // position
+            const bool real = c < kImg && r < kBand;
+            const int pix = real ? ((band % kBands) * kBand + r) * kImg + c : 0;
+            float4 zp[EPI == EPI_DGELU ? COUT / 4 : 1];
+            if constexpr (EPI == EPI_DGELU) {
+                const float4* src = reinterpret_cast<const float4*>(A.zprev) + (int64_t)img * (COUT / 4) * kPix + pix;
+#pragma unroll
+                for (int q = 0; q < COUT / 4; ++q) zp[q] = real ? __ldg(src + q * kPix) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            __syncwarp();
+            ok = bulk_wait(afull + acc, (t / kConvAccs) & 1, kMmaWaitLimit);
+            if (!ok) break;
+            tc_fence_after();
+            float v[32];
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + acc * L::NP;
+            if constexpr (L::NP == 32) tmem_ld32(taddr, v);
+            else tmem_ld16(taddr, v);
+            // the accumulator is free once its 4 warps have read it
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(aempty + acc);
+            if (!real) continue;
             if constexpr (EPI == EPI_GELU) {
                 float4* z = A.zout ? reinterpret_cast<float4*>(A.zout) + (int64_t)img * (COUT / 4) * kPix + pix : nullptr;
                 uint4* y = reinterpret_cast<uint4*>(A.yout) + (int64_t)img * (COUT / 8) * kPix + pix;
@@ -302,7 +356,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
                 for (int q = 0; q < COUT / 8; ++q) {
                     float zz[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) zz[i] = v[8 * q + i] + __ldg(A.bias + 8 * q + i);
+                    for (int k = 0; k < 8; ++k) zz[k] = v[8 * q + k] + __ldg(A.bias + 8 * q + k);
                     if (z) {
                         z[(2 * q) * kPix] = make_float4(zz[0], zz[1], zz[2], zz[3]);
                         z[(2 * q + 1) * kPix] = make_float4(zz[4], zz[5], zz[6], zz[7]);
@@ -313,7 +367,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
             } else if constexpr (EPI == EPI_LINEAR || EPI == EPI_APPLY) {
                 static_assert(EPI == EPI_GELU || EPI == EPI_DGELU || COUT == 8, "output layer");
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] += __ldg(A.bias + i);
+                for (int k = 0; k < 8; ++k) v[k] += __ldg(A.bias + k);
                 float4* y = reinterpret_cast<float4*>(A.zout) + ((int64_t)img * kPix + pix) * 2;
                 y[0] = make_float4(v[0], v[1], v[2], v[3]);
                 y[1] = make_float4(v[4], v[5], v[6], v[7]);
@@ -329,11 +383,10 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
                     }
                 }
             } else {
-                const float4* zp = reinterpret_cast<const float4*>(A.zprev) + (int64_t)img * (COUT / 4) * kPix + pix;
                 uint4* y = reinterpret_cast<uint4*>(A.yout) + (int64_t)img * (COUT / 8) * kPix + pix;
 #pragma unroll
                 for (int q = 0; q < COUT / 8; ++q) {
-                    const float4 z0 = __ldg(zp + (2 * q) * kPix), z1 = __ldg(zp + (2 * q + 1) * kPix);
+                    const float4 z0 = zp[2 * q], z1 = zp[2 * q + 1];
                     const float* g = v + 8 * q;
                     y[q * kPix] =
                         make_uint4(pack_bf16(g[0] * gelu_grad(z0.x), g[1] * gelu_grad(z0.y)),
@@ -344,6 +397,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
             }
         }
     }
+    if (!ok && lane == 0) atomicOr(A.status, kStatusMmaTimeout);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
