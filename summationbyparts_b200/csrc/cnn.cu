@@ -212,22 +212,6 @@ struct sbp_cnn {
 
 namespace {
 
-// Launch that may begin while the stream's previous kernel drains (dependency_wait in the kernels).
-template <class... P, class... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
 template <int CIN, int COUT, int EPI>
 cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     constexpr int bytes = ConvTcLayout<CIN, COUT>::BYTES;

@@ -21,6 +21,7 @@
 #include <cstdint>
 
 #include "bulk_copy.cuh"
+#include "dependent_launch.cuh"
 
 namespace sbp {
 namespace cnn {
@@ -108,15 +109,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }
 
-// Programmatic dependent launch (the kernels are launched with it, see launch_after in cnn.cu): a
-// kernel may start while its predecessor in the stream drains.  dependency_wait returns once every
-// earlier kernel has completed and its writes are visible; only then does a kernel let its own
-// successor start, so what a successor does before its wait (barriers, TMEM, zero padding, the
-// weights, which the optimiser's kernel two or more launches before wrote) sees finished work.
-__device__ __forceinline__ void dependency_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// The kernels are dependent launches (launch_after).  Before its dependency_wait a kernel sets up
+// barriers, TMEM and zero padding and reads the weights, which the optimiser's kernel two or more
+// launches before wrote.
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

@@ -51,6 +51,7 @@
 
 #include <type_traits>
 
+#include "dependent_launch.cuh"
 #include "euler_device.cuh"
 #include "eval_program.cuh"
 #include "interp.cuh"
@@ -648,12 +649,6 @@ __device__ __forceinline__ void closure_part(int part, const LD& ld, T* o) {
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
-}
-// Programmatic dependent launch: returns once every earlier kernel of the chain has completed and
-// its writes are visible; only then may the kernel's own successor start.
-__device__ __forceinline__ void dependency_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

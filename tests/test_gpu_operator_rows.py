@@ -48,3 +48,46 @@ def test_alignments(orc, op, dtype):
                 for b in range(nb):
                     want[oo + b * stride:oo + b * stride + ny * nx] = ref[b].ravel()
                 assert out.tobytes() == want.tobytes(), (name, ny, nx, oi, oo)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_applications_in_a_row(orc, graph):
+    """Each application reads what the one before it, on the same stream, wrote: after a copy, after an
+    event of another stream, and recorded in a graph.  Bit-identical to the oracle's chain."""
+    from summationbyparts_b200.operators import Upwind4
+    op = Upwind4()
+    for shape in ((64, 64), (601, 255), (2048, 2048)):
+        a = np.random.default_rng(shape[1]).uniform(-1, 1, shape)
+        x = [torch.zeros(shape, dtype=torch.float64, device="cuda") for _ in range(5)]
+        src = torch.from_numpy(a).cuda()
+        side, main = torch.cuda.Stream(), torch.cuda.Stream()
+
+        def chain():
+            x[0].copy_(src)
+            op.diffxi(x[0], x[1])
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                op.diffeta(x[1], x[2])
+            torch.cuda.current_stream().wait_stream(side)
+            op.dissxi(x[2], x[3])
+            op.disseta(x[3], x[4])
+
+        torch.cuda.synchronize()
+        with torch.cuda.stream(main):
+            chain()
+        torch.cuda.synchronize()
+        if graph:
+            for t in x:
+                t.zero_()
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=main):
+                chain()
+            for _ in range(3):
+                g.replay()
+            torch.cuda.synchronize()
+        ref = a
+        for t, direction, kind in zip(x[1:], (orc.XI, orc.ETA, orc.XI, orc.ETA),
+                                      (orc.DIFF, orc.DIFF, orc.DISS, orc.DISS)):
+            ref = orc.op_apply(0, direction, kind, ref)
+            assert t.cpu().numpy().tobytes() == ref.tobytes()
