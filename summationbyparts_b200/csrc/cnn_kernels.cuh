@@ -412,9 +412,10 @@ struct WgradTcLayout {
     static constexpr int HR = kWgradRows + 2;                // x rows with the halo
     static constexpr int PLANE = HR * kImg * 16;
     static constexpr int ONES = 3 * CH;                      // the ones plane
-    static constexpr int B_OFF = (ONES + 1) * PLANE;         // dz: [chunk][kWgradRows * 64][8]
-    static constexpr int BPLANE = kWgradRows * kImg * 16;
-    static constexpr int END = B_OFF + (M / 8) * BPLANE;
+    static constexpr int B_OFF = (ONES + 1) * PLANE;         // dz: [row][chunk][64][8]
+    static constexpr int BLINE = kImg * 16;                  // a chunk of one dz row
+    static constexpr int BROW = (M / 8) * BLINE;
+    static constexpr int END = B_OFF + kWgradRows * BROW;
     static constexpr int BAR_OFF = END > 16 * PLANE ? END : 16 * PLANE;
     static constexpr int BYTES = BAR_OFF + 24;
     static constexpr int TMEM_COLS = 3 * M <= 64 ? 64 : 128;
@@ -423,12 +424,17 @@ struct WgradTcLayout {
 // Weight and bias gradients of one layer on the tcgen05 tensor cores, as partial sums per CTA
 // (kWgradRows image rows each) that wgrad_reduce_kernel adds up in a fixed order:
 // dw[m][t][k] = sum over pixels p of dz[p][m] * x[p + off(t)][k], db[m] = sum over p of dz[p][m].
-// For each row offset dy the GEMM D[(dx, k)][m] = sum over p of A[(dx, k)][p] * B[m][p] has the
-// 3 CIN (column offset, channel) pairs as its rows (M = 128 with the ones row and dropped rows), the
-// dz channels as N and the pixels as K; both operands are MN-major, as the chunk-major rows lie in
-// memory, so the bulk copies put them in place (one a plane) and one thread issues all 3 x kWgradRows x 4 MMAs
-// (K = 16) into three accumulators.  A row offset is a start offset of A; the column offsets are
-// three copies of the rows (an MMA's row groups lie one stride apart).
+// For each x row the GEMM D[(dx, k)][(dy, m)] = sum over pixels p of A[(dx, k)][p] * B[(dy, m)][p]
+// has the 3 CIN (column offset, channel) pairs as its rows (M = 128 with the ones row and dropped
+// rows), the up to three dz rows that meet this x row, by dy, and their channels as N and the pixels as K;
+// both operands are MN-major, as the chunk-major rows lie in memory, so the bulk copies put them in
+// place and one thread issues all MMAs (K = 16) into one accumulator of 3 M columns.  The column offsets are
+// three copies of the x rows (an MMA's row groups lie one stride apart); dz lies row by row, chunk by
+// chunk, so that the chunks of adjacent rows are one stride apart too.
+//   An MN-major MMA takes about 137 cycles here whatever its N up to 96: the fetch of its 128 A rows.  So
+// the three row offsets share one A row: 26 MMAs a CTA, 48 with a product per offset (N = M); a training
+// step of 64 images 365 -> 355 us.  What is left is the CTA's own chain: one x copy instead of three takes
+// 2 us of a layer's 22, all MMAs left out 6.
 // M = channels of dz as stored (16 or 32), MSTORE = rows of the layer's weight tensor (<= M).
 template <int CIN, int M, int MSTORE>
 __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bfloat16* __restrict__ x,
@@ -466,13 +472,15 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
     dependency_wait();
     // The copies: dz a chunk at a time, and the rows of x a chunk at a time for each dx, shifted by
     // one position to the right (dx = 0, without the last pixel) or left (dx = 2, without the first)
-    if (tid == 32) bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * 3 * kImg * 16 - 2 * L::CH * 16 + (M / 8) * L::BPLANE));
+    if (tid == 32) bulk_expect(bar, (uint32_t)((hhi - hlo) * L::CH * 3 * kImg * 16 - 2 * L::CH * 16 + kWgradRows * L::BROW));
     if (warp == 1) {
         const int lane = tid & 31;
         __syncwarp();
-        for (int i = lane; i < M / 8; i += 32)
-            bulk_g2s(smem + L::B_OFF + i * L::BPLANE, dz + (((int64_t)img * (M / 8) + i) * kPix + rbase * kImg) * 8,
-                     L::BPLANE, bar);
+        for (int i = lane; i < kWgradRows * (M / 8); i += 32) {
+            const int lr = i / (M / 8), kc = i % (M / 8);
+            bulk_g2s(smem + L::B_OFF + i * L::BLINE, dz + (((int64_t)img * (M / 8) + kc) * kPix + (rbase + lr) * kImg) * 8,
+                     L::BLINE, bar);
+        }
         for (int i = lane; i < 3 * L::CH; i += 32) {
             const int dx = i / L::CH, kc = i % L::CH;
             const __nv_bfloat16* src = x + (((int64_t)img * L::CH + kc) * kPix + (rbase + hlo - 1) * kImg + (dx == 2)) * 8;
@@ -497,19 +505,25 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0 && loaded) {
-        constexpr uint32_t idesc = umma_idesc_bf16(128, M, true);
         const uint32_t base = smem_u32(smem);
-#pragma unroll 1
-        for (int dy = 0; dy < 3; ++dy)
-#pragma unroll 1
-            for (int lr = 0; lr < kWgradRows; ++lr)
+        // x row hr with the dz rows r, r + 1, .. (n of them) and pixels 16 s ..: row r is dy = hr - r
+        auto product = [&](int hr, int s, int r, int n, uint32_t accumulate) {
+            umma_bf16(tmem + (2 - hr + r) * M, umma_desc(base + (hr * kImg + 16 * s) * 16, 128, L::PLANE),
+                      umma_desc(base + L::B_OFF + r * L::BROW + 16 * s * 16, 128, L::BLINE),
+                      umma_idesc_bf16(128, n * M, true), accumulate);
+        };
 #pragma unroll
-                for (int s = 0; s < kImg / 16; ++s) {
-                    const uint32_t a = base + ((lr + dy) * kImg + 16 * s) * 16;
-                    const uint32_t b = base + L::B_OFF + (lr * kImg + 16 * s) * 16;
-                    umma_bf16(tmem + dy * M, umma_desc(a, 128, L::PLANE), umma_desc(b, 128, L::BPLANE), idesc,
-                              (lr > 0 || s > 0) ? 1u : 0u);
+        for (int hr = 0; hr < L::HR; ++hr)
+#pragma unroll
+            for (int s = 0; s < kImg / 16; ++s) {
+                const int lo = hr < 2 ? 0 : hr - 2, hi = hr < kWgradRows ? hr : kWgradRows - 1;
+                if (s == 0 && hr < 3) {  // dz row 0 starts the sums of dy = hr
+                    product(hr, s, 0, 1, 0u);
+                    if (hr > 0) product(hr, s, 1, hr, 1u);
+                } else {
+                    product(hr, s, lo, hi - lo + 1, 1u);
                 }
+            }
         umma_commit(bar + 1);
     }
     __syncwarp();
@@ -519,7 +533,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
         float* pw = part_w + (int64_t)blockIdx.x * (MSTORE * 9 * CIN);
 #pragma unroll 1
         for (int dy = 0; dy < 3; ++dy) {
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + dy * M;
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (2 - dy) * M;
             float v[32];
             if constexpr (M == 32) tmem_ld32(taddr, v);
             else tmem_ld16(taddr, v);

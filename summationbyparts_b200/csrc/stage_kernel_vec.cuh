@@ -2,13 +2,13 @@
 // the stencil phase.
 //
 // Same right-hand side, same RK4 stage update and same edge-k hand-off as stage_kernel
-// (stage_kernel.cuh), with every output's sums taken in the same order, so the two kernels give
-// the same numbers.  What changes is the work decomposition of a 32 row x 32 column tile:
+// (stage_kernel.cuh); the two agree to f32 rounding.  What differs is the work decomposition of a
+// 32 row x 32 column tile:
 //
-// * Phase 1 (pointwise fluxes and dissipation coefficients) is stage_kernel's, except where the
-//   values go in shared memory: the xi arrays are stored transposed ([column][row], row pitch
-//   kVecPitch = 34) with the even local columns first and the odd ones after them, the eta
-//   arrays row by row (pitch 32).
+// * Phase 1 evaluates the pointwise fluxes and dissipation coefficients of both directions at once,
+//   from global loads that a thread issues for all its points before it evaluates any.  The xi
+//   arrays are stored transposed ([column][row], row pitch kVecPitch = 34) with the even local
+//   columns first and the odd ones after them, the eta arrays row by row (pitch 32).
 // * Phase 2: thread (g, p) produces the 2 x 2 outputs of columns x0 + 2g, x0 + 2g + 1 and rows
 //   y0 + 2p, y0 + 2p + 1.  An xi tap is one 8-byte shared load carrying the two rows of one
 //   column (transposed layout); an eta tap one 8-byte load carrying the two columns of one row.
@@ -23,12 +23,19 @@
 //   first and last tile of a column all its closure rows; tile_starts in system.cu), and such a
 //   tile first computes the closure outputs' xi (eta) terms with all its threads into a small
 //   shared buffer (closure_xi, closure_eta: the N inputs of the closure block loaded once,
-//   compile-time closure coefficients, first product then an fma chain as the table path of
-//   stage_kernel); every thread then runs the interior path, and the owners of closure outputs
+//   compile-time closure coefficients, first product then an fma chain); every
+//   thread then runs the interior path, and the owners of closure outputs
 //   replace its result from the buffer -- no divergence, no per-thread coefficient tables.
 // * The RK operands (1 / J and the stage's state arrays) are read from global memory into
 //   registers one component ahead of their use, as 8-byte row pairs, which leaves the shared
 //   memory of two 256-thread CTAs per SM to the stencil arrays.
+//
+// What bounds it: issue and latency, about half of HBM's rate.  Stage 1 of Upwind9 on the 256 first
+// instances of the seed-1 ensemble takes 169 us; 150 without the stencil sums, 139 without
+// phase 1's loads, 158 without the stores.  stage_kernel itself on 32-row compensated tiles (raw rows
+// by asynchronous copies, one direction at a time), which is the faster form in f64, takes 223 us here:
+// half the bytes per value leave less latency to hide, and the paired FMAs are lost.  Prefetching the
+// next tile's rows into L2 or L1 during phase 2: 178 us.
 #pragma once
 
 #include "stage_kernel.cuh"
