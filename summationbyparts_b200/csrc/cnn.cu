@@ -11,6 +11,7 @@
 
 #include "cnn_kernels.cuh"
 #include "common.h"
+#include "dynamic_smem.h"
 
 using namespace sbp;
 using namespace sbp::cnn;
@@ -215,13 +216,9 @@ namespace {
 template <int CIN, int COUT, int EPI>
 cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     constexpr int bytes = ConvTcLayout<CIN, COUT>::BYTES;
-    static bool configured = false;  // per instantiation; the attribute is per function
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, EPI>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static DynamicSmem opt_in;
+    const cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&conv3x3_tc_kernel<CIN, COUT, EPI>), bytes);
+    if (e != cudaSuccess) return e;
     a.status = c->status;
     a.bands = n * (kImg / kBand);
     const int grid = a.bands < 2 * c->num_sms ? a.bands : 2 * c->num_sms;
@@ -253,15 +250,10 @@ template <int CIN, int M, int MSTORE>
 cudaError_t wgrad(const sbp_cnn* c, int n, int layer, const __nv_bfloat16* x, const __nv_bfloat16* dz) {
     const int parts = n * (kImg / kWgradRows);
     constexpr int bytes = WgradTcLayout<CIN, M>::BYTES;
-    static bool configured = false;  // per instantiation; the attribute is per function
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(wgrad_tc_kernel<CIN, M, MSTORE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    const cudaError_t e =
-        launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->status);
+    static DynamicSmem opt_in;
+    cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&wgrad_tc_kernel<CIN, M, MSTORE>), bytes);
+    if (e != cudaSuccess) return e;
+    e = launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->status);
     if (e != cudaSuccess) return e;
     const int nw = MSTORE * 9 * CIN, nb = MSTORE;
     return launch_after(wgrad_reduce_kernel, (nw + nb + 31) / 32, 32 * kReduceSplit, 0, c->st(), c->part_w, c->part_b, parts,

@@ -39,6 +39,7 @@
 
 #include "bulk_copy.cuh"
 #include "dependent_launch.cuh"
+#include "dynamic_smem.h"
 #include "op_apply.h"
 #include "sbp_ops.cuh"
 
@@ -385,12 +386,10 @@ template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
 cudaError_t launch_eta(const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride, const Extent& A,
                        cudaStream_t st) {
     constexpr size_t smem = eta_smem<OP, T, TR, TC, ALIGNED>();
-    static bool configured = false;  // per instantiation: the attribute belongs to the function
-    if (!configured && smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(op_eta_kernel<OP, KIND, T, TR, TC, ALIGNED>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if constexpr (smem > 48 * 1024) {
+        static DynamicSmem opt_in;
+        const cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&op_eta_kernel<OP, KIND, T, TR, TC, ALIGNED>), smem);
         if (e != cudaSuccess) return e;
-        configured = true;
     }
     const T idx = inv_spacing<T>(OpShape<OP>::h2, ny);
     const int simd = (int)(simd_lanes<T>() * (nx / simd_lanes<T>()));

@@ -1,0 +1,91 @@
+"""The library's host code on a runtime without a GPU (fake_cudart.cpp): which kernels a call launches,
+with which grids and shared memory, on which device, and what it returns.  CPU only; no kernel runs."""
+import concurrent.futures as cf
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+class Runtime:
+    """The library linked with the stand-in runtime, and what that runtime recorded."""
+
+    def __init__(self, path):
+        from summationbyparts_b200 import _capi
+        self.lib = ctypes.CDLL(path, mode=os.RTLD_LOCAL | os.RTLD_NOW)
+        for name, (res, args) in _capi.SIGNATURES.items():
+            f = getattr(self.lib, name)
+            f.restype, f.argtypes = res, args
+        self.lib.fake_launch_name.restype = ctypes.c_char_p
+        self.lib.fake_alloc.restype = ctypes.c_void_p
+        self.device(0)
+
+    def device(self, d):
+        assert self.lib.cudaSetDevice(d) == 0
+
+    def error(self):
+        return self.lib.sbp_last_error().decode()
+
+    def launches(self):
+        """(kernel, device, grid, threads, dynamic shared memory) of every launch since the last call."""
+        out = []
+        for i in range(self.lib.fake_launch_count()):
+            v = (ctypes.c_longlong * 6)()
+            self.lib.fake_launch_shape(i, v)
+            out.append((self.lib.fake_launch_name(i).decode(), v[0], tuple(v[1:4]), v[4], v[5]))
+        self.lib.fake_clear_launches()
+        return out
+
+    def allocations(self, host):
+        return [self.lib.fake_alloc(int(host), k) for k in range(self.lib.fake_alloc_count(int(host)))]
+
+
+@pytest.fixture(scope="module")
+def linked(tmp_path_factory):
+    from summationbyparts_b200 import build
+    with cf.ThreadPoolExecutor(os.cpu_count()) as ex:
+        objs = list(ex.map(lambda u: build._compile(*u, False), build.UNITS.items()))
+    out = str(tmp_path_factory.mktemp("rt") / "libsbp_host.so")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc())))
+    # symbols bind inside the library: another cudart in the process is not used
+    cmd = ["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I" + os.path.join(cuda, "include"),
+           os.path.join(HERE, "fake_cudart.cpp"), *objs, "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return out
+
+
+@pytest.fixture
+def rt(linked, tmp_path):
+    """A copy of the library per test: its statics are as in a new process."""
+    return Runtime(shutil.copy(linked, tmp_path / "lib.so"))
+
+
+PTR = 1 << 20  # an address that no host code reads
+
+
+@pytest.mark.parametrize("nx", [1533, 1536])  # rows off and on the 16-byte boundaries
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_operators_on_every_device(rt, nx, dtype):
+    """A column application large enough for the 48-row tiles takes more than 48 KB of shared memory, which
+    is allowed per function and device: it runs on each device of a process, whatever ran before."""
+    for d in (0, 3, 0, 1):
+        rt.device(d)
+        assert rt.lib.sbp_diffeta(2, dtype, PTR, 2 * PTR + 8, 1021, nx, 4, 1021 * nx, None) == 0, rt.error()
+        (name, dev, _, _, smem), = rt.launches()
+        assert "op_eta_kernel" in name and dev == d and smem > 48 * 1024
+
+
+def test_network_on_every_device(rt):
+    for d in (0, 2, 1):
+        net = ctypes.c_void_p()
+        assert rt.lib.sbp_cnn_create(d, 2, 0, ctypes.byref(net)) == 0, rt.error()
+        n = 2 * 4 * 64 * 64
+        states = (ctypes.c_double * n)()
+        assert rt.lib.sbp_cnn_gradients(net, 2, states, 0, 4 * 64 * 64, states, None, None) == 0, rt.error()
+        assert any(smem > 48 * 1024 for *_, smem in rt.launches())
+        assert rt.lib.sbp_cnn_destroy(net) == 0
