@@ -29,11 +29,12 @@ _DTYPES: dict = {}  # torch dtype -> C dtype code, filled on first use (torch is
 def _setup():
     import torch
 
-    _DTYPES.update({torch.float64: _capi.F64, torch.float32: _capi.F32})
     global _raw_stream
     # handle of the current stream of a device; the public call builds a Stream object each time
     _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
         lambda index: torch.cuda.current_stream(index).cuda_stream)
+    # last: a filled table tells other threads that all of this is there
+    _DTYPES.update({torch.float64: _capi.F64, torch.float32: _capi.F32})
 
 
 def _launch(fn, op_id: int, prev, fut) -> None:
