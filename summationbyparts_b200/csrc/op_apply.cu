@@ -48,9 +48,6 @@ namespace sbp {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kBulkWait = 1 << 22;  // mbarrier polls before a tile gives up
-// Tiles whose staged rows did not arrive within kBulkWait polls; their outputs are not written.
-__device__ unsigned g_bulk_timeouts = 0;
 
 template <class T>
 struct Vec;
@@ -168,6 +165,17 @@ __device__ __forceinline__ void fetch_rows(int nrows, const SRC& src, const W& w
     }
 }
 
+// A staged row again, by plain loads, for a thread that gave up waiting for the copies.  An application is
+// asynchronous and has no status to report, so a wait that runs out costs time and not the result.  Every
+// such thread fetches the whole tile (others may have seen the copies arrive, so it cannot count on
+// them); copies that still arrive write the same values.  They are waited for once more, with a limit, as
+// they end in the CTA's shared memory.  Out of line: within the kernels this cost 3% of a large odd field.
+template <class T>
+__device__ __forceinline__ void fetch_plainly(const T* __restrict__ s, T* d, int n) {
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) d[k] = s[k];
+}
+
 constexpr int kXiRows = 16;  // most rows of a row tile
 template <class T>
 constexpr int xi_cols() { return 128 * (16 / (int)sizeof(T)); }
@@ -176,13 +184,40 @@ constexpr int xi_pitch() { return xi_cols<T>() + 32; }  // covers the halo, clos
 template <class T>
 constexpr size_t xi_smem(int rows) { return (size_t)rows * xi_pitch<T>() * sizeof(T) + 16; }
 
+// Columns [lo, hi) of a row of parity `par` that the outputs of its tile at u0 read (aligned: whole vectors).
+template <int OP, class T, bool ALIGNED>
+__device__ __forceinline__ void xi_segment(int u0, int par, int nx, int& lo, int& hi) {
+    constexpr int TC = xi_cols<T>(), K = 16 / sizeof(T);
+    lo = hi = 0;
+    if constexpr (ALIGNED) {
+        region_of<OP>(u0, min(nx, u0 + TC), nx, lo, hi);
+        lo &= ~(K - 1);
+        hi = min(nx, (hi + K - 1) & ~(K - 1));
+    } else {
+        const int c0 = max(0, u0 - par), c1 = min(nx, u0 + TC - par);
+        if (c0 < c1) region_of<OP>(c0, c1, nx, lo, hi);
+    }
+}
+
+template <int OP, class T, bool ALIGNED>
+__device__ __noinline__ void xi_fetch_plainly(const T* __restrict__ src, T* buf, int nrows, int nx, int u0, uint64_t* bar) {
+#pragma unroll 1
+    for (int r = 0; r < nrows; ++r) {
+        const T* row = src + (int64_t)r * nx;
+        int lo, hi;
+        xi_segment<OP, T, ALIGNED>(u0, ALIGNED ? 0 : parity_of(row), nx, lo, hi);
+        fetch_plainly(row + lo, buf + r * xi_pitch<T>() + (ALIGNED ? 0 : parity_of(row + lo)), hi - lo);
+    }
+    bulk_wait(bar, 0, kBulkWaitPolls);
+}
+
 // Row direction (see the file comment): `tr` rows per tile, 2^lpr threads per row.  u counts elements
 // from the 16-byte boundary at or before a row's start; tile cb covers u in [cb TC, cb TC + TC).
 // vec_out: output rows have the alignment of the input rows, so vectors are stored whole.
 template <int OP, int KIND, class T, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
     op_xi_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int ncb, int tr,
-                 int lpr, bool vec_out, Extent A) {
+                 int lpr, bool vec_out, Extent A, int polls) {
     constexpr int M = OpShape<OP>::M, H = OpShape<OP>::H;
     constexpr int K = 16 / sizeof(T);
     constexpr int TC = xi_cols<T>(), P = xi_pitch<T>();
@@ -202,20 +237,12 @@ __global__ void __launch_bounds__(kThreads)
     const T* src = in + off;
     T* dst = out + off;
     auto row_parity = [&](int r) { return ALIGNED ? 0 : parity_of(src + (int64_t)r * nx); };
-    // columns [lo, hi) of row r that the tile's outputs read (aligned: whole vectors of them)
-    int lo_a = 0, hi_a = 0;
-    if constexpr (ALIGNED) {
-        region_of<OP>(u0, min(nx, u0 + TC), nx, lo_a, hi_a);
-        lo_a &= ~(K - 1);
-        hi_a = min(nx, (hi_a + K - 1) & ~(K - 1));
-    }
+    int lo_a = 0, hi_a = 0;  // aligned: the segment of every row
+    if constexpr (ALIGNED) xi_segment<OP, T, true>(u0, 0, nx, lo_a, hi_a);
     auto seg = [&](int r, int& lo, int& hi) {
         lo = lo_a;
         hi = hi_a;
-        if constexpr (!ALIGNED) {
-            const int par = row_parity(r), c0 = max(0, u0 - par), c1 = min(nx, u0 + TC - par);
-            if (c0 < c1) region_of<OP>(c0, c1, nx, lo, hi);
-        }
+        if constexpr (!ALIGNED) xi_segment<OP, T, false>(u0, row_parity(r), nx, lo, hi);
     };
     if (threadIdx.x == 0) bulk_mbar_init(bar, 1);
     __syncthreads();
@@ -241,10 +268,7 @@ __global__ void __launch_bounds__(kThreads)
                 [&](int r) { return buf + r * P; }, A, bar);
         }
     }
-    if (!bulk_wait(bar, 0, kBulkWait)) {
-        if (threadIdx.x == 0) atomicAdd(&g_bulk_timeouts, 1u);
-        return;
-    }
+    if (!bulk_wait(bar, 0, polls)) xi_fetch_plainly<OP, T, ALIGNED>(src, buf, nrows, nx, u0, bar);
     const int v = threadIdx.x & ((1 << lpr) - 1);
     for (int r = threadIdx.x >> lpr; r < nrows; r += kThreads >> lpr) {
         const int par = row_parity(r);
@@ -301,11 +325,21 @@ constexpr int eta_pitch() { return TC + (ALIGNED ? 0 : 2 * (16 / (int)sizeof(T))
 template <int OP, class T, int TR, int TC, bool ALIGNED>
 constexpr size_t eta_smem() { return (size_t)eta_region<OP, TR>() * eta_pitch<T, TC, ALIGNED>() * sizeof(T) + 16; }
 
+template <class T, int P, bool ALIGNED>
+__device__ __noinline__ void eta_fetch_plainly(const T* __restrict__ src, T* buf, int nrows, int nx, int tw, uint64_t* bar) {
+#pragma unroll 1
+    for (int r = 0; r < nrows; ++r) {
+        const T* row = src + (int64_t)r * nx;
+        fetch_plainly(row, buf + r * P + (ALIGNED ? 0 : parity_of(row)), tw);
+    }
+    bulk_wait(bar, 0, kBulkWaitPolls);
+}
+
 // Column direction (see the file comment).
 template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
     op_eta_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int simd,
-                  Extent A) {
+                  Extent A, int polls) {
     constexpr int M = OpShape<OP>::M, D = OpShape<OP>::D, H = OpShape<OP>::H;
     constexpr int K = 16 / sizeof(T), P = eta_pitch<T, TC, ALIGNED>();
     constexpr int GROUPS = kThreads / TC;  // row groups
@@ -338,10 +372,7 @@ __global__ void __launch_bounds__(kThreads)
                 [&](int r) { return buf + r * P; }, A, bar);
         }
     }
-    if (!bulk_wait(bar, 0, kBulkWait)) {
-        if (threadIdx.x == 0) atomicAdd(&g_bulk_timeouts, 1u);
-        return;
-    }
+    if (!bulk_wait(bar, 0, polls)) eta_fetch_plainly<T, P, ALIGNED>(src, buf, hi - lo, nx, tw, bar);
     const int j = threadIdx.x % TC, g = threadIdx.x / TC;
     if (j >= tw) return;
     const int col = c0 + j;
@@ -384,7 +415,7 @@ constexpr int kSms = 148;
 // two rows per thread instead of 24 to 48.
 template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
 cudaError_t launch_eta(const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride, const Extent& A,
-                       cudaStream_t st) {
+                       cudaStream_t st, int polls) {
     constexpr size_t smem = eta_smem<OP, T, TR, TC, ALIGNED>();
     if constexpr (smem > 48 * 1024) {
         static DynamicSmem opt_in;
@@ -395,20 +426,20 @@ cudaError_t launch_eta(const T* in, T* out, int64_t ny, int64_t nx, int64_t nbat
     const int simd = (int)(simd_lanes<T>() * (nx / simd_lanes<T>()));
     const int64_t items = nbatch * ((ny + TR - 1) / TR) * ((nx + TC - 1) / TC);
     return launch_after(op_eta_kernel<OP, KIND, T, TR, TC, ALIGNED>, (unsigned)items, kThreads, smem, st, in, out, (int)ny,
-                        (int)nx, bstride, idx, simd, A);
+                        (int)nx, bstride, idx, simd, A, polls);
 }
 
 template <int OP, int KIND, class T, bool ALIGNED>
 cudaError_t launch_t(int dir, const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride,
-                     cudaStream_t st) {
+                     cudaStream_t st, int polls) {
     constexpr int K = 16 / sizeof(T);
     const uintptr_t a = reinterpret_cast<uintptr_t>(in);
     const Extent A{a, a + ((uintptr_t)(nbatch - 1) * bstride + (uintptr_t)ny * nx) * sizeof(T)};
     if (dir == 1) {
         constexpr int TR = 48, TC = 1024 / sizeof(T);
         if (nbatch * ((ny + TR - 1) / TR) * ((nx + TC - 1) / TC) >= kSms)
-            return launch_eta<OP, KIND, T, TR, TC, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st);
-        return launch_eta<OP, KIND, T, 16, 32, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st);
+            return launch_eta<OP, KIND, T, TR, TC, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
+        return launch_eta<OP, KIND, T, 16, 32, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
     }
     constexpr int TC = xi_cols<T>();
     const int64_t ncb = (nx + (ALIGNED ? 0 : K - 1) + TC - 1) / TC;
@@ -422,19 +453,19 @@ cudaError_t launch_t(int dir, const T* in, T* out, int64_t ny, int64_t nx, int64
     const T idx = inv_spacing<T>(OpShape<OP>::h2, nx);
     const int64_t items = nbatch * ((ny + tr - 1) / tr) * ncb;
     return launch_after(op_xi_kernel<OP, KIND, T, ALIGNED>, (unsigned)items, kThreads, xi_smem<T>(tr), st, in, out, (int)ny,
-                        (int)nx, bstride, idx, (int)ncb, tr, lpr, vec_out, A);
+                        (int)nx, bstride, idx, (int)ncb, tr, lpr, vec_out, A, polls);
 }
 
 template <int OP, class T>
 cudaError_t launch_kind(int dir, int kind, const void* in, void* out, int64_t ny, int64_t nx, int64_t nbatch,
-                        int64_t bstride, cudaStream_t st) {
+                        int64_t bstride, cudaStream_t st, int polls) {
     const T* i = static_cast<const T*>(in);
     T* o = static_cast<T*>(out);
     constexpr int K = 16 / sizeof(T);
     const bool aligned = nx % K == 0 && bstride % K == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
     auto launch = [&](auto k) {
-        return aligned ? launch_t<OP, decltype(k)::value, T, true>(dir, i, o, ny, nx, nbatch, bstride, st)
-                       : launch_t<OP, decltype(k)::value, T, false>(dir, i, o, ny, nx, nbatch, bstride, st);
+        return aligned ? launch_t<OP, decltype(k)::value, T, true>(dir, i, o, ny, nx, nbatch, bstride, st, polls)
+                       : launch_t<OP, decltype(k)::value, T, false>(dir, i, o, ny, nx, nbatch, bstride, st, polls);
     };
     if (kind == DIFF) return launch(std::integral_constant<int, DIFF>{});
     if constexpr (OpShape<OP>::upwind) return launch(std::integral_constant<int, DISS>{});
@@ -443,14 +474,14 @@ cudaError_t launch_kind(int dir, int kind, const void* in, void* out, int64_t ny
 
 template <class T>
 cudaError_t launch_op(int op, int dir, int kind, const void* in, void* out, int64_t ny, int64_t nx, int64_t nbatch,
-                      int64_t bstride, cudaStream_t st) {
+                      int64_t bstride, cudaStream_t st, int polls) {
     switch (op) {
-        case UPWIND4: return launch_kind<UPWIND4, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
-        case UPWIND4H2: return launch_kind<UPWIND4H2, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
-        case UPWIND9: return launch_kind<UPWIND9, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
-        case UPWIND9H2: return launch_kind<UPWIND9H2, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
-        case SBP4: return launch_kind<SBP4, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
-        case SBP8: return launch_kind<SBP8, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st);
+        case UPWIND4: return launch_kind<UPWIND4, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+        case UPWIND4H2: return launch_kind<UPWIND4H2, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+        case UPWIND9: return launch_kind<UPWIND9, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+        case UPWIND9H2: return launch_kind<UPWIND9H2, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+        case SBP4: return launch_kind<SBP4, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+        case SBP8: return launch_kind<SBP8, T>(dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -458,9 +489,9 @@ cudaError_t launch_op(int op, int dir, int kind, const void* in, void* out, int6
 }  // namespace
 
 cudaError_t op_apply(int op, int dir, int kind, int dtype, const void* in, void* out, int64_t ny, int64_t nx,
-                     int64_t nbatch, int64_t bstride, cudaStream_t st) {
-    if (dtype == 0) return launch_op<double>(op, dir, kind, in, out, ny, nx, nbatch, bstride, st);
-    return launch_op<float>(op, dir, kind, in, out, ny, nx, nbatch, bstride, st);
+                     int64_t nbatch, int64_t bstride, cudaStream_t st, int polls) {
+    if (dtype == 0) return launch_op<double>(op, dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
+    return launch_op<float>(op, dir, kind, in, out, ny, nx, nbatch, bstride, st, polls);
 }
 
 }  // namespace sbp
