@@ -342,6 +342,9 @@ sbp_status sbp_cnn_destroy(sbp_cnn* net);
 /* Stream for all later work of the network (cudaStream_t; NULL = the legacy default stream).
  * Until it is called the network uses a stream of its own. */
 sbp_status sbp_cnn_set_stream(sbp_cnn* net, void* stream);
+/* Waits for the network's work.  The kernels' waits are bounded: one that gave up leaves outputs
+ * unwritten and the parameters unchanged until it is reported, once (SBP_ERR_CUDA), by the next of
+ * this call, sbp_cnn_get_params, and the calls that return a loss or gradients to the host. */
 sbp_status sbp_cnn_synchronize(sbp_cnn* net);
 /* Number of FP32 parameters (padded layout: per layer weights [cout][9][cin], then biases). */
 int64_t sbp_cnn_param_count(const sbp_cnn* net);

@@ -96,11 +96,13 @@ __device__ __forceinline__ void store_bf16_weight(const LayerParams& L, int e, f
 }
 
 // Adam (Kingma & Ba) on every layer (blockIdx.y), with the bias corrections c1 = 1 / (1 - beta1^t),
-// c2 = 1 / (1 - beta2^t) from the host; rewrites the bf16 weights.
+// c2 = 1 / (1 - beta2^t) from the host; rewrites the bf16 weights.  No update from gradients of a pass that
+// gave up (its status bit).
 __global__ void adam_kernel(const NetParams N, float* __restrict__ P, const float* __restrict__ G,
                             float* __restrict__ Mo, float* __restrict__ Ve, float lr, float b1, float b2, float c1,
-                            float c2, float eps) {
+                            float c2, float eps, const unsigned* __restrict__ status) {
     dependency_wait();
+    if (*status & kStatusMmaTimeout) return;
     const LayerParams& L = N.l[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.nw + L.cout) return;
@@ -204,7 +206,8 @@ struct sbp_cnn {
     float* y = nullptr;               // output [B][kPix][8]
     __nv_bfloat16* dz[kLayers] = {};  // output gradients
     float *part_w = nullptr, *part_b = nullptr, *part_loss = nullptr;
-    unsigned* status = nullptr;       // device status word of the tensor-core kernels
+    StatusWord status{};              // of the tensor-core kernels
+    int polls = kMmaWaitLimit;        // of every wait of the tensor-core kernels
     float4 in_mean{0, 0, 0, 0}, in_inv{1, 1, 1, 1}, out_scale{1, 1, 1, 1};
     int adam_t = 0;
     std::vector<void*> allocs;
@@ -220,6 +223,7 @@ cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     const cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&conv3x3_tc_kernel<CIN, COUT, EPI>), bytes);
     if (e != cudaSuccess) return e;
     a.status = c->status;
+    a.polls = c->polls;
     a.bands = n * (kImg / kBand);
     const int grid = a.bands < 2 * c->num_sms ? a.bands : 2 * c->num_sms;
     return launch_after(conv3x3_tc_kernel<CIN, COUT, EPI>, grid, kConvThreads, bytes, c->st(), a);
@@ -234,12 +238,13 @@ NetParams net_params(const sbp_cnn* c) {
 }
 constexpr int kMaxLayerParams = 32 * 9 * 32 + 32;
 
-// The device status word after the stream has drained: a tensor-core wait that gave up.
+// The status word after the stream has drained: a wait that gave up, reported once.
 sbp_status device_status(sbp_cnn* c) {
-    unsigned h = 0;
-    SBP_TRY_CUDA(cudaMemcpyAsync(&h, c->status, sizeof h, cudaMemcpyDeviceToHost, c->st()));
     SBP_TRY_CUDA(cudaStreamSynchronize(c->st()));
-    if (h & kStatusMmaTimeout) {
+    volatile unsigned* word = c->status.host;
+    if (*word & kStatusMmaTimeout) {
+        *word = 0;
+        SBP_TRY_CUDA(cudaMemsetAsync(c->status.dev, 0, sizeof(unsigned), c->st()));
         set_error("a convolution's tensor-core work did not complete in time");
         return SBP_ERR_CUDA;
     }
@@ -253,7 +258,8 @@ cudaError_t wgrad(const sbp_cnn* c, int n, int layer, const __nv_bfloat16* x, co
     static DynamicSmem opt_in;
     cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&wgrad_tc_kernel<CIN, M, MSTORE>), bytes);
     if (e != cudaSuccess) return e;
-    e = launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->status);
+    e = launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->polls,
+                     c->status);
     if (e != cudaSuccess) return e;
     const int nw = MSTORE * 9 * CIN, nb = MSTORE;
     return launch_after(wgrad_reduce_kernel, (nw + nb + 31) / 32, 32 * kReduceSplit, 0, c->st(), c->part_w, c->part_b, parts,
@@ -352,6 +358,11 @@ sbp_status refresh_bf16(sbp_cnn* c) {
 
 }  // namespace
 
+namespace sbp {
+// Polls of every later wait of the network's kernels.
+void cnn_wait_limit(sbp_cnn* c, int polls) { c->polls = polls; }
+}  // namespace sbp
+
 extern "C" {
 
 sbp_status sbp_cnn_create(int device, int max_batch, unsigned long long seed, sbp_cnn** out) {
@@ -369,6 +380,7 @@ sbp_status sbp_cnn_create(int device, int max_batch, unsigned long long seed, sb
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) c->num_sms = sms;
     auto fail = [&](sbp_status s) {
         for (void* p : c->allocs) cudaFree(p);
+        if (c->status.host) cudaFreeHost(c->status.host);
         if (c->own) cudaStreamDestroy(c->own);
         delete c;
         return s;
@@ -406,7 +418,9 @@ sbp_status sbp_cnn_create(int device, int max_batch, unsigned long long seed, sb
     e = e ?: alloc((void**)&c->part_w, B * (kImg / kWgradRows) * (32 * 9 * 32) * 4);
     e = e ?: alloc((void**)&c->part_b, B * (kImg / kWgradRows) * 32 * 4);
     e = e ?: alloc((void**)&c->part_loss, (B * kPix + 255) / 256 * 4);
-    e = e ?: alloc((void**)&c->status, sizeof(unsigned));
+    e = e ?: alloc((void**)&c->status.dev, sizeof(unsigned));
+    e = e ?: cudaHostAlloc((void**)&c->status.host, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) *c->status.host = 0;
     if (e != cudaSuccess) return fail(cuda_status(e, "network allocation"));
     // He-style initialisation for the GELU layers, a small output layer so the initial
     // correction is close to zero; padded entries stay zero.
@@ -439,6 +453,7 @@ sbp_status sbp_cnn_destroy(sbp_cnn* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->st());
     for (void* p : c->allocs) cudaFree(p);
+    cudaFreeHost(c->status.host);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
     return SBP_OK;
@@ -475,8 +490,7 @@ sbp_status sbp_cnn_get_params(sbp_cnn* c, float* host) {
     if (!c || !host) return SBP_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
     SBP_TRY_CUDA(cudaMemcpyAsync(host, c->P, c->nparams * 4, cudaMemcpyDeviceToHost, c->st()));
-    SBP_TRY_CUDA(cudaStreamSynchronize(c->st()));
-    return SBP_OK;
+    return device_status(c);
 }
 
 sbp_status sbp_cnn_set_params(sbp_cnn* c, const float* host) {
@@ -534,7 +548,7 @@ sbp_status sbp_cnn_train_step(sbp_cnn* c, int n, const void* d_coarse, int dtype
     const float c1 = float(1.0 / (1.0 - std::pow(double(b1), c->adam_t)));
     const float c2 = float(1.0 / (1.0 - std::pow(double(b2), c->adam_t)));
     SBP_TRY_CUDA(launch_after(adam_kernel, dim3((kMaxLayerParams + 255) / 256, kLayers), 256, 0, c->st(), net_params(c), c->P,
-                              c->G, c->Mo, c->Ve, lr, b1, b2, c1, c2, eps));
+                              c->G, c->Mo, c->Ve, lr, b1, b2, c1, c2, eps, c->status.dev));
     return SBP_OK;
 }
 
@@ -550,7 +564,6 @@ sbp_status sbp_cnn_apply(sbp_cnn* c, int n, const void* d_coarse, int dtype, int
 sbp_status sbp_cnn_synchronize(sbp_cnn* c) {
     clear_error();
     if (!c) return SBP_ERR_INVALID_ARGUMENT;
-    SBP_TRY_CUDA(cudaStreamSynchronize(c->st()));
     return device_status(c);
 }
 

@@ -145,10 +145,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Bit of the network's device status word set when a convolution gave up waiting for its
-// tensor-core work (the wait is bounded, so a fault cannot hang the stream).
+// Bit of the network's status word set when a kernel gave up waiting for its copies or its tensor-core
+// work (the waits are bounded, so a fault cannot hang the stream).  Such a kernel leaves outputs
+// unwritten: the optimiser changes nothing while the bit is set, and the host reports it at its next
+// synchronisation.  Before it returns it waits once more for what it has in flight, which ends
+// in the CTA's shared memory and TMEM.
 constexpr unsigned kStatusMmaTimeout = 1u;
+struct StatusWord {
+    unsigned* dev;
+    unsigned* host;  // the same in mapped host memory: the host reads it without a copy
+    __device__ void gave_up() const {
+        atomicOr(dev, kStatusMmaTimeout);
+        atomicOr_system(host, kStatusMmaTimeout);
+    }
+};
 constexpr int kMmaWaitLimit = 1 << 22;  // mbarrier polls before giving up
+
+// bulk_wait for a whole warp: the lanes agree, so that they stay together for what is warp-wide.
+__device__ __forceinline__ bool warp_wait(uint64_t* mbar, uint32_t parity, int limit) {
+    return __all_sync(0xffffffffu, bulk_wait(mbar, parity, limit));
+}
 
 // Shared-memory layout of the tcgen05 convolution (dynamic): the weights, then kConvStages band stages.
 // A band of kBand rows with one halo row on each side is one sequence of positions per channel chunk:
@@ -196,7 +212,8 @@ struct ConvArgs {
     float4 oscale;
     double* out;
     int bands;                 // bands of all images
-    unsigned* status;
+    int polls;                 // of every wait
+    StatusWord status;
 };
 
 // 3x3 convolution with zero padding as an implicit GEMM on the tcgen05 tensor cores:
@@ -263,28 +280,33 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
         }
         dependency_wait();
         int i = 0;
-        for (int band = blockIdx.x; band < A.bands && ok; band += gridDim.x, ++i) {
+        for (int band = blockIdx.x; band < A.bands; band += gridDim.x, ++i) {
             const int st = i % kConvStages, img = band / kBands, r0 = band % kBands * kBand;
-            if (i >= kConvStages) ok = bulk_wait(empty + st, (i / kConvStages - 1) & 1, kMmaWaitLimit);
+            if (i >= kConvStages) ok = warp_wait(empty + st, (i / kConvStages - 1) & 1, A.polls);
+            if (!ok) break;
             const int hlo = r0 == 0 ? 1 : 0, rows = (r0 + kBand == kImg ? L::HR - 1 : L::HR) - hlo;
-            if (lane == 0 && ok) bulk_expect(full + st, (uint32_t)(L::CH * rows * kImg * 16));
+            if (lane == 0) bulk_expect(full + st, (uint32_t)(L::CH * rows * kImg * 16));
             __syncwarp();
-            for (int k = lane; k < rows * L::CH && ok; k += 32) {
+            for (int k = lane; k < rows * L::CH; k += 32) {
                 const int kc = k % L::CH, hr = hlo + k / L::CH;
                 bulk_g2s(smem + L::X_OFF + st * L::STAGE + kc * L::PLANE + (1 + hr * L::PITCH) * 16,
                          A.x + (((int64_t)img * L::CH + kc) * kPix + (r0 + hr - 1) * kImg) * 8, kImg * 16, full + st);
             }
         }
+        // the copies of the weights and of the last bands have arrived, whatever the other warps did
+        ok = warp_wait(wbar, 0, kMmaWaitLimit) && ok;
+        for (int b = i < kConvStages ? 0 : i - kConvStages; b < i; ++b)
+            ok = warp_wait(full + b % kConvStages, (b / kConvStages) & 1, kMmaWaitLimit) && ok;
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP, false);
         const uint32_t wbase = smem_u32(smem);
         dependency_wait();
-        ok = bulk_wait(wbar, 0, kMmaWaitLimit);
+        ok = warp_wait(wbar, 0, A.polls);
         int i = 0, j = 0;  // bands and accumulator tiles so far
         for (int band = blockIdx.x; band < A.bands && ok; band += gridDim.x, ++i) {
             const int st = i % kConvStages, r0 = band % kBands * kBand;
             unsigned char* stage = smem + L::X_OFF + st * L::STAGE;
-            ok = bulk_wait(full + st, (i / kConvStages) & 1, kMmaWaitLimit);
+            ok = warp_wait(full + st, (i / kConvStages) & 1, A.polls);
             if (!ok) break;
             if (r0 == 0 || r0 + kBand == kImg) {
                 const int r = r0 == 0 ? 0 : L::HR - 1;
@@ -296,11 +318,12 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
             }
             __syncwarp();
             const uint32_t base = smem_u32(stage);
-            for (int h = 0; h < L::TILES && ok; ++h, ++j) {
+            for (int h = 0; h < L::TILES; ++h, ++j) {
                 const int acc = j % kConvAccs;
-                if (j >= kConvAccs) ok = bulk_wait(aempty + acc, (j / kConvAccs - 1) & 1, kMmaWaitLimit);
+                if (j >= kConvAccs) ok = warp_wait(aempty + acc, (j / kConvAccs - 1) & 1, A.polls);
+                if (!ok) break;
                 tc_fence_after();
-                if (lane == 0 && ok) {
+                if (lane == 0) {
 #pragma unroll
                     for (int t = 0; t < 9; ++t) {
                         const uint32_t a = base + (h * 128 + (t / 3) * L::PITCH + t % 3) * 16;
@@ -316,6 +339,8 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
                 __syncwarp();
             }
         }
+        // the products issued so far are done
+        if (j > 0) ok = warp_wait(afull + (j - 1) % kConvAccs, ((j - 1) / kConvAccs) & 1, kMmaWaitLimit) && ok;
     } else {
         dependency_wait();
         for (int t = (warp - 2) >> 2;; t += kConvGroups) {  // tile t of the CTA: tile t % TILES of its band t / TILES
@@ -332,7 +357,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
                 for (int q = 0; q < COUT / 4; ++q) zp[q] = real ? __ldg(src + q * kPix) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
             __syncwarp();
-            ok = bulk_wait(afull + acc, (t / kConvAccs) & 1, kMmaWaitLimit);
+            ok = warp_wait(afull + acc, (t / kConvAccs) & 1, A.polls);
             if (!ok) break;
             tc_fence_after();
             float v[32];
@@ -392,7 +417,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
             }
         }
     }
-    if (!ok && lane == 0) atomicOr(A.status, kStatusMmaTimeout);
+    if (!ok && lane == 0) A.status.gave_up();
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -440,8 +465,8 @@ template <int CIN, int M, int MSTORE>
 __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bfloat16* __restrict__ x,
                                                                 const __nv_bfloat16* __restrict__ dz,
                                                                 float* __restrict__ part_w,
-                                                                float* __restrict__ part_b,
-                                                                unsigned* __restrict__ status) {
+                                                                float* __restrict__ part_b, int polls,
+                                                                const StatusWord status) {
     using L = WgradTcLayout<CIN, M>;
     static_assert(CIN % 16 == 0 && M % 16 == 0 && MSTORE <= M && L::ONES < 16, "channel padding");
     extern __shared__ __align__(128) unsigned char smem[];
@@ -487,7 +512,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
             bulk_g2s(smem + i * L::PLANE + (hlo * kImg + (dx == 0)) * 16, src, ((hhi - hlo) * kImg - (dx != 1)) * 16, bar);
         }
     }
-    const bool loaded = bulk_wait(bar, 0, kMmaWaitLimit);
+    const bool arrived = bulk_wait(bar, 0, polls);
     // the column that a shifted copy took from the row beside it is zero padding, and so are the
     // rows outside the image
     for (int i = tid; i < L::HR * L::CH * 2; i += kWgradThreads) {
@@ -503,7 +528,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
         }
     // what the threads wrote becomes visible to the tensor core's proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
+    const bool loaded = __syncthreads_and(arrived);
     if (tid == 0 && loaded) {
         const uint32_t base = smem_u32(smem);
         // x row hr with the dz rows r, r + 1, .. (n of them) and pixels 16 s ..: row r is dy = hr - r
@@ -527,7 +552,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
         umma_commit(bar + 1);
     }
     __syncwarp();
-    const bool done = bulk_wait(bar + 1, 0, kMmaWaitLimit);
+    const bool done = loaded && warp_wait(bar + 1, 0, polls);
     tc_fence_after();
     if (done) {
         float* pw = part_w + (int64_t)blockIdx.x * (MSTORE * 9 * CIN);
@@ -546,8 +571,9 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
                 for (int m = 0; m < MSTORE; ++m) part_b[(int64_t)blockIdx.x * MSTORE + m] = v[m];
             }
         }
-    } else if ((tid & 31) == 0) {
-        atomicOr(status, kStatusMmaTimeout);
+    } else {
+        if ((tid & 31) == 0) status.gave_up();
+        bulk_wait(loaded ? bar + 1 : bar, 0, kMmaWaitLimit);
     }
     tc_fence_before();
     __syncthreads();

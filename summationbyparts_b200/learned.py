@@ -190,7 +190,7 @@ class CorrectionNet:
         y = torch.empty((n, COARSE * COARSE, 8), dtype=torch.float32, device=coarse.device)
         check(_capi.lib.sbp_cnn_forward(self.h, n, ctypes.c_void_p(coarse.data_ptr()), F64, 4 * COARSE * COARSE))
         check(_capi.lib.sbp_cnn_output(self.h, n, ctypes.c_void_p(y.data_ptr())))
-        self.stream.synchronize()
+        check(_capi.lib.sbp_cnn_synchronize(self.h))
         return y
 
     def train_step(self, coarse, fine_r, lr: float, want_loss: bool = False):
@@ -211,7 +211,7 @@ class CorrectionNet:
             b = min(a + self.max_batch, coarse.shape[0])
             check(_capi.lib.sbp_cnn_apply(self.h, b - a, ctypes.c_void_p(coarse[a].data_ptr()), F64,
                                           4 * COARSE * COARSE, ctypes.c_void_p(out[a].data_ptr())))
-        self.stream.synchronize()
+        check(_capi.lib.sbp_cnn_synchronize(self.h))
         return out
 
     def fit(self, coarse, fine_r, epochs: int, lr: float = 2e-3, seed: int = 0, batch: int | None = None):

@@ -89,3 +89,27 @@ def test_network_on_every_device(rt):
         assert rt.lib.sbp_cnn_gradients(net, 2, states, 0, 4 * 64 * 64, states, None, None) == 0, rt.error()
         assert any(smem > 48 * 1024 for *_, smem in rt.launches())
         assert rt.lib.sbp_cnn_destroy(net) == 0
+
+
+def test_network_reports_a_wait_that_gave_up(rt):
+    """The status word that a kernel sets when it gives up (a network's mapped host memory) reaches the
+    caller at the next synchronising call, whichever that is, and once."""
+    net = ctypes.c_void_p()
+    assert rt.lib.sbp_cnn_create(0, 1, 0, ctypes.byref(net)) == 0, rt.error()
+    word = ctypes.c_uint.from_address(rt.allocations(host=True)[-1])
+    params = (ctypes.c_float * rt.lib.sbp_cnn_param_count(net))()
+    states = (ctypes.c_double * (4 * 64 * 64))()
+    loss = ctypes.c_float()
+    one = (net, 1, states, 0, 4 * 64 * 64)
+    calls = {"synchronize": lambda: rt.lib.sbp_cnn_synchronize(net),
+             "get_params": lambda: rt.lib.sbp_cnn_get_params(net, params),
+             "gradients": lambda: rt.lib.sbp_cnn_gradients(*one, states, None, params),
+             "loss": lambda: rt.lib.sbp_cnn_train_step(*one, states, 1e-3, ctypes.byref(loss))}
+    for name, call in calls.items():
+        assert call() == 0, name
+        word.value = 1
+        assert rt.lib.sbp_cnn_apply(*one, states) == 0, name  # asynchronous: reports nothing yet
+        assert rt.lib.sbp_cnn_train_step(*one, states, 1e-3, None) == 0, name
+        assert call() != 0 and "in time" in rt.error(), name
+        assert call() == 0, name
+    assert rt.lib.sbp_cnn_destroy(net) == 0
