@@ -85,8 +85,8 @@ __device__ __forceinline__ T pressure(T g, T rho, T rhou, T rhov, T e) {
 // POW_FREE and gamma == 1.4 the powers are formed from square roots and products: with
 // b = 1 - K e^f, rho = b^(1/(gamma-1)) = b^2.5 = b^2 sqrt(b) and rho^gamma = b^3.5 = b^3 sqrt(b),
 // and e^(f/2) = sqrt(e^f); each is correctly rounded, so the values differ from pow and exp in
-// the last bits only.  The SAT boundary data use that form (it removes the two f64 pow and one
-// exp of every vortex edge point at every stage); initial data and the error norms use pow.
+// the last bits only.  That form serves the SAT boundary data of vortices without a radius (for the others
+// see vortex_point_fast); other gammas take pow.
 template <bool POW_FREE = false>
 __device__ inline void vortex_point(const InstanceDev& I, double gamma, double t, double x, double y, double q[4]) {
     const double PI = 3.14159265358979323846;
@@ -174,6 +174,13 @@ __device__ inline void vortex_point_fast(const InstanceDev& I, double t, double 
             q[3] += en - e_inf;
         }
     }
+}
+
+// The vortex data of the initial state and of the error norms: one function for both, so that a state is
+// without error against the data it was made from.
+__device__ __forceinline__ void vortex_data(const InstanceDev& I, double gamma, double t, double x, double y, double q[4]) {
+    if (gamma == 1.4 && I.v_regular) vortex_point_fast(I, t, x, y, q);
+    else vortex_point(I, gamma, t, x, y, q);
 }
 
 // Knuth's TwoSum: s + e == a + b exactly (round-to-nearest, no FMA involved).

@@ -65,8 +65,6 @@ __global__ void __launch_bounds__(kT) vortex_init_kernel(const BlockDev* __restr
     const int64_t n = (int64_t)B.nx * B.ny, np = B.npad, i0 = blockIdx.x * (int64_t)(kPer * kT) + threadIdx.x;
     if (i0 >= n || (instance >= 0 && B.instance != instance)) return;
     const InstanceDev& I = inst[B.instance];
-    // gamma = 1.4: the powers from square roots and products (vortex_point_fast)
-    const bool fast = gamma == 1.4 && I.v_regular;
     double x[kPer], y[kPer];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
@@ -81,8 +79,7 @@ __global__ void __launch_bounds__(kT) vortex_init_kernel(const BlockDev* __restr
         const double xk = k < 2 ? (k == 0 ? x[0] : x[1]) : (k == 2 ? x[2] : x[3]);
         const double yk = k < 2 ? (k == 0 ? y[0] : y[1]) : (k == 2 ? y[2] : y[3]);
         double q[4];
-        if (fast) vortex_point_fast(I, t, xk, yk, q);
-        else vortex_point(I, gamma, t, xk, yk, q);
+        vortex_data(I, gamma, t, xk, yk, q);
 #pragma unroll
         for (int c = 0; c < 4; ++c) store_state<PREC>(q_hi, q_lo, B.q_off + c * np + i, q[c], I.qref[c]);
     }
@@ -109,7 +106,7 @@ __global__ void error_kernel(const BlockDev* __restrict__ blocks, const Instance
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int row = (int)(i / B.nx), col = (int)(i - (int64_t)row * B.nx);
         double v[4];
-        vortex_point(I, gamma, I.time, xy[B.x_off + i], xy[B.x_off + np + i], v);
+        vortex_data(I, gamma, I.time, xy[B.x_off + i], xy[B.x_off + np + i], v);
         for (int c = 0; c < 4; ++c) {
             const double d = state_at(prec, q_hi, q_lo, B.q_off + c * np + i, I.qref[c]) - v[c];
             s += d * d * hx[col] * hy[row];
