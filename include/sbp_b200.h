@@ -261,20 +261,25 @@ sbp_status sbp_system_error(sbp_system* sys, double* per_instance);
 /* Field::h2_err (euler/src/lib.rs:377-431) of one block's state against a host field q. */
 sbp_status sbp_system_h2_err(sbp_system* sys, int block, const double* q, double* err);
 
-/* Tile schedule: output tiles of ty x tx points per CTA, `threads` threads per CTA
- * (0 = keep), for every operator group; clears the autotuner's per-group choices.  Until it is
- * called, a system too small to fill the GPU takes the fused form of the stage kernel (tiles of
- * 8 x 16 or 16 x 32 points, the SATs in the stage launches); f64 results do not depend on the form.
+/* Tile schedule: output tiles of ty x tx points per CTA, `threads` threads per CTA, for every
+ * operator group; clears the autotuner's per-group choices.  16 x 32 and 32 x 32 points with 256
+ * threads (0 = these); or the fused form of the stage kernel (the SATs in the stage launches, for
+ * systems without expression sides whose blocks pair operators of one family): 8 x 16 points with 288
+ * threads or 16 x 32 with 320.  Until it is called, a system too small to fill the GPU takes the fused
+ * form and any other 16 x 32 tiles.  f64 results do not depend on the schedule; compensated results
+ * are the same for all but 32 x 32 tiles, whose kernel agrees with the others to f32 rounding.
  * sbp_system_autotune searches, per operator group, the tile rows (16, 32) and the width of the
  * stage kernel's grid (as many persistent CTAs per SM as fit, one per SM, or one CTA per tile),
  * timing whole RK4 steps on the current state (state and time are restored) by coordinate
- * descent over the groups, and keeps the fastest; it returns the tile shape of the group with
- * the most points.  It starts from the current schedule, a small system's fused form included. */
+ * descent over the groups, and keeps the fastest; it returns the tile shape and the threads of the
+ * group with the most points, as sbp_system_set_tiles takes them.  It starts from the current schedule, a small system's fused form included. */
 sbp_status sbp_system_set_tiles(sbp_system* sys, int ty, int tx, int threads);
 sbp_status sbp_system_autotune(sbp_system* sys, int* ty, int* tx, int* threads);
 /* Schedule of one operator group: tile rows, persistent CTAs per SM (-1 = as many as fit,
  * 0 = one CTA per tile) and the resulting grid size of its stage kernel. */
 sbp_status sbp_system_group_tiles(sbp_system* sys, int group, int* ty, int* ctas_per_sm, int* grid);
+/* 1 if the group takes the fused form of the stage kernel, 0 if not, -1 on error. */
+int sbp_system_group_fused(sbp_system* sys, int group);
 
 /* Stream the system launches on (cudaStream_t as void*; NULL = a stream owned by the system). */
 sbp_status sbp_system_set_stream(sbp_system* sys, void* stream);

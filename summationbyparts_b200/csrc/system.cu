@@ -186,9 +186,10 @@ struct sbp_system {
     double* kbuf = nullptr;  // k of the stages of a general tableau (kMaxStages x nq, f64), on demand
     int kbuf_stages = 0;
     // schedule
-    int TY = 16, TX = kTileX, threads = kStageThreads;
+    int TY = 16, threads = kStageThreads;  // threads: of the stencil
     std::vector<TileChoice> tile_choice;  // per operator group; groups not listed use (TY, -1)
     bool tiles_auto = true;               // until a caller chooses: small systems take the fused form
+    bool fused = false;                   // a caller's choice: the fused form with TY rows
     int tiles_gen = 0;                    // bumped whenever the tile schedule changes
     std::vector<int> active;
     std::vector<Group> groups;
@@ -548,26 +549,40 @@ std::vector<int> tile_starts(int n, int T, int M) {
     return b;
 }
 
+// Whether the fused form with `ty` rows exists for every block: expression sides need their own kernel, and
+// pairs of operators of two families are not instantiated.
+bool fused_built(const sbp_system* s, int ty) {
+    if (s->has_eval) return false;
+    for (const BlockDev& B : s->hb) {
+        OpInfo ox, oy;
+        op_info(B.op_xi, ox);
+        op_info(B.op_eta, oy);
+        const bool upw = ox.upwind && oy.upwind && !s->force_trad;
+        if (!stage_kernel_ptr(s->prec, B.op_xi, B.op_eta, upw, ty | kTileFused, 0)) return false;
+    }
+    return true;
+}
 // The tile rows of the fused stage kernel for a system that leaves SMs without work, 0 where the other
 // forms are better.  The fused kernel evaluates the SATs beside the stencils, saves the edge and time
 // launches and overlaps successive stages, but runs one CTA an SM.  Measured per step (Upwind9 f64,
 // one vortex block; 8-row tiles, 16-row tiles, the separate form): 128^2 (128 tiles of 8 rows) 30,
 // 37, 60 us; 160^2 (200) 41, 37, 60; 350^2 (242 tiles of 16 rows) -, 64, 76; 400^2 (325) -, 88, 101;
 // 500^2 (512) -, 115, 111.  So 8 rows while their tiles fit the SMs at once, 16 rows up to three tiles
-// an SM.
+// an SM.  The line holds for the other operators and precision too; fused, separate with 16 and with 32
+// rows at 288^2 (162 tiles) and 448^2 (392): Upwind9 compensated 56, 70, 70 and 78, 89, 84; Upwind4 51,
+// 66, 68 and 74, 86, 99, compensated 49, 64, 64 and 70, 80, 73; SBP8 45, 60, 64 and 64, 78, 88,
+// compensated 43, 58, 58 and 60, 70, 65.
 // The rule goes by all blocks of the system and not by the instances or the chunk at hand, so every
-// schedule of a system takes the same form.  Expression sides need their own kernel, and pairs of
-// operators of two families are not instantiated.
+// schedule of a system takes the same form.
 int fused_rows(const sbp_system* s) {
-    if (!s->tiles_auto || s->has_eval) return 0;
+    if (!s->tiles_auto) return s->fused ? s->TY : 0;
     for (int ty : {8, 16}) {
+        if (!fused_built(s, ty)) return 0;
         int64_t tiles = 0;
         for (const BlockDev& B : s->hb) {
             OpInfo ox, oy;
             op_info(B.op_xi, ox);
             op_info(B.op_eta, oy);
-            const bool upw = ox.upwind && oy.upwind && !s->force_trad;
-            if (!stage_kernel_ptr(s->prec, B.op_xi, B.op_eta, upw, ty | kTileFused, 0)) return 0;
             tiles += (int64_t)(tile_starts(B.ny, ty, oy.M).size() - 1) * (tile_starts(B.nx, tile_tx(ty), ox.M).size() - 1);
         }
         if (tiles <= (ty == 8 ? 1 : 3) * (int64_t)s->num_sms) return ty;
@@ -1682,12 +1697,17 @@ sbp_status sbp_system_h2_err(sbp_system* sys, int block, const double* q, double
 sbp_status sbp_system_set_tiles(sbp_system* sys, int ty, int tx, int threads) {
     clear_error();
     if (!sys) return SBP_ERR_INVALID_ARGUMENT;
-    if ((ty != 16 && ty != 32) || tx != kTileX || (threads != 0 && threads != kStageThreads)) {
-        set_error("tiles are 16 or 32 rows x %d columns with %d threads", kTileX, kStageThreads);
+    const bool fused = (ty == 8 || ty == 16) && tx == tile_tx(ty) && threads == kStageThreads + sat_threads(ty);
+    if (!fused && ((ty != 16 && ty != 32) || tx != kTileX || (threads != 0 && threads != kStageThreads))) {
+        set_error("tiles are 16 or 32 rows x %d columns with %d threads, or those of the fused form", kTileX, kStageThreads);
+        return SBP_ERR_INVALID_ARGUMENT;
+    }
+    if (fused && !fused_built(sys, ty)) {
+        set_error("the fused form takes no expression sides and no operators of two families in a block");
         return SBP_ERR_INVALID_ARGUMENT;
     }
     sys->TY = ty;
-    sys->TX = tx;
+    sys->fused = fused;
     sys->threads = kStageThreads;
     sys->tile_choice.clear();
     sys->tiles_auto = false;
@@ -1800,19 +1820,24 @@ sbp_status sbp_system_autotune(sbp_system* sys, int* ty, int* tx, int* threads) 
         set_error("no tile candidate could run");
         return SBP_ERR_CUDA;
     }
-    // the tile rows of the group with the most points
-    int64_t most = -1;
-    int ty_main = sys->TY;
+    // the tiles of the group with the most points
     SBP_TRY(build_schedule(sys));
+    const Group* big = &sys->groups[0];
     for (const Group& g : sys->groups)
-        if (g.points > most) {
-            most = g.points;
-            ty_main = g.ty;
-        }
-    if (ty) *ty = ty_main;
-    if (tx) *tx = sys->TX;
-    if (threads) *threads = sys->threads;
+        if (g.points > big->points) big = &g;
+    if (ty) *ty = big->ty;
+    if (tx) *tx = tile_tx(big->ty);
+    if (threads) *threads = sys->threads + (big->fused ? sat_threads(big->ty) : 0);
     return SBP_OK;
+}
+
+int sbp_system_group_fused(sbp_system* sys, int group) {
+    clear_error();
+    if (!sys) return -1;
+    cudaSetDevice(sys->device);
+    if (sys->sched_dirty && build_schedule(sys) != SBP_OK) return -1;
+    if (group < 0 || group >= (int)sys->groups.size()) return -1;
+    return sys->groups[group].fused;
 }
 
 sbp_status sbp_system_group_tiles(sbp_system* sys, int group, int* ty, int* ctas_per_sm, int* grid) {

@@ -184,9 +184,16 @@ class BlockSystem:
         check(_capi.lib.sbp_system_group_tiles(self.h, group, ctypes.byref(ty), ctypes.byref(cps), ctypes.byref(grid)))
         return ty.value, cps.value, grid.value
 
+    def group_fused(self, group: int) -> bool:
+        """Whether one stage-kernel group takes the fused form (the SATs in the stage launches)."""
+        r = _capi.lib.sbp_system_group_fused(self.h, group)
+        if r < 0:
+            raise _capi.SbpError(1, _capi.lib.sbp_last_error().decode(errors='replace'))
+        return bool(r)
+
     def launch_stage(self, group: int, stage: int, with_edges: bool = False) -> None:
-        """Enqueue one group's stage kernel (and optionally its edge kernel) on the system's
-        stream.  Advances no time; the stage buffers are left as the launch leaves them."""
+        """Enqueue one group's stage kernel (and optionally its edge kernel; a fused group's stage kernel
+        always includes the SATs) on the system's stream.  Advances no time; the stage buffers are left as the launch leaves them."""
         check(_capi.lib.sbp_system_launch_stage(self.h, group, stage, int(with_edges)))
 
     # -- state

@@ -113,3 +113,58 @@ def test_network_reports_a_wait_that_gave_up(rt):
         assert call() != 0 and "in time" in rt.error(), name
         assert call() == 0, name
     assert rt.lib.sbp_cnn_destroy(net) == 0
+
+
+SYSTEMS = {"block": ("f64", 8), "block_f32c": ("f32c", 8), "multiblock": ("f64", 16), "ensemble": ("f64", 0)}
+
+
+@pytest.mark.parametrize("name", SYSTEMS)
+def test_autotune_reports_a_schedule_that_can_be_set(rt, monkeypatch, name):
+    """What autotune returns is the schedule (every candidate takes the same time here, so the first form
+    stays), and set_tiles takes it back: small systems keep the fused form both times."""
+    from summationbyparts_b200 import _capi, workloads
+    from summationbyparts_b200.system import BlockSystem
+    monkeypatch.setattr(_capi, "lib", rt.lib)
+    prec, rows = SYSTEMS[name]
+    if name == "ensemble":
+        insts = workloads.ensemble_instances(40, seed=1)
+        blocks, dts = workloads.ensemble_blocks(insts), [i.dt for i in insts]
+    else:
+        blocks, dts = workloads.multiblock() if name == "multiblock" else workloads.Config0().blocks(), [1e-3]
+    s = BlockSystem(blocks, len(dts), prec, 1.4)
+    for k, dt in enumerate(dts):
+        s.set_dt(dt, k)
+    launches = s.launches_per_step()
+    tiles = s.autotune()
+    assert tiles == {0: (16, 32, 256), 8: (8, 16, 288), 16: (16, 32, 320)}[rows]
+    for _ in range(2):
+        groups = range(len(s.groups()))
+        assert [s.group_fused(g) for g in groups] == [rows > 0 for _ in groups]
+        assert [s.group_tiles(g)[0] for g in groups] == [rows or 16 for _ in groups]
+        assert s.launches_per_step() == launches
+        rt.launches()
+        s.advance(1)
+        s.set_tiles(*tiles)
+    s.close()
+
+
+def test_tiles_that_cannot_be_set(rt, monkeypatch):
+    from summationbyparts_b200 import _capi, operators, workloads
+    from summationbyparts_b200.system import BC_EVAL, BC_VORTEX, BlockSpec, BlockSystem
+    monkeypatch.setattr(_capi, "lib", rt.lib)
+    x, y = workloads.warped(-5.0, 5.0, 64, -5.0, 5.0, 64)
+    v = (BC_VORTEX, 0)
+    fused = [(8, 16, 288), (16, 32, 320)]
+    other = [(8, 16, 0), (8, 32, 288), (8, 16, 256), (16, 16, 320), (16, 32, 288), (32, 32, 320), (24, 32, 0), (16, 32, 128)]
+    plain = [(16, 32, 0), (32, 32, 0), (16, 32, 256), (32, 32, 256)]
+    one = operators.Upwind9()
+    for op, bc, takes_fused in ((one, [v] * 4, True), (one, [(BC_EVAL, 0)] + [v] * 3, False),
+                                (operators.Pair(operators.SBP4(), operators.Upwind9()), [v] * 4, False)):
+        s = BlockSystem([BlockSpec(x, y, op, bc, 0)], 1, "f64", 1.4)
+        for t in plain + (fused if takes_fused else []):
+            s.set_tiles(*t)
+            assert s.group_fused(0) == (t in fused)
+        for t in other + ([] if takes_fused else fused):
+            with pytest.raises(_capi.SbpError):
+                s.set_tiles(*t)
+        s.close()
