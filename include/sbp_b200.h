@@ -324,7 +324,8 @@ int sbp_system_group_count(sbp_system* sys);
 /* Operator pair and grid points of one group. */
 sbp_status sbp_system_group_info(sbp_system* sys, int group, int* op_xi, int* op_eta, int64_t* points);
 /* Enqueue one group's stage kernel for RK4 stage 0..3 on the system's stream, followed by its
- * edge (SAT) kernel when with_edges != 0.  This advances no time and checks no status: it runs
+ * edge (SAT) kernel when with_edges != 0; the fused form's one kernel (sbp_system_group_fused) includes
+ * the SATs and takes no notice of with_edges.  This advances no time and checks no status: it runs
  * the stage on whatever the stage buffers hold, so a system used for it must be re-initialised
  * before its results mean anything. */
 sbp_status sbp_system_launch_stage(sbp_system* sys, int group, int stage, int with_edges);
