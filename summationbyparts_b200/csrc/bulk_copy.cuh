@@ -34,7 +34,8 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 
 // Wait for the barrier's phase `parity` to complete, polling at most `limit` times; false if it
-// did not complete (the caller then skips the work that needed the data).
+// did not complete (the caller then fetches the data itself or skips the work that needed them, and waits
+// once more before it gives up the shared memory that the copies end in).
 __device__ __forceinline__ bool bulk_wait(uint64_t* mbar, uint32_t parity, int limit) {
     for (int it = 0; it < limit; ++it) {
         uint32_t done;

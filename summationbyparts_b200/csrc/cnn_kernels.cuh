@@ -223,8 +223,9 @@ struct ConvArgs {
 //   warp 0     bulk copies of a band's rows into a free stage (1 KB per row and chunk)
 //   warp 1     zeroes a row outside the image, then one thread issues the 9 x CIN / 16 MMAs (K = 16
 //              each) of each of the band's 3 accumulator tiles into a free accumulator
-//   warps 2-13 take the finished tiles in turn, four warps a tile, warp w lanes 32 (w % 4) .. -- one
-//              position per thread, all channels -- and run the epilogue:
+//   warps 2-13 take the finished tiles, four warps each of a band's three, warp w lanes 32 (w % 4) .. --
+//              one position per thread, all channels -- and run the epilogue; of the 384 positions 256
+//              are pixels, all but 3 of them in the first two tiles:
 //   EPI_GELU   z = acc + bias -> zout (f32, if kept), gelu(z) -> yout (bf16)   (hidden layers)
 //   EPI_LINEAR acc + bias -> zout (f32, [pixel][8])                            (output layer)
 //   EPI_APPLY  as EPI_LINEAR, and coarse + y * out_scale -> out (f64 planes)
@@ -233,7 +234,8 @@ struct ConvArgs {
 // epilogue's issue slots and the tensor pipe (an M = 128, N = 32 product takes 64 cycles, 13 us of a
 // 32 -> 32 layer), then memory (34 MB a layer, 67 MB with pre-activations).  Measured, apply pass of 512
 // states / training step on 64: one CTA per band with copies, products and epilogue in sequence, 4
-// an SM 938 / 422 us; this form 743 / 374; one CTA an SM with 8-row bands 945 / 402; three an SM with
+// an SM 938 / 422 us; this form 743 / 374 before and 736 / 364 after its launches became dependent ones
+// (apply 739 with the votes and last waits of kStatusMmaTimeout); one CTA an SM with 8-row bands 945 / 402; three an SM with
 // one stage 755 / 394; three copies of a band, one per column offset, with no accumulator row spent
 // on padding 829 / 378 (three times the L2 traffic).
 template <int CIN, int COUT, int EPI>

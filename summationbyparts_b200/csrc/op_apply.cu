@@ -10,7 +10,7 @@
 // boundaries, which stays inside the array except at its first and last bytes, where the copy is
 // narrowed instead and a lane fetches the few elements left over (fetch_row).
 //
-// Row tiles: up to kXiRows rows x 4 KB.  A thread's outputs are one 16-byte vector of the row in
+// Row tiles: up to kXiRows rows x 2 KB.  A thread's outputs are one 16-byte vector of the row in
 // memory (a column is counted from the 16-byte boundary at or before its row's start), so window loads
 // from shared memory and stores are 16 bytes wide on every row, whatever its alignment; outputs
 // of the boundary closures and of the vectors that a row's ends cut are taken one by one

@@ -19,7 +19,7 @@
 // runs one thread per edge point.
 //
 // Work decomposition.  A persistent grid of 256-thread CTAs walks a list of (block, y0, x0)
-// output tiles of TY rows x 32 columns.  One direction at a time: the fluxes of the tile rows
+// output tiles of TY rows x tile_tx(TY) columns (32, with 8 rows 16).  One direction at a time: the fluxes of the tile rows
 // widened by the xi halo (Ehat and alpha_u q, 4 components each) go to a shared flux buffer and
 // every thread forms the xi sums of its micro-tile in registers; the fluxes of the tile columns
 // widened by the eta halo (Fhat, alpha_v q) then replace them in the same buffer for the eta sums.
@@ -100,8 +100,8 @@ struct StageArgs {
 constexpr int kStageK = 4;
 
 // Tiles along a line of n outputs (tile_starts in system.cu) start at multiples of T, except that
-// the last tile starts at e = n - M rounded down to even whenever a multiple of T would fall in
-// (e, n): so the first tile holds every start-closure output, the last every end-closure output,
+// the last tile starts at e = n - M (rounded down to even where T > M) whenever a multiple of T would fall
+// in (e, n): so the first tile holds every start-closure output, the last every end-closure output,
 // and no tile holds outputs of both ends (n >= 2 M).  The input region of a tile is then at most
 // T + 2 H wide (interior tiles and the first one: H on each side, [0, max(T + H, N)) for the
 // first; the tile before the last ends at e <= n - M, so its region stops H after it), or

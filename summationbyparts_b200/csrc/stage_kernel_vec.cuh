@@ -30,7 +30,7 @@
 //   registers one component ahead of their use, as 8-byte row pairs, which leaves the shared
 //   memory of two 256-thread CTAs per SM to the stencil arrays.
 //
-// What bounds it: issue and latency, about half of HBM's rate.  Stage 1 of Upwind9 on the 256 first
+// What bounds it: issue and latency, at 0.36 of the copy rate over the four stages.  Stage 1 of Upwind9 on the 256 first
 // instances of the seed-1 ensemble takes 169 us; 150 without the stencil sums, 139 without
 // phase 1's loads, 158 without the stores.  stage_kernel itself on 32-row compensated tiles (raw rows
 // by asynchronous copies, one direction at a time), which is the faster form in f64, takes 223 us here:

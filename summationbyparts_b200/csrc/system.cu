@@ -4,7 +4,8 @@
 // Per RK4 step the device runs, for each of the 4 stages, one persistent fused stage kernel per
 // operator pair present (all tiles of all active blocks of that pair in one launch) and its edge
 // kernel (uncoupled operator groups on their own streams, joined once per step), then one tiny
-// kernel that advances the instance times.  The whole step is captured once as a CUDA
+// kernel that advances the instance times.  Systems too small to fill the GPU take the fused form of
+// the stage kernel, with the SATs and the times in it (fused_rows).  The whole step is captured once as a CUDA
 // graph and replayed; the graph is re-captured only when the tile schedule or the set of
 // active instances changes.
 #include <cuda_runtime.h>
