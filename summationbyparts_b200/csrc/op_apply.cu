@@ -10,7 +10,7 @@
 // boundaries, which stays inside the array except at its first and last bytes, where the copy is
 // narrowed instead and a lane fetches the few elements left over (fetch_row).
 //
-// Row tiles: up to kXiRows rows x 2 KB.  A thread's outputs are one 16-byte vector of the row in
+// Row tiles: 16 or 4 rows x 2 KB.  A thread's outputs are one 16-byte vector of the row in
 // memory (a column is counted from the 16-byte boundary at or before its row's start), so window loads
 // from shared memory and stores are 16 bytes wide on every row, whatever its alignment; outputs
 // of the boundary closures and of the vectors that a row's ends cut are taken one by one
@@ -19,8 +19,8 @@
 // Arrays whose rows all start on 16-byte boundaries take instantiations (ALIGNED) in which that is
 // known: the bookkeeping of the general form costs 6% on 4 fields of 4096 x 4096.
 //
-// Column tiles: TR rows x TC adjacent columns, each thread one column over its share of the rows with
-// the D-tap window in a register ring.  The reference's fused / unfused column split falls on a
+// Column tiles: TR rows x TC adjacent columns (launch_t), each thread one column over its share of the rows
+// with the D-tap window in a register ring.  The reference's fused / unfused column split falls on a
 // multiple of 8 (f64) or 16 (f32) columns.
 //
 // Bound by memory: one read and one write of the field.  Upwind9, 4 fields of 1021 x 1533 f64 (rows off
@@ -410,9 +410,6 @@ __global__ void __launch_bounds__(kThreads)
 
 constexpr int kSms = 148;
 
-// Column tiles of 48 rows x 1 KB stream the largest share of a field per halo row; while they would
-// leave SMs without a tile (a 64 x 64 field is two of them), 16 rows x 32 columns do the work with
-// two rows per thread instead of 24 to 48.
 template <int OP, int KIND, class T, int TR, int TC, bool ALIGNED>
 cudaError_t launch_eta(const T* in, T* out, int64_t ny, int64_t nx, int64_t nbatch, int64_t bstride, const Extent& A,
                        cudaStream_t st, int polls) {
@@ -436,10 +433,22 @@ cudaError_t launch_t(int dir, const T* in, T* out, int64_t ny, int64_t nx, int64
     const uintptr_t a = reinterpret_cast<uintptr_t>(in);
     const Extent A{a, a + ((uintptr_t)(nbatch - 1) * bstride + (uintptr_t)ny * nx) * sizeof(T)};
     if (dir == 1) {
-        constexpr int TR = 48, TC = 1024 / sizeof(T);
-        if (nbatch * ((ny + TR - 1) / TR) * ((nx + TC - 1) / TC) >= kSms)
+        // Tiles of 16 rows x 32 columns, two rows per thread, while all of them fit the SMs at once; beyond that
+        // taller and wider ones, which load fewer halo rows (Upwind9 f64, us, tiles of 16 x 32, 24 rows x 1 KB, 48
+        // rows x 1 KB: 257 x 255 3.6, 5.5, 8.3; 768 x 768 7.1, 4.8, 6.6; 2048 x 2048 40, 15.4, 13.4).  f64 takes 48 rows
+        // once they give every SM a tile (467 x 1730 6.3, 24 rows 5.0; 756 x 998 x 2 7.9, 8.3); f32 keeps 24, whose
+        // shared memory lets more CTAs run (2049 x 2047 SBP4 8.9, 48 rows 12.1; 4096 x 4096 Upwind9 31.9, 33.9).
+        // Fields no wider than half of a tile take half the width, so that fewer threads are without a column
+        // (100,000 x 17 Upwind9 f64 28 instead of 35 us, 2000 fields of 17 x 19 f32 19 instead of 29).
+        constexpr int TC = 1024 / sizeof(T), TR = 6 * sizeof(T);
+        auto tiles = [&](int tr, int tc) { return nbatch * ((ny + tr - 1) / tr) * ((nx + tc - 1) / tc); };
+        if (tiles(16, 32) <= 5 * kSms)
+            return launch_eta<OP, KIND, T, 16, 32, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
+        if (nx <= TC / 2)
+            return launch_eta<OP, KIND, T, TR, TC / 2, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
+        if (TR > 24 && tiles(TR, TC) >= kSms)
             return launch_eta<OP, KIND, T, TR, TC, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
-        return launch_eta<OP, KIND, T, 16, 32, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
+        return launch_eta<OP, KIND, T, 24, TC, ALIGNED>(in, out, ny, nx, nbatch, bstride, A, st, polls);
     }
     constexpr int TC = xi_cols<T>();
     const int64_t ncb = (nx + (ALIGNED ? 0 : K - 1) + TC - 1) / TC;

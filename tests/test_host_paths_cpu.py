@@ -71,13 +71,13 @@ PTR = 1 << 20  # an address that no host code reads
 @pytest.mark.parametrize("nx", [1533, 1536])  # rows off and on the 16-byte boundaries
 @pytest.mark.parametrize("dtype", [0, 1])
 def test_operators_on_every_device(rt, nx, dtype):
-    """A column application large enough for the 48-row tiles takes more than 48 KB of shared memory, which
-    is allowed per function and device: it runs on each device of a process, whatever ran before."""
+    """A large f64 column application takes more than 48 KB of shared memory, which is allowed per function and
+    device: it runs on each device of a process, whatever ran before."""
     for d in (0, 3, 0, 1):
         rt.device(d)
         assert rt.lib.sbp_diffeta(2, dtype, PTR, 2 * PTR + 8, 1021, nx, 4, 1021 * nx, None) == 0, rt.error()
         (name, dev, _, _, smem), = rt.launches()
-        assert "op_eta_kernel" in name and dev == d and smem > 48 * 1024
+        assert "op_eta_kernel" in name and dev == d and (dtype == 1 or smem > 48 * 1024)
 
 
 def test_network_on_every_device(rt):
