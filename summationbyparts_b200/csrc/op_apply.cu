@@ -211,13 +211,17 @@ __device__ __noinline__ void xi_fetch_plainly(const T* __restrict__ src, T* buf,
     bulk_wait(bar, 0, kBulkWaitPolls);
 }
 
-// Row direction (see the file comment): `tr` rows per tile, 2^lpr threads per row.  u counts elements
+// Row direction (see the file comment): `tr` rows per tile, 2^lpr threads per row.  WIDE: 16 rows and 128
+// threads, known to the compiler, which saves a large aligned field of the lighter operators its loop over
+// a row's vectors: SBP4 on 1874 x 856 f64 8.1 to 7.0 us and on 20 x 1,000,000 f32 31.6 to 27.2, Upwind9 on 4 fields
+// of 4096 x 4096 f64 179 to 167 and f32 98 to 89.  u counts elements
 // from the 16-byte boundary at or before a row's start; tile cb covers u in [cb TC, cb TC + TC).
 // vec_out: output rows have the alignment of the input rows, so vectors are stored whole.
-template <int OP, int KIND, class T, bool ALIGNED>
+template <int OP, int KIND, class T, bool ALIGNED, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
-    op_xi_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int ncb, int tr,
-                 int lpr, bool vec_out, Extent A, int polls) {
+    op_xi_kernel(const T* __restrict__ in, T* __restrict__ out, int ny, int nx, int64_t bstride, T idx, int ncb, int rows,
+                 int lanes, bool vec_out, Extent A, int polls) {
+    const int tr = WIDE ? kXiRows : rows, lpr = WIDE ? 7 : lanes;
     constexpr int M = OpShape<OP>::M, H = OpShape<OP>::H;
     constexpr int K = 16 / sizeof(T);
     constexpr int TC = xi_cols<T>(), P = xi_pitch<T>();
@@ -461,8 +465,13 @@ cudaError_t launch_t(int dir, const T* in, T* out, int64_t ny, int64_t nx, int64
     const bool vec_out = (a - reinterpret_cast<uintptr_t>(out)) % 16 == 0;
     const T idx = inv_spacing<T>(OpShape<OP>::h2, nx);
     const int64_t items = nbatch * ((ny + tr - 1) / tr) * ncb;
-    return launch_after(op_xi_kernel<OP, KIND, T, ALIGNED>, (unsigned)items, kThreads, xi_smem<T>(tr), st, in, out, (int)ny,
-                        (int)nx, bstride, idx, (int)ncb, tr, lpr, vec_out, A, polls);
+    auto launch = [&](auto kernel) {
+        return launch_after(kernel, (unsigned)items, kThreads, xi_smem<T>(tr), st, in, out, (int)ny, (int)nx, bstride, idx,
+                            (int)ncb, tr, lpr, vec_out, A, polls);
+    };
+    if constexpr (ALIGNED)
+        if (tr == kXiRows && lpr == 7) return launch(op_xi_kernel<OP, KIND, T, ALIGNED, true>);
+    return launch(op_xi_kernel<OP, KIND, T, ALIGNED, false>);
 }
 
 template <int OP, class T>
