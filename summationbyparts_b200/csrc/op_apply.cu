@@ -31,7 +31,7 @@
 // previous kernel of the stream drains, and waits for it before it touches global memory.  The four
 // applications in a row on 64 x 64 f64 Upwind4: 21.4 to 19.3 us; on 4 fields of 1021 x 1533 f64 Upwind9:
 // 112 to 104 us; the two of SBP8 on 4 fields of 1537 x 2047 f32: 64 to 60 us; the four of Upwind9 on 4
-// fields of 4096 x 4096 f64: 813 to 796 us.
+// fields of 4096 x 4096 f64: 813 to 796 us (781 with the WIDE rows of op_xi_kernel).
 #include <cuda_runtime.h>
 
 #include <cstdint>
