@@ -207,7 +207,7 @@ struct sbp_cnn {
     __nv_bfloat16* dz[kLayers] = {};  // output gradients
     float *part_w = nullptr, *part_b = nullptr, *part_loss = nullptr;
     StatusWord status{};              // of the tensor-core kernels
-    int polls = kMmaWaitLimit;        // of every wait of the tensor-core kernels
+    bool give_up = false;             // the tensor-core kernels, at every wait
     float4 in_mean{0, 0, 0, 0}, in_inv{1, 1, 1, 1}, out_scale{1, 1, 1, 1};
     int adam_t = 0;
     std::vector<void*> allocs;
@@ -223,7 +223,7 @@ cudaError_t conv(const sbp_cnn* c, int n, ConvArgs a) {
     const cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&conv3x3_tc_kernel<CIN, COUT, EPI>), bytes);
     if (e != cudaSuccess) return e;
     a.status = c->status;
-    a.polls = c->polls;
+    a.give_up = c->give_up;
     a.bands = n * (kImg / kBand);
     const int grid = a.bands < 2 * c->num_sms ? a.bands : 2 * c->num_sms;
     return launch_after(conv3x3_tc_kernel<CIN, COUT, EPI>, grid, kConvThreads, bytes, c->st(), a);
@@ -258,7 +258,7 @@ cudaError_t wgrad(const sbp_cnn* c, int n, int layer, const __nv_bfloat16* x, co
     static DynamicSmem opt_in;
     cudaError_t e = opt_in.allow(reinterpret_cast<const void*>(&wgrad_tc_kernel<CIN, M, MSTORE>), bytes);
     if (e != cudaSuccess) return e;
-    e = launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->polls,
+    e = launch_after(wgrad_tc_kernel<CIN, M, MSTORE>, parts, kWgradThreads, bytes, c->st(), x, dz, c->part_w, c->part_b, c->give_up,
                      c->status);
     if (e != cudaSuccess) return e;
     const int nw = MSTORE * 9 * CIN, nb = MSTORE;
@@ -359,8 +359,8 @@ sbp_status refresh_bf16(sbp_cnn* c) {
 }  // namespace
 
 namespace sbp {
-// Polls of every later wait of the network's kernels.
-void cnn_wait_limit(sbp_cnn* c, int polls) { c->polls = polls; }
+// Whether every later wait of the network's kernels gives up at once, as after its last poll (for tests).
+void cnn_give_up(sbp_cnn* c, bool on) { c->give_up = on; }
 }  // namespace sbp
 
 extern "C" {

@@ -161,9 +161,10 @@ struct StatusWord {
 };
 constexpr int kMmaWaitLimit = 1 << 22;  // mbarrier polls before giving up
 
-// bulk_wait for a whole warp: the lanes agree, so that they stay together for what is warp-wide.
-__device__ __forceinline__ bool warp_wait(uint64_t* mbar, uint32_t parity, int limit) {
-    return __all_sync(0xffffffffu, bulk_wait(mbar, parity, limit));
+// bulk_wait for a whole warp: the lanes agree, so that they stay together for what is warp-wide.  give_up:
+// without a poll (the limit itself as an argument costs the apply pass of 512 states 4 of 728 us).
+__device__ __forceinline__ bool warp_wait(uint64_t* mbar, uint32_t parity, bool give_up = false) {
+    return __all_sync(0xffffffffu, !give_up && bulk_wait(mbar, parity, kMmaWaitLimit));
 }
 
 // Shared-memory layout of the tcgen05 convolution (dynamic): the weights, then kConvStages band stages.
@@ -212,7 +213,7 @@ struct ConvArgs {
     float4 oscale;
     double* out;
     int bands;                 // bands of all images
-    int polls;                 // of every wait
+    bool give_up;              // at every wait (for tests)
     StatusWord status;
 };
 
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
         int i = 0;
         for (int band = blockIdx.x; band < A.bands; band += gridDim.x, ++i) {
             const int st = i % kConvStages, img = band / kBands, r0 = band % kBands * kBand;
-            if (i >= kConvStages) ok = warp_wait(empty + st, (i / kConvStages - 1) & 1, A.polls);
+            if (i >= kConvStages) ok = warp_wait(empty + st, (i / kConvStages - 1) & 1, A.give_up);
             if (!ok) break;
             const int hlo = r0 == 0 ? 1 : 0, rows = (r0 + kBand == kImg ? L::HR - 1 : L::HR) - hlo;
             if (lane == 0) bulk_expect(full + st, (uint32_t)(L::CH * rows * kImg * 16));
@@ -296,19 +297,19 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
             }
         }
         // the copies of the weights and of the last bands have arrived, whatever the other warps did
-        ok = warp_wait(wbar, 0, kMmaWaitLimit) && ok;
+        ok = warp_wait(wbar, 0) && ok;
         for (int b = i < kConvStages ? 0 : i - kConvStages; b < i; ++b)
-            ok = warp_wait(full + b % kConvStages, (b / kConvStages) & 1, kMmaWaitLimit) && ok;
+            ok = warp_wait(full + b % kConvStages, (b / kConvStages) & 1) && ok;
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc_bf16(128, L::NP, false);
         const uint32_t wbase = smem_u32(smem);
         dependency_wait();
-        ok = warp_wait(wbar, 0, A.polls);
+        ok = warp_wait(wbar, 0, A.give_up);
         int i = 0, j = 0;  // bands and accumulator tiles so far
         for (int band = blockIdx.x; band < A.bands && ok; band += gridDim.x, ++i) {
             const int st = i % kConvStages, r0 = band % kBands * kBand;
             unsigned char* stage = smem + L::X_OFF + st * L::STAGE;
-            ok = warp_wait(full + st, (i / kConvStages) & 1, A.polls);
+            ok = warp_wait(full + st, (i / kConvStages) & 1, A.give_up);
             if (!ok) break;
             if (r0 == 0 || r0 + kBand == kImg) {
                 const int r = r0 == 0 ? 0 : L::HR - 1;
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
             const uint32_t base = smem_u32(stage);
             for (int h = 0; h < L::TILES; ++h, ++j) {
                 const int acc = j % kConvAccs;
-                if (j >= kConvAccs) ok = warp_wait(aempty + acc, (j / kConvAccs - 1) & 1, A.polls);
+                if (j >= kConvAccs) ok = warp_wait(aempty + acc, (j / kConvAccs - 1) & 1, A.give_up);
                 if (!ok) break;
                 tc_fence_after();
                 if (lane == 0) {
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
             }
         }
         // the products issued so far are done
-        if (j > 0) ok = warp_wait(afull + (j - 1) % kConvAccs, ((j - 1) / kConvAccs) & 1, kMmaWaitLimit) && ok;
+        if (j > 0) ok = warp_wait(afull + (j - 1) % kConvAccs, ((j - 1) / kConvAccs) & 1) && ok;
     } else {
         dependency_wait();
         for (int t = (warp - 2) >> 2;; t += kConvGroups) {  // tile t of the CTA: tile t % TILES of its band t / TILES
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_tc_kernel(const ConvA
                 for (int q = 0; q < COUT / 4; ++q) zp[q] = real ? __ldg(src + q * kPix) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
             __syncwarp();
-            ok = warp_wait(afull + acc, (t / kConvAccs) & 1, A.polls);
+            ok = warp_wait(afull + acc, (t / kConvAccs) & 1, A.give_up);
             if (!ok) break;
             tc_fence_after();
             float v[32];
@@ -467,7 +468,7 @@ template <int CIN, int M, int MSTORE>
 __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bfloat16* __restrict__ x,
                                                                 const __nv_bfloat16* __restrict__ dz,
                                                                 float* __restrict__ part_w,
-                                                                float* __restrict__ part_b, int polls,
+                                                                float* __restrict__ part_b, bool give_up,
                                                                 const StatusWord status) {
     using L = WgradTcLayout<CIN, M>;
     static_assert(CIN % 16 == 0 && M % 16 == 0 && MSTORE <= M && L::ONES < 16, "channel padding");
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
             bulk_g2s(smem + i * L::PLANE + (hlo * kImg + (dx == 0)) * 16, src, ((hhi - hlo) * kImg - (dx != 1)) * 16, bar);
         }
     }
-    const bool arrived = bulk_wait(bar, 0, polls);
+    const bool arrived = !give_up && bulk_wait(bar, 0, kMmaWaitLimit);
     // the column that a shifted copy took from the row beside it is zero padding, and so are the
     // rows outside the image
     for (int i = tid; i < L::HR * L::CH * 2; i += kWgradThreads) {
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(kWgradThreads) wgrad_tc_kernel(const __nv_bflo
         umma_commit(bar + 1);
     }
     __syncwarp();
-    const bool done = loaded && warp_wait(bar + 1, 0, polls);
+    const bool done = loaded && warp_wait(bar + 1, 0);
     tc_fence_after();
     if (done) {
         float* pw = part_w + (int64_t)blockIdx.x * (MSTORE * 9 * CIN);
