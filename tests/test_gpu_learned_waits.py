@@ -1,5 +1,6 @@
-"""A network kernel whose bounded waits run out: each gives up at its first wait, without a poll.  The call that next synchronises raises, the optimiser has changed nothing, and afterwards the
-network works as before, to the last bit."""
+"""A network kernel whose bounded waits run out: each gives up at its first wait, without a poll.  The call
+that next synchronises raises, the optimiser has changed nothing, and afterwards the network works as
+before, to the last bit."""
 import ctypes
 
 import pytest
