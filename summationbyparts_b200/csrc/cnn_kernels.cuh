@@ -236,7 +236,7 @@ struct ConvArgs {
 // 32 -> 32 layer), then memory (34 MB a layer, 67 MB with pre-activations).  Measured, apply pass of 512
 // states / training step on 64: one CTA per band with copies, products and epilogue in sequence, 4
 // an SM 938 / 422 us; this form 743 / 374 before and 736 / 364 after its launches became dependent ones
-// (apply 739 with the votes and last waits of kStatusMmaTimeout); one CTA an SM with 8-row bands 945 / 402; three an SM with
+// (apply 741 with the votes and last waits of kStatusMmaTimeout); one CTA an SM with 8-row bands 945 / 402; three an SM with
 // one stage 755 / 394; three copies of a band, one per column offset, with no accumulator row spent
 // on padding 829 / 378 (three times the L2 traffic).
 template <int CIN, int COUT, int EPI>
